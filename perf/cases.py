@@ -103,7 +103,7 @@ def _cell(seed, rmin, rmax, loose=False):
     cloud in which a third have a neighbour within half a millimetre and few touch one."""
     n, rng = 1500, _rng(seed, 1)
     r = rng.uniform(rmin, rmax, n)
-    side = ((4.0 / 3.0) * math.pi * (r ** 3).sum() / (0.11 if loose else 0.58)) ** (1.0 / 3.0)
+    side = ((4.0 / 3.0) * math.pi * (r ** 3).sum() / (0.16 if loose else 0.58)) ** (1.0 / 3.0)
     x = torch.tensor(rng.uniform(0.0, side, (3, n)) / rmax, dtype=torch.float32, device=_device())
     rr = torch.tensor(r * (rng.uniform(0.996, 1.04, n) if loose else 1.0) / rmax, dtype=torch.float32, device=_device())
     reach, box = rr[:, None] + rr[None, :], float(side / rmax)
