@@ -25,13 +25,140 @@
 #include "xd_grid.cuh"
 #include "xd_internal.cuh"
 #include "xd_physics64.cuh"
+#include "xd_scan.cuh"
 
 namespace xd {
 
 // ------------------------------------------------------- particle-particle
 
-template <bool HIST>
-__global__ void __launch_bounds__(128) k_p2p(Params P, const double* __restrict__ pos,
+// Results of a warp's contacts in its ScanBuf (9 values): T = Fn + Ft (the
+// normal force alone when the slip is zero), Ft, M.
+enum { kContact = 1u, kSlip = 2u };
+
+__device__ __forceinline__ void put3(double (*res)[32], int a, unsigned lane, d3 v)
+{
+    res[a][lane] = v.x;
+    res[a + 1][lane] = v.y;
+    res[a + 2][lane] = v.z;
+}
+__device__ __forceinline__ d3 get3(const double (*res)[32], int a, unsigned lane)
+{
+    return mk(res[a][lane], res[a + 1][lane], res[a + 2][lane]);
+}
+
+// A position and radius in FP32 for the search's near tests, and the sum of
+// its coordinates' sizes, which bounds their rounding.
+struct Near4 {
+    float x, y, z, r, size;
+};
+__device__ __forceinline__ Near4 near_of(const d4& p)
+{
+    Near4 n{ f32_of(p.x), f32_of(p.y), f32_of(p.z), f32_of(p.w), 0.f };
+    n.size = fabsf(n.x) + fabsf(n.y) + fabsf(n.z);
+    return n;
+}
+
+// Whether two spheres may touch: the FP32 distance against the radii with a
+// margin above the rounding of both (2^-23 of every coordinate, and of the
+// sums).  A value that is not finite, and any distance below 1e-15 m (where
+// squares leave the FP32 range), counts as near.
+__device__ __forceinline__ bool spheres_near(const Near4& a, const Near4& b)
+{
+    const float dx = b.x - a.x, dy = b.y - a.y, dz = b.z - a.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    const float lim = (a.r + b.r) * 1.000001f + (a.size + b.size) * 2e-7f;
+    return !(d2 > lim * lim * 1.000002f && d2 > 1e-30f);
+}
+
+// calculate_p2p_kernel<1> (impl:403-485), a warp for 32 / LP particles.
+//
+// Bound by the FP64 pipe: some 250 operations a contact.  The candidates (65
+// a particle on cells of one diameter, a thousand on the coarse cells of a
+// mesh) are tested in FP32 from integer-cut coordinates, and the FP64 law
+// runs on contacts alone, one per lane (xd_scan.cuh).  Every operation on a
+// contact and the order of every sum are the thread-per-particle form's, so
+// the results are the same bits.  A bed of 120,989 spheres: 0.4 ms, 3.5 ms
+// with the law evaluated where a thread found a contact; 8,000 spheres 50 us
+// (438), 17,159 on a mesh's cells of 2.5 cm 212 us (2,527).
+template <int LP>
+__global__ void __launch_bounds__(64, 8) k_p2p(Params P, const double* __restrict__ pos,
+                                               const double* __restrict__ vel, const double* __restrict__ omega,
+                                               double* __restrict__ force, double* __restrict__ moment,
+                                               const double* __restrict__ mass, const unsigned* __restrict__ sorted,
+                                               const unsigned* __restrict__ cstart, const unsigned* __restrict__ cend,
+                                               const xd_contact_property* __restrict__ cp, unsigned np)
+{
+    using Buf = ScanBuf<LP, double, 9>;
+    __shared__ Buf bufs[2];
+    __shared__ PairConst pc;
+    if (threadIdx.x == 0) pc = load_pair_const(cp);
+    __syncthreads();
+    Buf& B = bufs[threadIdx.x / 32u];
+    constexpr unsigned NP = 32 / LP;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned groups = (np + NP - 1u) / NP;
+    for (unsigned g = blockIdx.x * 2u + threadIdx.x / 32u; g < groups; g += gridDim.x * 2u) {
+        const unsigned id0 = g * NP, id = id0 + lane / LP;
+        const bool valid = id < np;
+        d4 ip = d4{ 0, 0, 0, 0 };
+        int3 gp = make_int3(0, 0, 0);
+        if (valid) {
+            ip = ld4(pos, id);
+            gp = grid_pos_fast(P, ip.x, ip.y, ip.z);
+        }
+        const Near4 mine = near_of(ip);
+        const unsigned runs = stage_runs<LP>(B, valid, gp, cstart, cend,
+                                             [&](int x, int y, int z) { return grid_hash(P, x, y, z); });
+        d3 Ft = mk(0, 0, 0), M = mk(0, 0, 0), sumF = mk(0, 0, 0), sumM = mk(0, 0, 0);
+        scan_contacts<LP>(
+            B, runs, sorted,
+            [&](unsigned k, unsigned) { return k != id && k < np && spheres_near(mine, near_of(ld4(pos, k))); },
+            [&](unsigned o, unsigned k, unsigned l) {
+                const unsigned i = id0 + o;
+                const d4 a = ld4(pos, i), b = ld4(pos, k);
+                const d3 rp = mk(b.x - a.x, b.y - a.y, b.z - a.z);
+                const double dist = length(rp);
+                const double cdist = (a.w + b.w) - dist;
+                if (!(cdist > 0)) return 0u;
+                const d3 ivel = ld3(vel, i), jvel = ld3(vel, k), iomega = ld3(omega, i), jomega = ld3(omega, k);
+                const d3 unit = rp / dist;
+                const d3 rv = P.rolling ? (jvel + cross(jomega, -b.w * unit)) - (ivel + cross(iomega, a.w * unit))
+                                        : (jvel - ivel);
+                const Fc c = get_constant(pc, a.w, b.w, __ldg(mass + i), __ldg(mass + k));
+                d3 Fn, t = mk(0, 0, 0), m = mk(0, 0, 0);
+                const bool slip = dhs(c, a.w, b.w, pc.Ei, pc.Ej, pc.pri, pc.prj, pc.coh, cdist, rv, unit, P.dt, t,
+                                      Fn, m);
+                if (!slip) {
+                    put3(B.res, 0, l, Fn);
+                    return (unsigned)kContact;
+                }
+                put3(B.res, 0, l, Fn + t);
+                put3(B.res, 3, l, t);
+                put3(B.res, 6, l, m);
+                return (unsigned)(kContact | kSlip);
+            },
+            [&](unsigned code, unsigned l) {
+                d3 t = get3(B.res, 0, l);
+                if (code & kSlip) {
+                    Ft = get3(B.res, 3, l);
+                    M = get3(B.res, 6, l);
+                } else {   // the tangential force and moment of the contact before stay (impl:390-400)
+                    t = t + Ft;
+                }
+                sumF += t;
+                sumM += M;
+            });
+        const unsigned me = id0 + lane;
+        if (lane < NP && me < np) {
+            st3(force, me, ld3rw(force, me) + sumF);
+            st3(moment, me, ld3rw(moment, me) + sumM);
+        }
+    }
+}
+
+// With tangential history: a thread per particle (the tables are read and
+// written contact by contact in search order).
+__global__ void __launch_bounds__(128) k_p2p_hist(Params P, const double* __restrict__ pos,
                                              const double* __restrict__ vel,
                                              const double* __restrict__ omega,
                                              double* __restrict__ force, double* __restrict__ moment,
@@ -45,7 +172,7 @@ __global__ void __launch_bounds__(128) k_p2p(Params P, const double* __restrict_
     unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= np) return;
     HistState hs;
-    if (HIST) hist_begin(ht, id, hs);
+    hist_begin(ht, id, hs);
     const PairConst pc = load_pair_const(cp);
     d4 ip = ld4(pos, id);
     d3 ipos = xyz(ip);
@@ -79,16 +206,11 @@ __global__ void __launch_bounds__(128) k_p2p(Params P, const double* __restrict_
                         d3 rv = P.rolling ? (jvel + cross(jomega, -jr * unit)) - (ivel + cross(iomega, ir * unit))
                                           : (jvel - ivel);
                         Fc c = get_constant(pc, ir, jr, im, jm);
-                        if (HIST) {
-                            Fn = normal_force(c, ir, jr, pc.Ei, pc.Ej, pc.pri, pc.prj, pc.coh, cdist, rv, unit);
-                            d3 d;
-                            int sl = hist_slot(ht, hs, id, k, d);
-                            hist_tangential(c, ir, rv, unit, P.dt, Fn, d, Ft, M);
-                            hist_store(ht, sl, id, d);
-                        } else {
-                            dhs(c, ir, jr, pc.Ei, pc.Ej, pc.pri, pc.prj, pc.coh, cdist, rv, unit, P.dt,
-                                Ft, Fn, M);
-                        }
+                        Fn = normal_force(c, ir, jr, pc.Ei, pc.Ej, pc.pri, pc.prj, pc.coh, cdist, rv, unit);
+                        d3 d;
+                        int sl = hist_slot(ht, hs, id, k, d);
+                        hist_tangential(c, ir, rv, unit, P.dt, Fn, d, Ft, M);
+                        hist_store(ht, sl, id, d);
                         sumF += Fn + Ft;
                         sumM += M;
                     }
@@ -96,7 +218,7 @@ __global__ void __launch_bounds__(128) k_p2p(Params P, const double* __restrict_
             }
         }
     }
-    if (HIST) hist_end(ht, hs, id, 0u);
+    hist_end(ht, hs, id, 0u);
     double* f = force + 3 * (size_t)id;
     double* m = moment + 3 * (size_t)id;
     f[0] += sumF.x; f[1] += sumF.y; f[2] += sumF.z;
@@ -108,8 +230,79 @@ __global__ void __launch_bounds__(128) k_p2p(Params P, const double* __restrict_
 // Planes applied in order; each adds Fn + Ft to the running force exactly
 // like one plane_contact_force_kernel launch per plane.  cp_stride = 0
 // shares one property (cube), 1 gives one per plane.
-template <bool HIST>
-__global__ void __launch_bounds__(128) k_planes(Params P, const xd_plane_info* __restrict__ planes,
+//
+// Every region of plane_detection needs |wp.z| < r (wp.z the offset along
+// uw), so a particle whose FP32 offset exceeds r by more than its rounding
+// has no contact and adds zero.  The few that remain are gathered by block
+// and run the FP64 code side by side: one warp of a block's eight instead of
+// every warp that holds a particle near the wall.
+__global__ void __launch_bounds__(256) k_planes(Params P, const xd_plane_info* __restrict__ planes,
+                                                const xd_contact_property* __restrict__ cps, unsigned cp_stride,
+                                                unsigned nplanes, const double* __restrict__ pos,
+                                                const double* __restrict__ vel, const double* __restrict__ omega,
+                                                double* __restrict__ force, double* __restrict__ moment,
+                                                const double* __restrict__ mass, unsigned np)
+{
+    __shared__ unsigned near_of_block[256], who[256];
+    __shared__ unsigned count;
+    const unsigned mine = blockIdx.x * blockDim.x + threadIdx.x;
+    Near4 p{};
+    if (mine < np) p = near_of(ld4(pos, mine));
+    for (unsigned w0 = 0; w0 < nplanes; w0 += 32u) {
+        if (threadIdx.x == 0) count = 0;
+        __syncthreads();
+        unsigned near = 0;
+        for (unsigned w = w0; w < min(nplanes, w0 + 32u); ++w) {
+            const xd_plane_info* q = planes + w;
+            const float ux = f32_of(__ldg(q->uw)), uy = f32_of(__ldg(q->uw + 1)), uz = f32_of(__ldg(q->uw + 2));
+            const float x0 = f32_of(__ldg(q->xw)), y0 = f32_of(__ldg(q->xw + 1)), z0 = f32_of(__ldg(q->xw + 2));
+            const float h = (p.x - x0) * ux + (p.y - y0) * uy + (p.z - z0) * uz;
+            const float err = (fabsf(p.x) + fabsf(x0)) * fabsf(ux) + (fabsf(p.y) + fabsf(y0)) * fabsf(uy) +
+                              (fabsf(p.z) + fabsf(z0)) * fabsf(uz);
+            if (!(fabsf(h) > p.r * 1.000001f + err * 1e-6f + 1e-30f)) near |= 1u << (w - w0);
+        }
+        if (mine < np && near) {
+            const unsigned t = atomicAdd(&count, 1u);
+            near_of_block[t] = near;
+            who[t] = mine;
+        }
+        __syncthreads();
+        if (threadIdx.x < count) {
+            const unsigned id = who[threadIdx.x];
+            const double m = __ldg(mass + id);
+            const d4 ip = ld4(pos, id);
+            const d3 ipos3 = xyz(ip);
+            const double r = ip.w;
+            const d3 ivel = ld3(vel, id);
+            const d3 iomega = ld3(omega, id);
+            d3 f = ld3rw(force, id);
+            d3 mo = ld3rw(moment, id);
+            for (unsigned left = near_of_block[threadIdx.x]; left; left &= left - 1u) {
+                const unsigned w = w0 + (unsigned)(__ffs(left) - 1);
+                const PlaneD pe = load_plane(planes + w);
+                d3 Fn = mk(0, 0, 0), Ft = mk(0, 0, 0), M = mk(0, 0, 0);
+                const d3 dp = ipos3 - pe.xw;
+                d3 unit = mk(0, 0, 0);
+                const d3 wp = mk(dot(dp, pe.u1), dot(dp, pe.u2), dot(dp, pe.uw));
+                const double cdist = plane_detection(pe, ipos3, wp, unit, r);
+                if (cdist > 0) {
+                    const PairConst pc = load_pair_const(cps + (size_t)w * cp_stride);
+                    const d3 dv = P.rolling ? -(ivel + cross(iomega, r * unit)) : -ivel;
+                    const Fc c = get_constant(pc, r, 0.0, m, 0.0);
+                    dhs(c, 0, 0, 0, 0, 0, 0, pc.coh, cdist, dv, unit, P.dt, Ft, Fn, M);
+                }
+                f += Fn + Ft;
+                mo += M;
+            }
+            st3(force, id, f);
+            st3(moment, id, mo);
+        }
+        __syncthreads();
+    }
+}
+
+// The same with tangential history, a thread per particle.
+__global__ void __launch_bounds__(128) k_planes_hist(Params P, const xd_plane_info* __restrict__ planes,
                                                 const xd_contact_property* __restrict__ cps,
                                                 unsigned cp_stride, unsigned nplanes,
                                                 const double* __restrict__ pos,
@@ -123,7 +316,7 @@ __global__ void __launch_bounds__(128) k_planes(Params P, const xd_plane_info* _
     unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= np) return;
     HistState hs;
-    if (HIST) hist_begin(ht, id, hs);
+    hist_begin(ht, id, hs);
     double m = __ldg(mass + id);
     d4 ip = ld4(pos, id);
     d3 ipos3 = xyz(ip);
@@ -144,20 +337,16 @@ __global__ void __launch_bounds__(128) k_planes(Params P, const xd_plane_info* _
             PairConst pc = load_pair_const(cp);
             d3 dv = P.rolling ? -(ivel + cross(iomega, r * unit)) : -ivel;
             Fc c = get_constant(pc, r, 0.0, m, 0.0);
-            if (HIST) {
-                Fn = normal_force(c, 0, 0, 0, 0, 0, 0, pc.coh, cdist, dv, unit);
-                d3 d;
-                int sl = hist_slot(ht, hs, id, kHistPlane | w, d);
-                hist_tangential(c, 0.0, dv, unit, P.dt, Fn, d, Ft, M);
-                hist_store(ht, sl, id, d);
-            } else {
-                dhs(c, 0, 0, 0, 0, 0, 0, pc.coh, cdist, dv, unit, P.dt, Ft, Fn, M);
-            }
+            Fn = normal_force(c, 0, 0, 0, 0, 0, 0, pc.coh, cdist, dv, unit);
+            d3 d;
+            int sl = hist_slot(ht, hs, id, kHistPlane | w, d);
+            hist_tangential(c, 0.0, dv, unit, P.dt, Fn, d, Ft, M);
+            hist_store(ht, sl, id, d);
         }
         f += Fn + Ft;
         mo += M;
     }
-    if (HIST) hist_end(ht, hs, id, 1u);
+    hist_end(ht, hs, id, 1u);
     st3(force, id, f);
     st3(moment, id, mo);
 }
@@ -544,12 +733,18 @@ int launch_p2p(const Params& P, const double* pos, const double* vel, const doub
                unsigned np, cudaStream_t s, const HistTable* ht)
 {
     if (np == 0) return XD_OK;
-    if (ht)
-        k_p2p<true><<<div_up(np, 128), 128, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart,
-                                                    cend, cp, np, *ht);
-    else
-        k_p2p<false><<<div_up(np, 128), 128, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart,
-                                                     cend, cp, np, HistTable{});
+    if (ht) {
+        k_p2p_hist<<<div_up(np, 128), 128, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart, cend,
+                                                   cp, np, *ht);
+        return launch_status("calculate_p2p");
+    }
+    const int lp = scan_lanes(np);
+    const unsigned nb = scan_blocks(np, lp);
+#define XD_P2P(LP) k_p2p<LP><<<nb, 64, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart, cend, cp, np)
+    if (lp == 1) XD_P2P(1);
+    else if (lp == 4) XD_P2P(4);
+    else XD_P2P(8);
+#undef XD_P2P
     return launch_status("calculate_p2p");
 }
 
@@ -560,11 +755,11 @@ int launch_planes(const Params& P, const xd_plane_info* planes, const xd_contact
 {
     if (np == 0 || nplanes == 0) return XD_OK;
     if (ht)
-        k_planes<true><<<div_up(np, 128), 128, 0, s>>>(P, planes, cps, cp_stride, nplanes, pos, vel, omega,
-                                                       force, moment, mass, np, *ht);
+        k_planes_hist<<<div_up(np, 128), 128, 0, s>>>(P, planes, cps, cp_stride, nplanes, pos, vel, omega, force,
+                                                      moment, mass, np, *ht);
     else
-        k_planes<false><<<div_up(np, 128), 128, 0, s>>>(P, planes, cps, cp_stride, nplanes, pos, vel, omega,
-                                                        force, moment, mass, np, HistTable{});
+        k_planes<<<div_up(np, 256), 256, 0, s>>>(P, planes, cps, cp_stride, nplanes, pos, vel, omega, force, moment,
+                                                 mass, np);
     return launch_status("plane_contact_force");
 }
 

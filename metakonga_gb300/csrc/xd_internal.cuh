@@ -77,7 +77,16 @@ struct Params {
     double cohesion;
     double g[3];
     double wo[3];
+    float wof[3];    // FP32 estimates of wo and 1 / cs (set_cell_estimate): cell_of
+    float inv_csf;
 };
+
+// Sets the FP32 estimates after wo or cs has changed.
+inline void set_cell_estimate(Params& p)
+{
+    for (int i = 0; i < 3; ++i) p.wof[i] = (float)p.wo[i];
+    p.inv_csf = (float)(1.0 / p.cs);
+}
 
 inline Params to_params(const xd_device_parameters& h)
 {
@@ -97,6 +106,7 @@ inline Params to_params(const xd_device_parameters& h)
         p.g[i] = h.gravity[i];
         p.wo[i] = h.world_origin[i];
     }
+    set_cell_estimate(p);
     return p;
 }
 

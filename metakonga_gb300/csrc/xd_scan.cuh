@@ -1,0 +1,218 @@
+// The contact search shared by the FP64 and FP32 contact kernels: each
+// particle's 27 cells scanned with an FP32 test that never misses a contact,
+// the partners that pass collected per particle in search order, and the
+// exact contact law then run on them one per lane.
+//
+// What it is for: a thread per particle that evaluates the law where it finds
+// a contact runs the law for a lane or two at a time (a packed bed has four
+// contacts among some 65 candidates), and GB300 issues an FP64 instruction of
+// a warp in about 16 cycles whatever its lanes do.  Collected first, a warp's
+// contacts fill its lanes.  The order of every particle's sums stays the
+// reference's search order.
+#pragma once
+
+#include "xd_internal.cuh"
+
+namespace xd {
+
+constexpr unsigned kFullWarp = 0xffffffffu;
+
+// An FP64 value rounded towards zero to FP32 in integer instructions (the
+// conversion instruction runs on the FP64 pipe): relative error below 2^-23;
+// below the FP32 range it becomes 0 or a wrong value below 2^-126, beyond it
+// (or not finite) infinity.
+__device__ __forceinline__ float f32_of(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int t = (int)(hi & 0x7fffffffu) - 0x38000000;   // exponent from bias 1023 to bias 127
+    unsigned b = __funnelshift_l(lo, (unsigned)t, 3);
+    if (t < 0) b = 0u;
+    if (t >= 0x0ff00000) b = 0x7f800000u;
+    return __uint_as_float(b | (hi & 0x80000000u));
+}
+
+// grid_pos (the reference's floor((x - wo) / cs) in FP64) from an FP32
+// estimate: where the estimate is farther from a cell face than its error
+// bound it has the same integer part, and elsewhere (about one coordinate in
+// 4,000 on a 128-cell axis, or a value that is not finite) the FP64 division
+// decides.  Bound: x is cut by 2^-23 of itself, wo rounded by 2^-24, and the
+// difference, the product and the reciprocal round by 2^-24 each.
+__device__ __forceinline__ int cell_of(const Params& P, double x, int a)
+{
+    const float xf = f32_of(x), q = (xf - P.wof[a]) * P.inv_csf, f = floorf(q);
+    const float e = (fabsf(xf) + fabsf(P.wof[a])) * P.inv_csf * 5e-7f;
+    if (q - f > e && f + 1.0f - q > e && fabsf(q) < 1e6f) return (int)f;
+    return (int)floor((x - P.wo[a]) / P.cs);
+}
+__device__ __forceinline__ int3 grid_pos_fast(const Params& P, double x, double y, double z)
+{
+    return make_int3(cell_of(P, x, 0), cell_of(P, y, 1), cell_of(P, z, 2));
+}
+
+// One warp's buffer for P particles of 32 / P lanes each: the runs of sorted
+// slots that their cells cover, the partners found (k-th of particle o at
+// [k * P + o]), the order in which they are taken, and NR values of result
+// per lane.
+template <int LP, typename Real, int NR>
+struct ScanBuf {
+    static constexpr int kParticles = 32 / LP;
+    static constexpr int kSlots = LP == 1 ? 16 : 24;
+    uint2 run[27][kParticles];
+    Real res[NR][32];
+    unsigned cand[kSlots * kParticles];
+    unsigned short slot[kSlots * kParticles];
+    unsigned short pos[kSlots * kParticles];
+};
+
+// The cells of lane group o's particle (cell gp, when valid) into run[][o]:
+// the sorted slots of its 27 cells in search order (x fastest), empty cells
+// left out and cells whose slots follow on from the one before joined to it.
+// hash(x, y, z): a cell's number.  Returns the number of runs.
+template <int LP, typename Buf, typename Hash>
+__device__ __forceinline__ unsigned stage_runs(Buf& B, bool valid, int3 gp, const unsigned* __restrict__ cstart,
+                                               const unsigned* __restrict__ cend, Hash hash)
+{
+    const unsigned lane = threadIdx.x & 31u, o = lane / LP, sub = lane % LP;
+    constexpr int kEach = (27 + LP - 1) / LP;
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        const int c = q * LP + (int)sub;
+        if (valid && c < 27) {
+            const unsigned h = hash(gp.x + c % 3 - 1, gp.y + (c / 3) % 3 - 1, gp.z + c / 9 - 1);
+            const unsigned st = __ldg(cstart + h);
+            B.run[c][o] = make_uint2(st, st == 0xffffffffu ? st : __ldg(cend + h));
+        }
+    }
+    __syncwarp();
+    unsigned n = 0;
+    if (valid && sub == 0) {
+        uint2 cur = make_uint2(0u, 0u);
+        for (int c = 0; c < 27; ++c) {
+            const uint2 b = B.run[c][o];
+            if (b.x >= b.y) continue;
+            if (b.x == cur.y && cur.x != cur.y) {
+                cur.y = b.y;
+            } else {
+                if (cur.x != cur.y) B.run[n++][o] = cur;
+                cur = b;
+            }
+        }
+        if (cur.x != cur.y) B.run[n++][o] = cur;
+    }
+    n = __shfl_sync(kFullWarp, n, (int)(o * LP));
+    __syncwarp();
+    return n;
+}
+
+// The warp's contacts.  near(k, o): whether entry k of the sorted list may
+// touch particle o (never false for one that does).  eval(o, k, lane): the
+// law of that pair, its result into B.res[][lane]; returns a code, 0 for no
+// contact.  add(code, lane): the result in B.res[][lane] to the sums of the
+// calling lane's particle; lane o adds particle o's, in search order.
+//
+// Each round collects partners until a particle's slots could overflow, then
+// takes them level by level (every particle's first, then every particle's
+// second, ...), 32 at a time: a group of 32 then holds one or two of most
+// particles and the adding runs on most lanes.
+template <int LP, typename Buf, typename Near, typename Eval, typename Add>
+__device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsigned* __restrict__ sorted, Near near,
+                                              Eval eval, Add add)
+{
+    constexpr unsigned P = 32 / LP, U = LP == 1 ? 4u : (LP == 4 ? 2u : 1u), S = Buf::kSlots;
+    const unsigned lane = threadIdx.x & 31u, o = lane / LP, sub = lane % LP;
+    const unsigned group = LP == 32 ? kFullWarp : ((1u << LP) - 1u) << (o * LP);
+    unsigned r = 0, j = 0, e = 0;
+    bool more = nruns != 0u;
+    if (more) {
+        const uint2 b = B.run[0][o];
+        j = b.x;
+        e = b.y;
+    }
+    while (true) {
+        unsigned cnt = 0;
+        while (true) {
+            const bool act = more && cnt + LP * U <= S;
+            if (!__any_sync(kFullWarp, act)) break;
+            unsigned k[U];
+            bool in[U];
+#pragma unroll
+            for (unsigned u = 0; u < U; ++u) {
+                const unsigned jj = j + u * LP + sub;
+                in[u] = act && jj < e;
+                k[u] = in[u] ? __ldg(sorted + jj) : 0u;
+            }
+#pragma unroll
+            for (unsigned u = 0; u < U; ++u) in[u] = in[u] && near(k[u], o);
+#pragma unroll
+            for (unsigned u = 0; u < U; ++u) {
+                if (LP == 1) {
+                    if (in[u]) B.cand[cnt++ * P + o] = k[u];
+                } else {
+                    const unsigned b = __ballot_sync(kFullWarp, in[u]) & group;
+                    if (in[u]) B.cand[(cnt + __popc(b & ((1u << lane) - 1u))) * P + o] = k[u];
+                    cnt += __popc(b);
+                }
+            }
+            if (act) {
+                j += LP * U;
+                if (j >= e) {
+                    more = ++r < nruns;
+                    if (more) {
+                        const uint2 b = B.run[r][o];
+                        j = b.x;
+                        e = b.y;
+                    }
+                }
+            }
+        }
+        // lane o < P owns particle o
+        const unsigned mine = LP == 1 ? cnt : __shfl_sync(kFullWarp, cnt, (int)((lane * LP) & 31u));
+        const unsigned own = lane < P ? mine : 0u;
+        const unsigned levels = __reduce_max_sync(kFullWarp, own);
+        unsigned total = 0;
+        for (unsigned l = 0; l < levels; ++l) {
+            const unsigned b = __ballot_sync(kFullWarp, own > l);
+            if (own > l) {
+                const unsigned p = total + __popc(b & ((1u << lane) - 1u));
+                B.slot[p] = (unsigned short)(l * P + lane);
+                B.pos[l * P + lane] = (unsigned short)p;
+            }
+            total += __popc(b);
+        }
+        __syncwarp();
+        unsigned done = 0;
+        for (unsigned base = 0; base < total; base += 32u) {
+            if (base + lane < total) {
+                const unsigned s = B.slot[base + lane];
+                B.cand[s] = eval(s % P, B.cand[s], lane);
+            }
+            __syncwarp();
+            for (; done < own; ++done) {
+                const unsigned p = B.pos[done * P + lane];
+                if (p >= base + 32u) break;
+                const unsigned code = B.cand[done * P + lane];
+                if (code) add(code, p - base);
+            }
+            __syncwarp();
+        }
+        if (!__any_sync(kFullWarp, more)) return;
+    }
+}
+
+// Lanes per particle of a scan over np particles.  A warp of 32 particles
+// scans the candidates of each in turn, which is the least work; below about
+// four waves' worth of such warps the chip is not full and more lanes per
+// particle shorten the chain of loads and of contacts that one warp goes
+// through.
+inline int scan_lanes(unsigned np) { return np >= 48000u ? 1 : (np >= 16000u ? 4 : 8); }
+
+// Blocks of two warps for it: at most one wave (eight blocks an SM), whose
+// warps then take several groups of particles and form the contact
+// property's constants once.
+inline unsigned scan_blocks(unsigned np, int lp)
+{
+    const unsigned groups = div_up(np, 32u / (unsigned)lp), blocks = div_up(groups, 2u);
+    return blocks < 152u * 8u ? blocks : 152u * 8u;
+}
+
+}  // namespace xd

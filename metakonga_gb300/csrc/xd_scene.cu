@@ -951,6 +951,7 @@ int xd_scene_set_particle_grid(xd_scene* s, const unsigned grid[3], double cell_
     s->Pp.ncell = (unsigned)nc;
     s->Pp.cs = cell_size;
     for (int a = 0; a < 3; ++a) s->Pp.wo[a] = origin[a];
+    set_cell_estimate(s->Pp);
     s->split = true;
     return XD_OK;
 }
