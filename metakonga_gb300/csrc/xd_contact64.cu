@@ -453,12 +453,188 @@ int launch_cylinder(const Params& P, const xd_cylinder_info* cyl, const xd_conta
 
 __device__ __forceinline__ d3 ldp(const double* a) { return mk(__ldg(a), __ldg(a + 1), __ldg(a + 2)); }
 
-// Reaction on the polygon bodies: NB > 0 keeps per-thread sums for NB
-// bodies and reduces them per block in a fixed order (block partials are
-// summed by k_polygon_reaction_final); NB == 0 adds with atomics (used when
-// the caller does not say how many bodies there are).
-template <int NB, bool HIST>
-__global__ void __launch_bounds__(128) k_polygon(Params P, const xd_polygon_info* __restrict__ dpi,
+// Whether a sphere may touch triangle t: its box, then its FP32 distance,
+// each against the radius with a margin above the rounding of the world
+// coordinates (2^-23 of each) and of the region test.  A triangle so thin that the FP32 region test could go astray
+// (sin^2 of the angle at P below 1e-3) counts as near, as does a value that
+// is not finite.
+__device__ __forceinline__ bool triangle_near(const Near4& p, const xd_polygon_info* __restrict__ t)
+{
+    const float ax = f32_of(__ldg(t->P)), ay = f32_of(__ldg(t->P + 1)), az = f32_of(__ldg(t->P + 2));
+    const float bx = f32_of(__ldg(t->Q)), by = f32_of(__ldg(t->Q + 1)), bz = f32_of(__ldg(t->Q + 2));
+    const float cx = f32_of(__ldg(t->R)), cy = f32_of(__ldg(t->R + 1)), cz = f32_of(__ldg(t->R + 2));
+    const float size = fabsf(ax) + fabsf(ay) + fabsf(az) + fabsf(bx) + fabsf(by) + fabsf(bz) + fabsf(cx) +
+                       fabsf(cy) + fabsf(cz);
+    const float reach = p.r * 1.00001f + (size + p.size) * 1e-6f + 1e-15f;
+    if (fminf(ax, fminf(bx, cx)) - p.x > reach || p.x - fmaxf(ax, fmaxf(bx, cx)) > reach) return false;
+    if (fminf(ay, fminf(by, cy)) - p.y > reach || p.y - fmaxf(ay, fmaxf(by, cy)) > reach) return false;
+    if (fminf(az, fminf(bz, cz)) - p.z > reach || p.z - fmaxf(az, fmaxf(bz, cz)) > reach) return false;
+    const float ux = bx - ax, uy = by - ay, uz = bz - az, vx = cx - ax, vy = cy - ay, vz = cz - az;
+    const float uu = ux * ux + uy * uy + uz * uz, vv = vx * vx + vy * vy + vz * vz;
+    const float uv = ux * vx + uy * vy + uz * vz;
+    if (!(uu * vv - uv * uv > 1e-3f * uu * vv && uu * vv > 1e-30f)) return true;
+    bool face;
+    const float d2 = tri_dist2_f(ax - p.x, ay - p.y, az - p.z, bx - p.x, by - p.y, bz - p.z, cx - p.x, cy - p.y,
+                                 cz - p.z, face);
+    const float lim = reach + 1e-4f * (sqrtf(uu) + sqrtf(vv));
+    return !(d2 > lim * lim);
+}
+
+// particle_polygonObject_collision_kernel<1> (impl:923-1021), a warp for
+// 32 / LP particles.
+//
+// A mesh's cells are as large as its triangles: here a particle's 27 cells
+// hold a thousand particles and a hundred triangles or none, and few
+// triangles touch it.  Entries are tested in FP32 (triangle_near) and the
+// FP64 closest point and law run on those that pass, one per lane, each
+// particle adding its own in search order (xd_scan.cuh).  A bed of 17,159
+// spheres on a cone of 4,096 triangles: 136 us, 3,512 with the closest point
+// of every triangle in the cells formed in FP64 by a thread per particle.
+//
+// Reaction on the polygon bodies: NB > 0 keeps sums for NB bodies, summed per
+// warp over all its particles by a fixed shuffle tree and over the warps by
+// k_polygon_reaction_final; NB == 0 adds with atomics (used when the caller
+// does not say how many bodies there are).
+enum { kMoment = 4u, kBodyShift = 3u };
+
+template <int NB, int LP>
+__global__ void __launch_bounds__(64) k_polygon(Params P, const xd_polygon_info* __restrict__ dpi,
+                                                xd_polygon_mass_info* __restrict__ dpmi,
+                                                const double* __restrict__ pos, const double* __restrict__ vel,
+                                                const double* __restrict__ omega, double* __restrict__ force,
+                                                double* __restrict__ moment, const double* __restrict__ mass,
+                                                const unsigned* __restrict__ sorted,
+                                                const unsigned* __restrict__ cstart,
+                                                const unsigned* __restrict__ cend,
+                                                const xd_contact_property* __restrict__ cp,
+                                                double* __restrict__ partials)
+{
+    using Buf = ScanBuf<LP, double, 12>;
+    __shared__ Buf bufs[2];
+    Buf& B = bufs[threadIdx.x / 32u];
+    constexpr int NBR = NB > 0 ? NB : 1;
+    constexpr unsigned NP = 32 / LP;
+    double react[NBR][6];
+#pragma unroll
+    for (int b = 0; b < NBR; ++b)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) react[b][q] = 0.0;
+    bool reacted = false;
+    const unsigned cnp = P.np, lane = threadIdx.x & 31u;
+    const unsigned warp = blockIdx.x * 2u + threadIdx.x / 32u;
+    const unsigned groups = (cnp + NP - 1u) / NP;
+    for (unsigned g = warp; g < groups; g += gridDim.x * 2u) {
+        const unsigned id0 = g * NP, id = id0 + lane / LP;
+        const bool valid = id < cnp;
+        d4 ip = d4{ 0, 0, 0, 0 };
+        int3 gp = make_int3(0, 0, 0);
+        if (valid) {
+            ip = ld4(pos, id);
+            gp = grid_pos_fast(P, ip.x, ip.y, ip.z);
+        }
+        const Near4 mine = near_of(ip);
+        const unsigned runs = stage_runs<LP>(B, valid, gp, cstart, cend,
+                                             [&](int x, int y, int z) { return grid_hash(P, x, y, z); });
+        d3 Ft = mk(0, 0, 0), sumF = mk(0, 0, 0), sumM = mk(0, 0, 0);
+        bool touched = false;
+        scan_contacts<LP>(
+            B, runs, sorted,
+            [&](unsigned k, unsigned) { return k >= cnp && triangle_near(mine, dpi + (k - cnp)); },
+            // values: Fn + Ft, Ft and the reaction's moment, or without slip Fn, -- and the contact point
+            // from the body's origin; then M, where it is not zero (a normal that is not a number)
+            [&](unsigned o, unsigned k, unsigned l) {
+                const unsigned i = id0 + o;
+                const xd_polygon_info* tri = dpi + (k - cnp);
+                const d4 a = ld4(pos, i);
+                const d3 ipos = xyz(a);
+                const d3 Pv = ldp(tri->P), Qv = ldp(tri->Q), Rv = ldp(tri->R);
+                const d3 cpt = closest_pt_triangle(Pv, Qv, Rv, ipos);
+                const double dist = length(ipos - cpt);
+                const double cdist = a.w - dist;
+                if (!(cdist > 0)) return 0u;
+                const unsigned pidx = (unsigned)__ldg(&tri->id);
+                const xd_polygon_mass_info* pmi = dpmi + pidx;
+                const d3 po2cp = cpt - ldv(pmi->origin);
+                const d3 ivel = ld3(vel, i), iomega = ld3(omega, i);
+                d3 unit = -cross(Qv - Pv, Rv - Pv);
+                unit = unit / length(unit);
+                const d3 pvel = ldv(pmi->vel), pom = ldv(pmi->omega);
+                const d3 dv = P.rolling ? (pvel + cross(pom, po2cp)) - (ivel + cross(iomega, a.w * unit))
+                                        : (pvel - ivel);
+                const PairConst pc = load_pair_const(cp + pidx);
+                const Fc c = get_constant(pc, a.w, 0, __ldg(mass + i), 0);
+                d3 Fn, t = mk(0, 0, 0), m = mk(0, 0, 0);
+                const bool slip = dhs(c, 0, 0, 0, 0, 0, 0, 0, cdist, dv, unit, P.dt, t, Fn, m);
+                unsigned code = kContact | (pidx << kBodyShift);
+                if (slip) {
+                    code |= kSlip;
+                    put3(B.res, 0, l, Fn + t);
+                    put3(B.res, 3, l, t);
+                    put3(B.res, 6, l, -cross(po2cp, Fn + t));
+                    if (m.x != 0.0 || m.y != 0.0 || m.z != 0.0) {
+                        code |= kMoment;
+                        put3(B.res, 9, l, m);
+                    }
+                } else {
+                    put3(B.res, 0, l, Fn);
+                    put3(B.res, 6, l, po2cp);
+                }
+                return code;
+            },
+            [&](unsigned code, unsigned l) {
+                d3 t = get3(B.res, 0, l), rm = get3(B.res, 6, l);
+                if (code & kSlip) {
+                    Ft = get3(B.res, 3, l);
+                } else {
+                    t = t + Ft;
+                    rm = -cross(rm, t);
+                }
+                sumF += t;
+                if (code & kMoment) sumM += get3(B.res, 9, l);
+                touched = true;
+                const unsigned pidx = code >> kBodyShift;
+                if (NB == 0 || pidx >= (unsigned)NBR) {
+                    // body count not declared, or an id beyond it: no slot, add directly
+                    atomicAdd(dpmi[pidx].force + 0, -t.x);
+                    atomicAdd(dpmi[pidx].force + 1, -t.y);
+                    atomicAdd(dpmi[pidx].force + 2, -t.z);
+                    atomicAdd(dpmi[pidx].moment + 0, rm.x);
+                    atomicAdd(dpmi[pidx].moment + 1, rm.y);
+                    atomicAdd(dpmi[pidx].moment + 2, rm.z);
+                    return;
+                }
+#pragma unroll
+                for (int b = 0; b < NBR; ++b)
+                    if ((unsigned)b == pidx) {
+                        react[b][0] -= t.x; react[b][1] -= t.y; react[b][2] -= t.z;
+                        react[b][3] += rm.x; react[b][4] += rm.y; react[b][5] += rm.z;
+                    }
+            });
+        const unsigned me = id0 + lane;
+        if (touched) {   // lanes that own a particle; the others add zero
+            st3(force, me, ld3rw(force, me) + sumF);
+            st3(moment, me, ld3rw(moment, me) + sumM);
+            reacted = true;
+        }
+    }
+    if (NB > 0) {
+        const bool any = __any_sync(kFullWarp, reacted);
+#pragma unroll
+        for (int b = 0; b < NBR; ++b)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                double v = react[b][q];
+                if (any)
+                    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(kFullWarp, v, o);
+                if (lane == 0) partials[((size_t)warp * NBR + b) * 6 + q] = v;
+            }
+    }
+}
+
+// The same with tangential history, a thread per particle; the reactions
+// summed by block (the tables are read and written contact by contact).
+template <int NB>
+__global__ void __launch_bounds__(128) k_polygon_hist(Params P, const xd_polygon_info* __restrict__ dpi,
                                                  xd_polygon_mass_info* __restrict__ dpmi,
                                                  const double* __restrict__ pos,
                                                  const double* __restrict__ vel,
@@ -492,7 +668,7 @@ __global__ void __launch_bounds__(128) k_polygon(Params P, const xd_polygon_info
         d3 M = mk(0, 0, 0), Fn = mk(0, 0, 0), Ft = mk(0, 0, 0);
         d3 sum_force = mk(0, 0, 0), sum_moment = mk(0, 0, 0);
         HistState hs;
-        if (HIST) hist_begin(ht, id, hs);
+        hist_begin(ht, id, hs);
         for (int z = -1; z <= 1; z++)
             for (int y = -1; y <= 1; y++)
                 for (int x = -1; x <= 1; x++) {
@@ -523,15 +699,11 @@ __global__ void __launch_bounds__(128) k_polygon(Params P, const xd_polygon_info
                                               : (pvel - ivel);
                             PairConst pc = load_pair_const(cp + pidx);
                             Fc c = get_constant(pc, ir, 0, im, 0);
-                            if (HIST) {
-                                Fn = normal_force(c, 0, 0, 0, 0, 0, 0, 0, cdist, dv, unit);
-                                d3 d;
-                                int sl = hist_slot(ht, hs, id, kHistTri | k, d);
-                                hist_tangential(c, 0.0, dv, unit, P.dt, Fn, d, Ft, M);
-                                hist_store(ht, sl, id, d);
-                            } else {
-                                dhs(c, 0, 0, 0, 0, 0, 0, 0, cdist, dv, unit, P.dt, Ft, Fn, M);
-                            }
+                            Fn = normal_force(c, 0, 0, 0, 0, 0, 0, 0, cdist, dv, unit);
+                            d3 d;
+                            int sl = hist_slot(ht, hs, id, kHistTri | k, d);
+                            hist_tangential(c, 0.0, dv, unit, P.dt, Fn, d, Ft, M);
+                            hist_store(ht, sl, id, d);
                             sum_force += Fn + Ft;
                             sum_moment += M;
                             d3 rf = -(Fn + Ft);
@@ -562,7 +734,7 @@ __global__ void __launch_bounds__(128) k_polygon(Params P, const xd_polygon_info
                         }
                     }
                 }
-        if (HIST) hist_end(ht, hs, id, 2u);
+        hist_end(ht, hs, id, 2u);
         double* f = force + 3 * (size_t)id;
         double* m = moment + 3 * (size_t)id;
         f[0] += sum_force.x; f[1] += sum_force.y; f[2] += sum_force.z;
@@ -585,19 +757,26 @@ __global__ void __launch_bounds__(128) k_polygon(Params P, const xd_polygon_info
     }
 }
 
-// Sums the block partials of each body in block order and adds the total to
-// dpmi[b].force / .moment.
-__global__ void k_polygon_reaction_final(const double* __restrict__ partials, unsigned nblocks,
-                                         unsigned nbodies, unsigned nbr,
-                                         xd_polygon_mass_info* __restrict__ dpmi)
+// Sums the partials of each body (of a warp, or of a block with history) in a
+// fixed order and adds the total to dpmi[b].force / .moment: a block per
+// component, so that its FP64 additions run on an SM of their own; thread t
+// takes partials t, t + 128, ..., then a shuffle tree and the warps in order.
+__global__ void __launch_bounds__(128) k_polygon_reaction_final(const double* __restrict__ partials, unsigned count,
+                                                                unsigned nbr,
+                                                                xd_polygon_mass_info* __restrict__ dpmi)
 {
-    unsigned t = threadIdx.x;   // one thread per (body, component)
-    if (t >= nbodies * 6) return;
-    unsigned b = t / 6, q = t % 6;
+    __shared__ double part[4];
+    const unsigned b = blockIdx.x / 6u, q = blockIdx.x % 6u;
     double s = 0.0;
-    for (unsigned blk = 0; blk < nblocks; ++blk) s += partials[((size_t)blk * nbr + b) * 6 + q];
-    if (q < 3) dpmi[b].force[q] += s;
-    else dpmi[b].moment[q - 3] += s;
+#pragma unroll 4
+    for (unsigned k = threadIdx.x; k < count; k += 128u) s += partials[((size_t)k * nbr + b) * 6 + q];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(kFullWarp, s, o);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x / 32u] = s;
+    __syncthreads();
+    if (threadIdx.x) return;
+    s = (part[0] + part[1]) + (part[2] + part[3]);
+    if (q < 3u) dpmi[b].force[q] += s;
+    else dpmi[b].moment[q - 3u] += s;
 }
 
 // ----------------------------------------------------------- mesh update
@@ -772,11 +951,13 @@ static unsigned nbr_for(unsigned nbodies)
     return 8;
 }
 
+// Partials of the reaction: one per warp of the scan, or per block with history.
 size_t polygon_scratch_bytes(unsigned np, unsigned nbodies)
 {
-    unsigned nbr = nbr_for(nbodies);
+    const unsigned nbr = nbr_for(nbodies);
     if (nbr == 0) return 0;
-    return sizeof(double) * 6 * (size_t)nbr * div_up(np ? np : 1u, 128);
+    const unsigned parts = div_up(np ? np : 1u, 128);
+    return sizeof(double) * 6 * (size_t)nbr * (parts > kScanWarps ? parts : kScanWarps);
 }
 
 int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_info* dpmi,
@@ -787,17 +968,21 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
 {
     unsigned np = P.np;
     if (np == 0) return XD_OK;
-    unsigned nb = div_up(np, 128);
-    unsigned nbr = nbr_for(nbodies);
+    const unsigned nbr = nbr_for(nbodies);
+    const int lp = scan_lanes(np);
+    const unsigned nb = ht ? div_up(np, 128) : scan_blocks(np, lp);
     double* part = static_cast<double*>(scratch);
-#define XD_POLY(NBV)                                                                              \
-    do {                                                                                          \
-        if (ht)                                                                                   \
-            k_polygon<NBV, true><<<nb, 128, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, \
-                                                    mass, sidx, cstart, cend, cp, part, *ht);     \
-        else                                                                                      \
-            k_polygon<NBV, false><<<nb, 128, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, \
-                                                     mass, sidx, cstart, cend, cp, part, HistTable{}); \
+#define XD_POLY_LP(NBV, LP)                                                                                   \
+    k_polygon<NBV, LP><<<nb, 64, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, sidx, cstart, cend, \
+                                         cp, part)
+#define XD_POLY(NBV)                                                                                          \
+    do {                                                                                                      \
+        if (ht)                                                                                               \
+            k_polygon_hist<NBV><<<nb, 128, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, sidx,   \
+                                                   cstart, cend, cp, part, *ht);                              \
+        else if (lp == 1) XD_POLY_LP(NBV, 1);                                                                 \
+        else if (lp == 4) XD_POLY_LP(NBV, 4);                                                                 \
+        else XD_POLY_LP(NBV, 8);                                                                              \
     } while (0)
     switch (nbr) {
     case 0: XD_POLY(0); break;
@@ -807,9 +992,10 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
     default: XD_POLY(8); break;
     }
 #undef XD_POLY
+#undef XD_POLY_LP
     int st = launch_status("particle_polygon_collision");
     if (st != XD_OK || nbr == 0) return st;
-    k_polygon_reaction_final<<<1, 64, 0, s>>>(part, nb, nbodies, nbr, dpmi);
+    k_polygon_reaction_final<<<6 * nbodies, 128, 0, s>>>(part, ht ? nb : 2u * nb, nbr, dpmi);
     return launch_status("particle_polygon_collision (reaction)");
 }
 

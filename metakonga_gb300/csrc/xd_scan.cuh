@@ -200,19 +200,23 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
 }
 
 // Lanes per particle of a scan over np particles.  A warp of 32 particles
-// scans the candidates of each in turn, which is the least work; below about
-// four waves' worth of such warps the chip is not full and more lanes per
-// particle shorten the chain of loads and of contacts that one warp goes
-// through.
-inline int scan_lanes(unsigned np) { return np >= 48000u ? 1 : (np >= 16000u ? 4 : 8); }
+// fills its lanes best (131 contacts of a bed in five groups); with few
+// particles the chip is not full and more lanes shorten the chain of loads
+// and contacts that one warp goes through.  FP64 pairs, us with 1 / 4 / 8
+// lanes: a bed of 2,000 spheres 77 / 35 / 26, 8,000 77 / 54 / 54, 17,000
+// 97 / 85 / 94, 60,000 197 / 238 / 285, 120,989 349 / 461 / 556; on a mesh's
+// wide cells 17,159 591 / 216 / 251 and 60,000 2,018 / 1,809 / 2,253, for
+// which the upper line lies above where a bed alone would put it (30,000).
+inline int scan_lanes(unsigned np) { return np >= 48000u ? 1 : (np >= 10000u ? 4 : 8); }
 
 // Blocks of two warps for it: at most one wave (eight blocks an SM), whose
 // warps then take several groups of particles and form the contact
 // property's constants once.
+constexpr unsigned kScanWarps = 152u * 8u * 2u;
 inline unsigned scan_blocks(unsigned np, int lp)
 {
     const unsigned groups = div_up(np, 32u / (unsigned)lp), blocks = div_up(groups, 2u);
-    return blocks < 152u * 8u ? blocks : 152u * 8u;
+    return blocks < kScanWarps / 2u ? blocks : kScanWarps / 2u;
 }
 
 }  // namespace xd
