@@ -14,7 +14,7 @@ struct HistTable;   // xd_physics64.cuh: tangential-spring history of a scene
 
 int launch_hash(const Params& P, unsigned* hash, unsigned* index, const double* pos, unsigned n,
                 unsigned sid, cudaStream_t s);
-int launch_fill_cells(unsigned* cstart, unsigned* cend, unsigned ncell, cudaStream_t s);
+int launch_fill_cells(unsigned* cstart, unsigned* cend, unsigned ncell, cudaStream_t s, unsigned* err = nullptr);
 // The cell ranges of n keys already sorted in hash (with their values in
 // index): cstart/cend at the runs' ends, sorted_index = index; a key >= ncell
 // is skipped and raises *err.  Cells without keys are left as they are.

@@ -139,9 +139,16 @@ void* workspace(size_t bytes, int* status);
 
 inline unsigned div_up(unsigned a, unsigned b) { return (a + b - 1) / b; }
 
-// radix sort (xd_sort.cu): keys per tile (8 warps x 4 rounds x 32 lanes)
-constexpr unsigned kSortTile = 1024;
+// radix sort (xd_sort.cu): keys per tile, so that a sort has 65 to 128 tiles
+// from 2^16 to 2^20 keys: enough to fill the chip, and few enough that their
+// digit counts (2,048 a tile, 1 MB up to 2^20 keys) stay small beside the keys.
+__host__ __device__ constexpr unsigned sort_tile(unsigned n)
+{
+    return n <= (1u << 17) ? 1024u : (n <= (1u << 18) ? 2048u : (n <= (1u << 19) ? 4096u : 8192u));
+}
 size_t radix_sort_scratch_bytes(unsigned n);
+// Kernel launches of one sort.
+unsigned radix_sort_launches(unsigned n, unsigned key_bits);
 int radix_sort_pairs(unsigned* keys, unsigned* vals, unsigned n, unsigned key_bits, void* scratch,
                      cudaStream_t s, unsigned** out_keys, unsigned** out_vals);
 

@@ -248,7 +248,6 @@ struct MixedScene {
     unsigned* hkey2 = nullptr;
     double* hdelta2 = nullptr;
     unsigned long long* hoverflow = nullptr;
-    unsigned passes = 0;          // radix passes of one re-binning
     bool use_graphs = true;
     bool kinematic = false;   // bodies moved by their own vel and omega every step
     unsigned rec_cap_alloc = 0;
@@ -2888,7 +2887,6 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
     A(alloc(s, &s->prec, s->nplanes));
     A(alloc(s, &s->cps, s->nplanes));
     A(alloc(s, &s->counters, kCounters));
-    s->passes = (key_bits_for(s->ncell) + 7) / 8;
     if (st == XD_OK) A(cuda_status(cudaMemset(s->counters, 0, sizeof(unsigned) * kCounters), "mixed counters"));
     if (st == XD_OK && s->nplanes) {
         A(cuda_status(cudaMemcpy(s->planes, d.planes, sizeof(xd_plane_info) * s->nplanes, cudaMemcpyHostToDevice), "mixed planes"));
@@ -3606,8 +3604,9 @@ unsigned long long mixed_rebuild_launches(MixedScene* s)
     // keys, sort, permute, copy back, cell bounds (2), list build; with
     // triangles also their lists, and for a mesh that moves on the device
     // its cell table (count, scan, fill, pad and their sort)
-    unsigned long long k = (s->n > 1 ? 5ull * s->passes : 0ull) + 6;
-    if (s->ntri) k += 1 + (s->kinematic ? 4 + 5ull * ((key_bits_for(s->ncell + 1) + 7) / 8) : 0ull);
+    unsigned long long k = radix_sort_launches(s->n, key_bits_for(s->ncell)) + 6ull;
+    if (s->ntri)
+        k += 1 + (s->kinematic ? 4ull + radix_sort_launches(s->tpair_cap, key_bits_for(s->ncell + 1)) : 0ull);
     if (s->nbodies) k += 1;   // the reactions flushed first
     return k;
 }

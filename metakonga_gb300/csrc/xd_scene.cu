@@ -676,10 +676,9 @@ unsigned long long xd_scene_launches(xd_scene* s, unsigned nsteps)
     if (!s || nsteps == 0) return 0;
     if (s->mixed) return mixed_launches(s->mixed, nsteps);
     unsigned ng = s->np + s->ntri;
-    unsigned passes = (key_bits_for(s->ncell) + 7) / 8;
     unsigned long long per = 0;
     per += 1 + (s->ntri ? 1 : 0);                 // hash (+ triangle spheres)
-    per += ng > 1 ? 5ull * passes : 0;            // radix sort
+    per += radix_sort_launches(ng, key_bits_for(s->ncell));   // sort
     per += 2;                                     // fill + cell bounds
     per += 1;                                     // particle-particle
     per += s->nplanes ? 1 : 0;                    // planes
