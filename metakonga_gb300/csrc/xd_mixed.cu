@@ -73,7 +73,6 @@ constexpr unsigned kContactMaxThreads = 128;   // the largest block size a scene
 constexpr unsigned kContactMode = 1;           // default pair pass: warp-cooperative
 constexpr unsigned kContactWarpsTotal = 152 * 16;   // warps of a full contact grid (every SM, 16 warps each)
 constexpr int kMaxBodies = 8;                  // polygon bodies of a mixed scene
-constexpr unsigned kGuardBit = 0x80000000u;    // list entry decided by the FP64 test
 
 // Counter words.
 enum {
@@ -936,33 +935,12 @@ __device__ __forceinline__ int exact_touch(const MixParams& P, const Master& M, 
     return exact_touch_q<COUNT>(P, M, i, j, qai, qbi, __ldg(qa + j), __ldg(qb + j), counters);
 }
 
-// The candidate test of pair (i, j): FP32 prefilter, then the exact test.
-template <bool COUNT>
-__device__ __forceinline__ int touch(const MixParams& P, const Master& M, unsigned i, unsigned j,
-                                     const float4& pi, const longlong2& qai, const longlong2& qbi,
-                                     const float4* __restrict__ pf, const longlong2* __restrict__ qa,
-                                     const longlong2* __restrict__ qb, unsigned* __restrict__ counters)
-{
-    const float4 pj = __ldg(pf + j);
-    const float dxf = pj.x - pi.x, dyf = pj.y - pi.y, dzf = pj.z - pi.z;
-    const float Rt = pi.w + P.tol + pj.w;
-    if (fmaf(dxf, dxf, fmaf(dyf, dyf, dzf * dzf)) >= Rt * Rt) return 0;
-    return exact_touch<COUNT>(P, M, i, j, qai, qbi, qa, qb, counters);
-}
-
-// Visits the contacts of slot i in the reference's order (neighbour rows z
-// then y, each row's slots ascending): fn(j, guard) for every touching j.
-// Candidates pass an FP32 prefilter, then the exact integer test; pairs in
-// the guard band are decided by fp64_cdist.
-template <bool COUNT, typename Fn>
-__device__ __forceinline__ void for_each_contact(const MixParams& P, const Master& M, unsigned i,
-                                                 const float4& pi, const longlong2& qai,
-                                                 const longlong2& qbi, unsigned key,
-                                                 const float4* __restrict__ pf,
-                                                 const longlong2* __restrict__ qa,
-                                                 const longlong2* __restrict__ qb,
-                                                 const unsigned* __restrict__ lb,
-                                                 unsigned* __restrict__ counters, Fn fn)
+// Visits the candidates of slot i in the reference's order (neighbour rows z
+// then y, each row's slots ascending): fn(j) for every j != i whose FP32
+// distance is below r_j + rt0.
+template <typename Fn>
+__device__ __forceinline__ void for_each_near(const MixParams& P, unsigned i, const float4& pi, float rt0, unsigned key,
+                                              const float4* __restrict__ pf, const unsigned* __restrict__ lb, Fn fn)
 {
     // row (dz, dy) starts at cell key - 1 + dy gx + dz gx gy; the next row's
     // bounds are loaded while this row's candidates are visited
@@ -978,13 +956,45 @@ __device__ __forceinline__ void for_each_contact(const MixParams& P, const Maste
         }
         for (unsigned j = s; j < e; ++j) {
             if (j == i) continue;
-            const int t = touch<COUNT>(P, M, i, j, pi, qai, qbi, pf, qa, qb, counters);
-            if (t) fn(j, t == 2);
+            const float4 pj = __ldg(pf + j);
+            const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            const float Rt = rt0 + pj.w;
+            if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) >= Rt * Rt) continue;
+            fn(j);
         }
         s = sn;
         e = en;
         c0 = c1;
     }
+}
+
+// Visits the contacts of slot i in that order: fn(j, guard) for every
+// touching j.  Candidates pass an FP32 prefilter, then the exact integer
+// test; pairs in the guard band are decided by fp64_cdist.
+template <bool COUNT, typename Fn>
+__device__ __forceinline__ void for_each_contact(const MixParams& P, const Master& M, unsigned i,
+                                                 const float4& pi, const longlong2& qai,
+                                                 const longlong2& qbi, unsigned key,
+                                                 const float4* __restrict__ pf,
+                                                 const longlong2* __restrict__ qa,
+                                                 const longlong2* __restrict__ qb,
+                                                 const unsigned* __restrict__ lb,
+                                                 unsigned* __restrict__ counters, Fn fn)
+{
+    for_each_near(P, i, pi, pi.w + P.tol, key, pf, lb, [&](unsigned j) {
+        const int t = exact_touch<COUNT>(P, M, i, j, qai, qbi, qa, qb, counters);
+        if (t) fn(j, t == 2);
+    });
+}
+
+// Radius of particle i plus the most that the FP32 distance of its view to
+// another's can be off: a coordinate is within 2^-23 of itself of the FP64
+// one (the conversion rounds its high part and its sum), so the distance is
+// off by less than 2^-22 of the sum of i's coordinates (the partner's are its
+// own, but for a diameter); the squares round by 2^-21 of the radii.
+__device__ __forceinline__ float near_reach(const MixParams& P, const float4& pi)
+{
+    return pi.w + ((fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z)) * 3e-7f + (pi.w + P.rmaxf) * 2e-6f + 1e-10f);
 }
 
 constexpr unsigned kIncomplete = 0x80000000u;   // vcount flag: the list is not complete
@@ -1299,6 +1309,21 @@ struct Own {
     float4 pr;     // residuals of its fixed-point position and radius (metres)
 };
 
+// The partner's data a contact reads.
+struct Partner {
+    longlong2 qa, qb;
+    float4 pr, vh, vl, wh;
+    float r;
+};
+
+__device__ __forceinline__ Partner load_partner(const Master& M, unsigned j, const float4* __restrict__ pf,
+                                                const longlong2* __restrict__ qa, const longlong2* __restrict__ qb,
+                                                const float4* __restrict__ pr)
+{
+    return Partner{ __ldg(qa + j),   __ldg(qb + j),   __ldg(pr + j),    __ldg(M.vh + j),
+                    __ldg(M.vl + j), __ldg(M.wh + j), __ldg(pf + j).w };
+}
+
 // When an FP32 contact force term is re-formed in FP64.  The per-particle
 // force error is judged against max(sum_c |F_c|, m g); each contact's FP32
 // error is kept below kForceTol of its own scale max(|Fn|, m g), so that the
@@ -1339,17 +1364,14 @@ __device__ __forceinline__ bool slip_needs_fp64(float wt, float ee, float lin, f
 // warp-cooperative pass sums them in list order afterwards; see accumulate).
 template <int HIST, bool OUT = false>
 __device__ __forceinline__ void contact_force(const MixParams& P, const Master& M, const Own& I,
-                                              unsigned j, bool guard, const double* __restrict__ mass0,
-                                              const float4* __restrict__ pf,
-                                              const longlong2* __restrict__ qa,
-                                              const longlong2* __restrict__ qb,
-                                              const float4* __restrict__ pr,
+                                              unsigned j, const Partner& J, bool guard,
+                                              const double* __restrict__ mass0,
                                               unsigned* __restrict__ counters, PairAcc& A,
                                               const HistTable& ht, HistState& hs, PairOut* o = nullptr)
 {
     const unsigned i = I.i;
     const float dt = P.dtf;
-    const longlong2 qaj = __ldg(qa + j), qbj = __ldg(qb + j);
+    const longlong2 qaj = J.qa, qbj = J.qb;
     const long long ddx = qaj.x - I.qa.x, ddy = qaj.y - I.qa.y, ddz = qbj.x - I.qb.x;
     const long long D2 = ddx * ddx + ddy * ddy + ddz * ddz;
     const float D2f = (float)D2;
@@ -1380,13 +1402,13 @@ __device__ __forceinline__ void contact_force(const MixParams& P, const Master& 
     // The fixed point's residuals restore the FP64 positions: the overlap
     // gains (e_ri + e_rj) - u . (e_j - e_i) (the 2^-36 m grid alone would move
     // a light contact's overlap by up to ~3e-11 m, a part in 1e5 of 3e-6 m)
-    const float4 ej = __ldg(pr + j);
+    const float4 ej = J.pr;
     const f3 de = fk(ej.x - I.pr.x, ej.y - I.pr.y, ej.z - I.pr.z);
     const float ude = fdot(u, de);
     if (!guard) delta += (I.pr.w + ej.w) - ude;
-    const float4 vj4 = __ldg(M.vh + j), vjl = __ldg(M.vl + j), wj4 = __ldg(M.wh + j);
+    const float4 vj4 = J.vh, vjl = J.vl, wj4 = J.wh;
     const f3 wj = fk(wj4.x, wj4.y, wj4.z);
-    const float jr = __ldg(pf + j).w, jim = vj4.w;
+    const float jr = J.r, jim = vj4.w;
     const float ir = I.r;
     // vj - vi formed exactly from the double-float velocities
     float dvs[3], dvt[3];
@@ -1956,7 +1978,7 @@ __device__ __forceinline__ void contact_entry(const MixParams& P, const ContactA
             I.pr = __ldg(C.pr + i);
             have_v = true;
         }
-        contact_force<HIST>(P, M, I, j, guard, mass0, pf, qa, qb, C.pr, counters, A, ht, hs);
+        contact_force<HIST>(P, M, I, j, load_partner(M, j, pf, qa, qb, C.pr), guard, mass0, counters, A, ht, hs);
         if (RECORD && nc < rec_cap) rec_pairs[(size_t)i * rec_cap + nc] = j;
         ++nc;
     };
@@ -2153,19 +2175,23 @@ __device__ __forceinline__ void contact_entry(const MixParams& P, const ContactA
 //
 // In a packed bed every listed particle has several contacts, and a thread
 // per particle leaves most lanes idle while the warp runs the longest list.
-// Here the 32 particles of a warp are done together in rounds.  Each lane
-// first scans its own particle's Verlet list (or its cells) and keeps up to
-// kCoopSlots touching partners in shared memory; then the warp's partners,
-// level by level (every lane's first, then every lane's second, ...), are
-// spread over the lanes, one contact per lane, each forming its contact's
-// force with contact_force; and each particle's lane adds its own contacts'
-// terms in its list order (accumulate).  With the contacts by level, a group
+// Here the particles of a warp (32, or fewer: run_size) are done together in
+// rounds.  Each lane first scans its own particle's Verlet list (or its cells)
+// by FP32 distance and keeps up to kCoopSlots partners that may touch in
+// shared memory; then the warp's partners, level by level (every lane's first,
+// then every lane's second, ...), are spread over the lanes, one per lane,
+// each decided by the exact test and its force formed with contact_force; and
+// each particle's lane adds its own contacts' terms in its list order
+// (accumulate).  With the contacts by level, a group
 // of 32 holds one or two of most particles, so the adding is spread over
 // the lanes instead of running on a few of them.  The sums are
 // therefore the same bits as the per-particle pass's.  A lane with more
 // than kCoopSlots contacts goes on in the next round where it stopped.
 
 constexpr unsigned kCoopSlots = 16;
+// List entries that a lane loads together (a 199,583-sphere bed's pass 62 us;
+// 66 with four at a time and the exact test, three times the bytes, in the scan).
+constexpr unsigned kScanAtOnce = 8;
 
 struct CoopBuf {
     unsigned cand[32 * kCoopSlots];   // k-major: lane L's k-th candidate at [k * 32 + L]
@@ -2208,19 +2234,25 @@ __device__ __forceinline__ unsigned level_order(PairBuf& PB, unsigned cnt, unsig
 // the partners before `done` skipped, up to kCoopSlots after them kept in
 // mine[0], mine[32], ...; returns whether more are left.  Out of line:
 // rare, and the pass's loop stays short.
-__device__ __noinline__ bool coop_cells(const MixParams& P, const ContactArgs& C, unsigned i, float4 pi,
-                                        longlong2 qai, longlong2 qbi, unsigned& done, unsigned* mine,
-                                        unsigned& cnt)
+__device__ __noinline__ bool coop_cells(const MixParams& P, const ContactArgs& C, unsigned i, float4 pi, float rt0,
+                                        unsigned& done, unsigned* mine, unsigned& cnt)
 {
     unsigned seen = 0;
-    for_each_contact<true>(P, C.M, i, pi, qai, qbi, __ldg(C.keys + i), C.pf, C.qa, C.qb, C.lb, C.counters,
-                           [&](unsigned j, bool guard) {
-                               if (seen >= done && cnt < kCoopSlots)
-                                   mine[32u * cnt++] = j | (guard ? kGuardBit : 0u);
-                               ++seen;
-                           });
+    for_each_near(P, i, pi, rt0, __ldg(C.keys + i), C.pf, C.lb, [&](unsigned j) {
+        if (seen >= done && cnt < kCoopSlots) mine[32u * cnt++] = j;
+        ++seen;
+    });
     done += cnt;
     return seen > done;
+}
+
+// A read-only load issued where it stands: the compiler otherwise moves the
+// loads of a batch behind the branches that use them, one after another.
+__device__ __forceinline__ float4 load_now(const float4* p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
 }
 
 // Own data of slot i as contact_force reads it.
@@ -2252,13 +2284,11 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
     const unsigned n = P.n;
     float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
     unsigned vc = 0;
-    longlong2 qai = make_longlong2(0, 0), qbi = make_longlong2(0, 0);
     if (valid) {
         pi = __ldg(C.pf + i);
         vc = __ldg(C.vcount + i);
-        qai = __ldg(C.qa + i);
-        qbi = __ldg(C.qb + i);
     }
+    const float rt0 = near_reach(P, pi);
     const bool incomplete = (vc & kIncomplete) != 0u;
     PairAcc A;
     A.Ft = fk(0.f, 0.f, 0.f);
@@ -2274,37 +2304,28 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
         unsigned cnt = 0;
         if (more) {
             if (!incomplete) {
-                const float rt0 = pi.w + P.tol;
-                // four list entries at a time, their loads issued together
-                // (the partner's view and fixed point are loaded whether or
-                // not the prefilter passes: most entries touch in a bed)
+                // kScanAtOnce list entries at a time, their loads issued together
                 while (kpos < vc && cnt < kCoopSlots) {
-                    unsigned jj[4];
-                    float4 pp[4];
-                    longlong2 aa[4], bb[4];
+                    unsigned jj[kScanAtOnce];
+                    float4 pp[kScanAtOnce];
 #pragma unroll
-                    for (unsigned q = 0; q < 4u; ++q)
+                    for (unsigned q = 0; q < kScanAtOnce; ++q)
                         jj[q] = kpos + q < vc ? __ldg(C.vlist + (size_t)(kpos + q) * n + i) : i;
 #pragma unroll
-                    for (unsigned q = 0; q < 4u; ++q) {
-                        pp[q] = __ldg(C.pf + jj[q]);
-                        aa[q] = __ldg(C.qa + jj[q]);
-                        bb[q] = __ldg(C.qb + jj[q]);
-                    }
+                    for (unsigned q = 0; q < kScanAtOnce; ++q) pp[q] = load_now(C.pf + jj[q]);
 #pragma unroll
-                    for (unsigned q = 0; q < 4u; ++q) {
+                    for (unsigned q = 0; q < kScanAtOnce; ++q) {
                         if (kpos >= vc || cnt >= kCoopSlots) break;
                         ++kpos;
                         const float dx = pp[q].x - pi.x, dy = pp[q].y - pi.y, dz = pp[q].z - pi.z;
                         const float Rt = rt0 + pp[q].w;
                         if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) >= Rt * Rt) continue;
-                        const int c = exact_touch_q<true>(P, C.M, i, jj[q], qai, qbi, aa[q], bb[q], C.counters);
-                        if (c) mine[32u * cnt++] = jj[q] | (c == 2 ? kGuardBit : 0u);
+                        mine[32u * cnt++] = jj[q];
                     }
                 }
                 more = kpos < vc;
             } else {
-                more = coop_cells(P, C, i, pi, qai, qbi, done, mine, cnt);
+                more = coop_cells(P, C, i, pi, rt0, done, mine, cnt);
             }
         }
         __syncwarp();
@@ -2316,22 +2337,25 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
             const unsigned sc = c < total ? PB.slot[c] : 0u;
             const unsigned iL = __shfl_sync(0xffffffffu, i, sc & 31u);
             if (c < total) {
-                const unsigned e = B.cand[sc];
+                const unsigned j = B.cand[sc];
                 const Own I = load_own(P, C, iL);
+                const Partner J = load_partner(C.M, j, C.pf, C.qa, C.qb, C.pr);
+                const int t = exact_touch_q<true>(P, C.M, iL, j, I.qa, I.qb, J.qa, J.qb, C.counters);
                 PairOut o;
-                contact_force<0, true>(P, C.M, I, e & ~kGuardBit, (e & kGuardBit) != 0u, C.mass0, C.pf, C.qa,
-                                       C.qb, C.pr, C.counters, A, C.ht, hs, &o);
-                B.res[0][lane] = o.Fn.x;
-                B.res[1][lane] = o.Fn.y;
-                B.res[2][lane] = o.Fn.z;
-                B.res[9][lane] = o.slip ? 1.f : 0.f;
-                if (o.slip) {
-                    B.res[3][lane] = o.Ft.x;
-                    B.res[4][lane] = o.Ft.y;
-                    B.res[5][lane] = o.Ft.z;
-                    B.res[6][lane] = o.Mm.x;
-                    B.res[7][lane] = o.Mm.y;
-                    B.res[8][lane] = o.Mm.z;
+                if (t) contact_force<0, true>(P, C.M, I, j, J, t == 2, C.mass0, C.counters, A, C.ht, hs, &o);
+                B.res[9][lane] = !t ? -1.f : (o.slip ? 1.f : 0.f);
+                if (t) {
+                    B.res[0][lane] = o.Fn.x;
+                    B.res[1][lane] = o.Fn.y;
+                    B.res[2][lane] = o.Fn.z;
+                    if (o.slip) {
+                        B.res[3][lane] = o.Ft.x;
+                        B.res[4][lane] = o.Ft.y;
+                        B.res[5][lane] = o.Ft.z;
+                        B.res[6][lane] = o.Mm.x;
+                        B.res[7][lane] = o.Mm.y;
+                        B.res[8][lane] = o.Mm.z;
+                    }
                 }
             }
             __syncwarp();
@@ -2340,9 +2364,11 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
                 const unsigned p = PB.pos[kacc * 32u + lane];
                 if (p >= base + 32u) break;
                 const unsigned k = p - base;
+                const float code = B.res[9][k];
+                if (code < 0.f) continue;   // near, not touching
                 PairOut o;
                 o.Fn = fk(B.res[0][k], B.res[1][k], B.res[2][k]);
-                o.slip = B.res[9][k] != 0.f;
+                o.slip = code != 0.f;
                 if (o.slip) {
                     o.Ft = fk(B.res[3][k], B.res[4][k], B.res[5][k]);
                     o.Mm = fk(B.res[6][k], B.res[7][k], B.res[8][k]);
@@ -2411,8 +2437,18 @@ __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const Conta
         unsigned cnt = 0;
         for (; more && wm && cnt < kCoopSlots; wm &= wm - 1u)
             mine[32u * cnt++] = kWallPlane | (unsigned)(__ffs(wm) - 1);
-        for (; more && kb < ke && cnt < kCoopSlots; ++kb)
-            mine[32u * cnt++] = listed ? __ldg(C.tlist + (size_t)kb * n + i) : __ldg(C.tpt + kb);
+        while (more && kb < ke && cnt < kCoopSlots) {   // four ids at a time, their loads issued together
+            unsigned t[4];
+#pragma unroll
+            for (unsigned q = 0; q < 4u; ++q)
+                if (kb + q < ke) t[q] = listed ? __ldg(C.tlist + (size_t)(kb + q) * n + i) : __ldg(C.tpt + kb + q);
+#pragma unroll
+            for (unsigned q = 0; q < 4u; ++q)
+                if (kb < ke && cnt < kCoopSlots) {
+                    mine[32u * cnt++] = t[q];
+                    ++kb;
+                }
+        }
         more = more && (wm || kb < ke);
         __syncwarp();
         const unsigned total = level_order(WB.c, cnt, lane);
@@ -2460,16 +2496,28 @@ __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const Conta
     C.Fc[i] = F;
 }
 
+// Listed particles that a warp of a cooperative pass takes at a time: 32,
+// which fill its lanes with contacts best, or 16 or 8 where `total` of them
+// would leave warps without any -- a run is a chain of loads and of groups of
+// 32 contacts, and a short list's pass lasts as long as one run.  With runs of
+// 32 always, us a step: 8,000 spheres' pairs and walls 24 (16 with this), the
+// walls of a 199,583-sphere hopper (1,000 spheres near its cone) 24 (16.5),
+// of twelve hoppers in a batch 106 (35).
+__host__ __device__ __forceinline__ unsigned run_size(unsigned total, unsigned warps)
+{
+    return total <= warps * 8u ? 8u : (total <= warps * 16u ? 16u : 32u);
+}
+
 __global__ void __launch_bounds__(kContactMaxThreads) k_mx_walls(MixParams P, ContactArgs C)
 {
     extern __shared__ WallBuf wall_buf[];
     WallBuf& B = wall_buf[threadIdx.x / 32u];
     const unsigned front = C.counters[CN_HTRI];
-    const unsigned warps = gridDim.x * (blockDim.x / 32u);
-    const unsigned gw = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
-    for (unsigned t0 = gw * 32u; t0 < front; t0 += warps * 32u) {
-        const unsigned t = t0 + (threadIdx.x & 31u);
-        const bool valid = t < front;
+    const unsigned warps = gridDim.x * (blockDim.x / 32u), run = run_size(front, warps);
+    const unsigned gw = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u, lane = threadIdx.x & 31u;
+    for (unsigned t0 = gw * run; t0 < front; t0 += warps * run) {
+        const unsigned t = t0 + lane;
+        const bool valid = lane < run && t < front;
         walls_entry_coop(P, C, valid, valid ? __ldg(C.hlist + t) : 0u, B);
     }
 }
@@ -2481,16 +2529,17 @@ __global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, 
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) C.counters[CN_REBUILD] = 0;
     const unsigned total = C.counters[CN_HEAVY], front = C.counters[CN_HTRI];
-    // runs of 32 consecutive list entries go to the warps of all blocks in
-    // turn: every SM gets an equal share however short the list
+    // runs of consecutive list entries go to the warps of all blocks in turn:
+    // every SM gets an equal share however short the list
     const unsigned warps = gridDim.x * (blockDim.x / 32u);
     const unsigned gw = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
     if (COOP) {
         extern __shared__ PairBuf pair_buf[];
         PairBuf& B = pair_buf[threadIdx.x / 32u];
-        for (unsigned t0 = gw * 32u; t0 < total; t0 += warps * 32u) {
-            const unsigned t = t0 + (threadIdx.x & 31u);
-            const bool valid = t < total;
+        const unsigned run = run_size(total, warps), lane = threadIdx.x & 31u;
+        for (unsigned t0 = gw * run; t0 < total; t0 += warps * run) {
+            const unsigned t = t0 + lane;
+            const bool valid = lane < run && t < total;
             contact_entry_coop(P, C, valid, valid ? __ldg(C.hlist + list_index(t, front, P.n)) : 0u, B);
         }
         return;
@@ -3431,9 +3480,10 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
     if (st != XD_OK) return st;
     s->cells_clean = true;
     ph.begin(3, q);
-    // the list holds at most n particles: no more warps than that
-    const unsigned ct = s->cthreads;
-    const unsigned grid = std::max(1u, std::min(kContactWarpsTotal * 32u / ct, (n + ct - 1) / ct));
+    // the list holds at most n particles: no more warps than there are runs of
+    // 8 of them (of 32 in the per-particle pass)
+    const unsigned ct = s->cthreads, each = s->cmode == 1 ? ct / 4u : ct;
+    const unsigned grid = std::max(1u, std::min(kContactWarpsTotal * 32u / ct, (n + each - 1) / each));
     // tangential springs: updated by a step, read only by the diagnostic evaluation (MODE 3)
     const HistTable ht = history_table(s);
     const int hist = s->hslots ? (MODE == 3 ? 2 : 1) : 0;
@@ -3922,7 +3972,7 @@ namespace {
 
 constexpr unsigned kBatchGroup = 32;
 constexpr unsigned kBatchGraphSteps = 4;   // later steps captured per graph launch
-constexpr unsigned kBatchGrab = 2;         // runs of 32 listed particles a contact warp takes at a time
+constexpr unsigned kBatchGrab = 2;         // runs of 32 listed particles that a contact warp takes at a time
 
 
 // One scene of a batch as the batch kernels read it.
@@ -4001,19 +4051,29 @@ __global__ void k_batch_group(const unsigned* __restrict__ flags, unsigned first
     if (t < count && flags[first + t]) cudaGraphSetConditional(hs[first + t], 1u);
 }
 
-// Runs of 32 listed particles per scene, as an exclusive prefix over scenes,
-// of counter word `cw` (CN_HEAVY: every listed particle; CN_HTRI: those with
-// walls in reach) into runs[0, ns]; runs[ns + 1] (the launch's next free
-// run) cleared.
+// Runs of listed particles per scene, as an exclusive prefix over scenes, of
+// counter word `cw` (CN_HEAVY: every listed particle; CN_HTRI: those with
+// walls in reach) into runs[0, ns]; runs[ns + 1] (the launch's next free run)
+// cleared, and the particles a run holds (run_size of all scenes' together)
+// in runs[ns + 2].
 __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsigned cw, unsigned* __restrict__ runs,
                            unsigned* c, unsigned& carry)
 {
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
+    unsigned all = 0;
+    for (unsigned sc = threadIdx.x; sc < ns; sc += 1024u) all += D[sc].C.counters[cw];
+    all = __reduce_add_sync(0xffffffffu, all);
+    if ((threadIdx.x & 31u) == 0 && all) atomicAdd(&carry, all);
+    __syncthreads();
+    const unsigned run = run_size(carry, kContactWarpsTotal);
+    __syncthreads();
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
     for (unsigned base = 0; base < ns; base += 1024u) {
         const unsigned sc = base + threadIdx.x;
         const unsigned h = sc < ns ? D[sc].C.counters[cw] : 0u;
-        c[threadIdx.x] = (h + 31u) / 32u;
+        c[threadIdx.x] = (h + run - 1u) / run;
         __syncthreads();
         // inclusive scan (Hillis-Steele)
         for (unsigned off = 1; off < 1024u; off <<= 1) {
@@ -4030,23 +4090,24 @@ __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsign
     if (threadIdx.x == 0) {
         runs[0] = 0;
         runs[ns + 1] = 0;
+        runs[ns + 2] = run;
     }
     __syncthreads();
 }
 
 // The runs of the contact launch (chunk_start) and of the wall launch
-// (chunk_start + ns + 2).
+// (chunk_start + ns + 3).
 __global__ void __launch_bounds__(1024) k_batch_chunks(const BatchScene* __restrict__ D, unsigned ns,
                                                        unsigned* __restrict__ chunk_start)
 {
     __shared__ unsigned c[1024];
     __shared__ unsigned carry;
     batch_runs(D, ns, CN_HEAVY, chunk_start, c, carry);
-    batch_runs(D, ns, CN_HTRI, chunk_start + ns + 2, c, carry);
+    batch_runs(D, ns, CN_HTRI, chunk_start + ns + 3, c, carry);
 }
 
 // The contact pass of every scene: each warp takes the next kBatchGrab runs
-// of all scenes' lists from a counter (chunk_start[ns + 1], cleared by
+// (one, where runs are short) of all scenes' lists from a counter (chunk_start[ns + 1], cleared by
 // k_batch_chunks) until none are left, so that warps that drew cheap runs
 // take more; a run's result does not depend on which warp computes it.  A
 // warp loads the scene of a run into its own shared-memory slot when the
@@ -4072,13 +4133,14 @@ __global__ void __launch_bounds__(kContactMaxThreads) k_batch_contact(const Batc
     unsigned char* const bufs = batch_smem + batch_scene_bytes(nwarps);
     const unsigned total = __ldg(chunk_start + ns);
     unsigned* next = chunk_start + ns + 1;
+    const unsigned run = __ldg(chunk_start + ns + 2), grab = run == 32u ? kBatchGrab : 1u;
     unsigned cur = 0xffffffffu, lo = 0, heavy = 0, front = 0;
     for (;;) {
     unsigned c0 = 0;
-    if (lane == 0) c0 = atomicAdd(next, kBatchGrab);
+    if (lane == 0) c0 = atomicAdd(next, grab);
     c0 = __shfl_sync(0xffffffffu, c0, 0);
     if (c0 >= total) break;
-    const unsigned c1 = min(total, c0 + kBatchGrab);
+    const unsigned c1 = min(total, c0 + grab);
     for (unsigned ch = c0; ch < c1; ++ch) {
         if (cur == 0xffffffffu || ch >= __ldg(chunk_start + cur + 1)) {
             // the scene holding run ch: the last s with chunk_start[s] <= ch
@@ -4097,16 +4159,16 @@ __global__ void __launch_bounds__(kContactMaxThreads) k_batch_contact(const Batc
             heavy = W.C.counters[CN_HEAVY];
             front = W.C.counters[CN_HTRI];
         }
-        const unsigned t = (ch - lo) * 32u + lane;
+        const unsigned t = (ch - lo) * run + lane;
         if (KIND == 1) {
-            const bool valid = t < heavy;
+            const bool valid = lane < run && t < heavy;
             contact_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + list_index(t, front, W.P.n)) : 0u,
                                reinterpret_cast<PairBuf*>(bufs)[wb]);
         } else if (KIND == 2) {
-            const bool valid = t < front;
+            const bool valid = lane < run && t < front;
             walls_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + t) : 0u,
                              reinterpret_cast<WallBuf*>(bufs)[wb]);
-        } else if (t < heavy) {
+        } else if (lane < run && t < heavy) {
             contact_entry<false, 0>(W.P, W.C, __ldg(W.C.hlist + list_index(t, front, W.P.n)));
         }
     }
@@ -4159,7 +4221,7 @@ static void launch_batch_walls(const MixedBatch* b, unsigned ns, cudaStream_t q)
     const unsigned ct = b->cthreads, grid = kContactWarpsTotal * 32u / ct, w = ct / 32u;
     if (b->cmode == 1 && b->walls)
         k_batch_contact<2><<<grid, ct, batch_scene_bytes(w) + w * sizeof(WallBuf), q>>>(b->d_scenes, ns,
-                                                                                         b->d_chunks + ns + 2);
+                                                                                         b->d_chunks + ns + 3);
 }
 
 static void launch_batch_contact(const MixedBatch* b, unsigned ns, cudaStream_t q)
@@ -4382,7 +4444,7 @@ int prepare_batch(MixedBatch* b)
     M(&b->d_scenes, ns, "batch scenes");
     M(&b->d_block_scene, block_scene.size(), "batch blocks");
     M(&b->d_flags, ns, "batch flags");
-    M(&b->d_chunks, 2 * (ns + 2), "batch runs");
+    M(&b->d_chunks, 2 * (ns + 3), "batch runs");
     M(&b->d_handles[0], ng + ns, "batch handles");
     M(&b->d_handles[1], ng + ns, "batch handles");
     M(&b->d_handles[2], (size_t)(ng + ns) * kBatchGraphSteps, "batch handles");
