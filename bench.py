@@ -1051,8 +1051,9 @@ def run_batched(a):
     con_ms = pair_ms + wall_ms
     # what a step costs beyond its two big kernels (the decision kernel, run
     # prefix, graph and conditional nodes, and the re-binnings): the most a
-    # persistent batch kernel could save
-    other_ms = ms / a.steps - adv_ms - con_ms
+    # persistent batch kernel could save.  The step graphs run the wall runs
+    # beside the pair runs in one launch, kernel timing one after the other.
+    other_ms = max(0.0, ms / a.steps - adv_ms - con_ms)
     adv_gbs = n_tot * B_ADVANCE / (adv_ms / 1e3) / 1e9
     con_gbs = contact_bytes / (con_ms / 1e3) / 1e9
     adv_traffic = _traffic_from_profiles("advance_batch_hopper.md", "traffic_bytes_per_particle")
@@ -1088,8 +1089,7 @@ def run_batched(a):
     # per step: advance, decision, run prefix and contact over all scenes; per
     # call the finish and each scene's body-reaction sum; per re-binning its
     # kernels and its group's decision kernel
-    walls_pass = 1 if tunings[0].get("contact_mode", 1) == 1 else 0   # the cooperative pass's wall launch
-    launches = ((4 + walls_pass) * a.steps + 1 + sum(1 for sc in scs if sc.ntri)
+    launches = (4 * a.steps + 1 + sum(1 for sc in scs if sc.ntri)
                 + sum((b[0] - r[0]) * (b[1] + 1) for r, b in zip(rb0, rb1)))
 
     # e2e: every scene's state uploaded from pinned host memory, K steps, the

@@ -184,8 +184,9 @@ struct MixedScene {
     longlong2* qa = nullptr;
     longlong2* qb = nullptr;
     float4* pr = nullptr;         // quantisation residuals of x, y, z and r (metres)
-    float4* Fc = nullptr;
+    float4* Fc = nullptr;         // contact force; .w nonzero: the walls' part is in Fw
     float4* Mc = nullptr;
+    float4* Fw = nullptr;         // wall force (the cooperative pass's wall runs)
     // Verlet lists (slots of the current cell order, rebuilt with the cells)
     unsigned* hlist = nullptr;    // particles with neighbours or planes in reach
     unsigned short* wmask = nullptr;   // planes in reach of each particle
@@ -702,12 +703,26 @@ __device__ __forceinline__ double drift(const MixParams& P, double x, float vhi,
 // that does not sets CN_REBUILD.  The last block to finish passes the flag to
 // the graph's conditional node (use_cond), one caller as the conditional
 // requires.
+// The contact force of slot i: the pairs' and, where its .w says so, the walls'.
+__device__ __forceinline__ float4 contact_sum(const float4* __restrict__ Fc, const float4* __restrict__ Fw, unsigned i)
+{
+    float4 f = Fc[i];
+    if (f.w != 0.f) {
+        const float4 w = Fw[i];
+        f.x += w.x;
+        f.y += w.y;
+        f.z += w.z;
+    }
+    return f;
+}
+
 // One slot of the advance (MODE 0: drift; MODE 1: kick with the last
 // contact forces, then drift), its contact view, and whether it has left half
 // the skin since the last build.
 template <int MODE>
 __device__ __forceinline__ bool advance_one(const MixParams& P, const Master& M, const float4* __restrict__ Fc,
-                                            const float4* __restrict__ Mc, const float4* __restrict__ pref,
+                                            const float4* __restrict__ Mc, const float4* __restrict__ Fw,
+                                            const float4* __restrict__ pref,
                                             float4* __restrict__ pf, longlong2* __restrict__ qa,
                                             longlong2* __restrict__ qb, float4* __restrict__ pr,
                                             const unsigned i)
@@ -719,7 +734,7 @@ __device__ __forceinline__ bool advance_one(const MixParams& P, const Master& M,
         if (MODE == 1) {
             float4 wh = M.wh[i], wl = M.wl[i];
             float2 b2 = M.b2[i];
-            kick(P, vh, vl, wh, wl, ab, b2, Fc[i], Mc[i]);
+            kick(P, vh, vl, wh, wl, ab, b2, contact_sum(Fc, Fw, i), Mc[i]);
             M.vh[i] = vh;
             M.vl[i] = vl;
             M.wh[i] = wh;
@@ -742,7 +757,7 @@ __device__ __forceinline__ bool advance_one(const MixParams& P, const Master& M,
 
 template <int MODE>
 __global__ void __launch_bounds__(256) k_mx_advance(MixParams P, Master M, const float4* __restrict__ Fc,
-                                                    const float4* __restrict__ Mc,
+                                                    const float4* __restrict__ Mc, const float4* __restrict__ Fw,
                                                     const float4* __restrict__ pref,
                                                     float4* __restrict__ pf, longlong2* __restrict__ qa,
                                                     longlong2* __restrict__ qb, float4* __restrict__ pr,
@@ -751,7 +766,7 @@ __global__ void __launch_bounds__(256) k_mx_advance(MixParams P, Master M, const
 {
     __shared__ bool last;
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool out = i < P.n && advance_one<MODE>(P, M, Fc, Mc, pref, pf, qa, qb, pr, i);
+    const bool out = i < P.n && advance_one<MODE>(P, M, Fc, Mc, Fw, pref, pf, qa, qb, pr, i);
     // only the flag must be visible to the last block: the lanes that set it
     // fence; the state and view writes need no ordering here
     if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) {
@@ -824,11 +839,12 @@ __global__ void __launch_bounds__(256) k_mx_copyback(MixParams P, Master S, Mast
 
 // MODE 2: velocity only, in place (the last step of a call).
 __device__ __forceinline__ void finish_one(const MixParams& P, const Master& M, const float4* __restrict__ Fc,
-                                           const float4* __restrict__ Mc, const unsigned i)
+                                           const float4* __restrict__ Mc, const float4* __restrict__ Fw,
+                                           const unsigned i)
 {
     float4 vh = M.vh[i], vl = M.vl[i], wh = M.wh[i], wl = M.wl[i], ab = M.ab[i];
     float2 b2 = M.b2[i];
-    kick(P, vh, vl, wh, wl, ab, b2, Fc[i], Mc[i]);
+    kick(P, vh, vl, wh, wl, ab, b2, contact_sum(Fc, Fw, i), Mc[i]);
     M.vh[i] = vh;
     M.vl[i] = vl;
     M.wh[i] = wh;
@@ -838,10 +854,10 @@ __device__ __forceinline__ void finish_one(const MixParams& P, const Master& M, 
 }
 
 __global__ void __launch_bounds__(256) k_mx_finish(MixParams P, Master M, const float4* __restrict__ Fc,
-                                                   const float4* __restrict__ Mc)
+                                                   const float4* __restrict__ Mc, const float4* __restrict__ Fw)
 {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < P.n) finish_one(P, M, Fc, Mc, i);
+    if (i < P.n) finish_one(P, M, Fc, Mc, Fw, i);
 }
 
 // ---- cell lower bounds -----------------------------------------------------
@@ -1588,6 +1604,7 @@ struct ContactArgs {
     double* rxn;
     float4* Fc;
     float4* Mc;
+    float4* Fw;
     unsigned* counters;
     unsigned* rec_count;
     unsigned* rec_pairs;
@@ -2274,10 +2291,10 @@ __device__ __forceinline__ Own load_own(const MixParams& P, const ContactArgs& C
 }
 
 // The contact pass of list entries (valid lanes: slot i) without tangential
-// history, every lane of the warp taking part: pairs cooperatively, then
-// each particle's planes and triangles (walls_fp32) by its own lane.
+// history, every lane of the warp taking part.  walls: the particle has walls
+// in reach, whose force a wall run leaves in Fw.
 __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const ContactArgs& C, bool valid, unsigned i,
-                                                   PairBuf& PB)
+                                                   bool walls, PairBuf& PB)
 {
     CoopBuf& B = PB.c;
     const unsigned lane = threadIdx.x & 31u;
@@ -2379,25 +2396,29 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
         }
     }
     if (!valid) return;
-    // the walls are added by the wall pass (walls_entry)
-    C.Fc[i] = make_float4(A.sumF.x, A.sumF.y, A.sumF.z, 0.f);
+    // the walls' part comes from a wall run (walls_entry_coop), into Fw
+    C.Fc[i] = make_float4(A.sumF.x, A.sumF.y, A.sumF.z, walls ? 1.f : 0.f);
     C.Mc[i] = make_float4(A.sumM.x, A.sumM.y, A.sumM.z, 0.f);
 }
 
-// The wall pass after the cooperative pair pass, warp-cooperative as well:
-// the listed particles with walls in reach (the front of the list) list
-// their wall candidates (planes in reach, then their triangles) into the
-// warp's buffer, the candidates are spread one per lane in level order
-// (level_order, wall_eval), and
-// each particle's lane adds its results in candidate order (wall_add) and
-// then its wall force to its pair force -- the additions the per-particle
-// pass makes after its pairs (F += walls).  A launch of its own: the wall
-// code's FP64 region tests and registers stay out of the pair pass.
-// The wall pass's shared memory per warp: the candidate buffer, and each
-// lane's particle data read once by its own lane for all its candidates.
+// The walls beside the cooperative pairs, warp-cooperative as well: the listed
+// particles with walls in reach (the front of the list) list their wall
+// candidates (planes in reach, then their triangles) into the warp's buffer,
+// the candidates are spread one per lane in level order (level_order,
+// wall_eval), and each particle's lane adds its results in candidate order
+// (wall_add).  The sum goes to Fw, and whoever reads the contact force adds it
+// to the pairs' (contact_sum), the addition the per-particle pass makes after
+// its pairs: so pairs and walls need no order between them and share a launch,
+// in which the few wall runs, each a long chain of FP64 region tests, run
+// beside the pairs' instead of after them.
+//
+// A wall run holds kWallRun particles, whose data their lanes write to shared
+// memory once for all their candidates.
+constexpr unsigned kWallRun = 8;
+
 struct WallBuf {
     PairBuf c;
-    WallOwn own[32];
+    WallOwn own[kWallRun];
 };
 
 __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const ContactArgs& C, bool valid, unsigned i,
@@ -2427,7 +2448,7 @@ __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const Conta
         }
     }
     const bool any = wm || kb < ke;
-    if (any) WB.own[lane] = load_wall_own(P, C, i);
+    if (any) WB.own[lane] = load_wall_own(P, C, i);   // lane < kWallRun
     f3 f = fk(0.f, 0.f, 0.f), Ftri = fk(0.f, 0.f, 0.f);
     RxnAcc ra;
     ra.b = 0xffffffffu;
@@ -2487,43 +2508,26 @@ __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const Conta
             __syncwarp();
         }
     }
-    if (!valid || !any) return;
+    if (!valid) return;
     rxn_flush(C, n, i, ra);
-    float4 F = C.Fc[i];
-    F.x += f.x;
-    F.y += f.y;
-    F.z += f.z;
-    C.Fc[i] = F;
+    C.Fw[i] = make_float4(f.x, f.y, f.z, 0.f);
 }
 
-// Listed particles that a warp of a cooperative pass takes at a time: 32,
-// which fill its lanes with contacts best, or 16 or 8 where `total` of them
-// would leave warps without any -- a run is a chain of loads and of groups of
-// 32 contacts, and a short list's pass lasts as long as one run.  With runs of
-// 32 always, us a step: 8,000 spheres' pairs and walls 24 (16 with this), the
-// walls of a 199,583-sphere hopper (1,000 spheres near its cone) 24 (16.5),
-// of twelve hoppers in a batch 106 (35).
+// Listed particles that a warp of the cooperative pair pass takes at a time:
+// 32, which fill its lanes with contacts best, or 16 or 8 where `total` of
+// them would leave warps without any -- a run is a chain of loads and of groups
+// of 32 contacts, and a short list's pass lasts as long as one run.  With runs
+// of 32 always, 8,000 spheres' pairs and walls took 24 us a step (16 with this).
 __host__ __device__ __forceinline__ unsigned run_size(unsigned total, unsigned warps)
 {
     return total <= warps * 8u ? 8u : (total <= warps * 16u ? 16u : 32u);
 }
 
-__global__ void __launch_bounds__(kContactMaxThreads) k_mx_walls(MixParams P, ContactArgs C)
-{
-    extern __shared__ WallBuf wall_buf[];
-    WallBuf& B = wall_buf[threadIdx.x / 32u];
-    const unsigned front = C.counters[CN_HTRI];
-    const unsigned warps = gridDim.x * (blockDim.x / 32u), run = run_size(front, warps);
-    const unsigned gw = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u, lane = threadIdx.x & 31u;
-    for (unsigned t0 = gw * run; t0 < front; t0 += warps * run) {
-        const unsigned t = t0 + lane;
-        const bool valid = lane < run && t < front;
-        walls_entry_coop(P, C, valid, valid ? __ldg(C.hlist + t) : 0u, B);
-    }
-}
-
-// COOP: the warp-cooperative pair pass (no history, no recording; dynamic
-// shared memory of one PairBuf per warp).
+// COOP: the warp-cooperative passes (no history, no recording; dynamic shared
+// memory of one WallBuf per warp): the wall runs first, from the first warp
+// on, and the pair runs from the last warp on, so that the warps with a wall
+// run are those with the fewest pair runs.  A 199,583-sphere hopper 62 us a
+// step (62 and, after them, 16.5 with the walls in a launch of their own).
 template <bool RECORD, int HIST, bool COOP>
 __global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, ContactArgs C)
 {
@@ -2534,13 +2538,19 @@ __global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, 
     const unsigned warps = gridDim.x * (blockDim.x / 32u);
     const unsigned gw = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
     if (COOP) {
-        extern __shared__ PairBuf pair_buf[];
-        PairBuf& B = pair_buf[threadIdx.x / 32u];
-        const unsigned run = run_size(total, warps), lane = threadIdx.x & 31u;
-        for (unsigned t0 = gw * run; t0 < total; t0 += warps * run) {
+        extern __shared__ WallBuf wall_buf[];
+        WallBuf& B = wall_buf[threadIdx.x / 32u];
+        const unsigned lane = threadIdx.x & 31u;
+        for (unsigned t0 = gw * kWallRun; t0 < front; t0 += warps * kWallRun) {
+            const unsigned t = t0 + lane;
+            const bool valid = lane < kWallRun && t < front;
+            walls_entry_coop(P, C, valid, valid ? __ldg(C.hlist + t) : 0u, B);
+        }
+        const unsigned run = run_size(total, warps);
+        for (unsigned t0 = (warps - 1u - gw) * run; t0 < total; t0 += warps * run) {
             const unsigned t = t0 + lane;
             const bool valid = lane < run && t < total;
-            contact_entry_coop(P, C, valid, valid ? __ldg(C.hlist + list_index(t, front, P.n)) : 0u, B);
+            contact_entry_coop(P, C, valid, valid ? __ldg(C.hlist + list_index(t, front, P.n)) : 0u, t < front, B.c);
         }
         return;
     }
@@ -2692,13 +2702,14 @@ __global__ void __launch_bounds__(256) k_mx_store(MixParams P, Master M, const d
 __global__ void __launch_bounds__(256) k_mx_store_forces(MixParams P, Master M,
                                                          const float4* __restrict__ Fc,
                                                          const float4* __restrict__ Mc,
+                                                         const float4* __restrict__ Fw,
                                                          double* __restrict__ force,
                                                          double* __restrict__ moment)
 {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
     const size_t o = __float_as_uint(M.wl[i].w);
-    const float4 f = Fc[i], t = Mc[i];
+    const float4 f = contact_sum(Fc, Fw, i), t = Mc[i];
     force[3 * o + 0] = f.x;
     force[3 * o + 1] = f.y;
     force[3 * o + 2] = f.z;
@@ -2918,6 +2929,7 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
     A(alloc(s, &s->pr, n));
     A(alloc(s, &s->Fc, n));
     A(alloc(s, &s->Mc, n));
+    A(alloc(s, &s->Fw, n));
     A(alloc(s, &s->hlist, n));
     A(alloc(s, &s->wmask, n));
     A(alloc(s, &s->vcount, n));
@@ -3431,6 +3443,7 @@ static ContactArgs contact_args(MixedScene* s, unsigned* rc, unsigned* rp, unsig
     C.rxn = s->rxn;
     C.Fc = s->Fc;
     C.Mc = s->Mc;
+    C.Fw = s->Fw;
     C.counters = s->counters;
     C.rec_count = rc;
     C.rec_pairs = rp;
@@ -3457,7 +3470,7 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
         if (st != XD_OK) return st;
     }
     ph.begin(0, q);
-    k_mx_advance<MODE><<<blocks(n, 256), 256, 0, q>>>(s->P, M, s->Fc, s->Mc, s->pref, s->pf, s->qa, s->qb, s->pr,
+    k_mx_advance<MODE><<<blocks(n, 256), 256, 0, q>>>(s->P, M, s->Fc, s->Mc, s->Fw, s->pref, s->pf, s->qa, s->qb, s->pr,
                                                       s->counters, cond ? *cond : 0, cond ? 1 : 0);
     st = launch_status("mixed advance");
     ph.end(0, q);
@@ -3504,10 +3517,8 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
     } else {
         if (hist == 2) XD_MX_CONTACT(false, 2);
         else if (hist == 1) XD_MX_CONTACT(false, 1);
-        else if (s->cmode == 1) {
-            k_mx_contact<false, 0, true><<<grid, ct, (ct / 32u) * sizeof(PairBuf), q>>>(s->P, C);
-            if (s->P.nplanes || s->P.ntri) k_mx_walls<<<grid, ct, (ct / 32u) * sizeof(WallBuf), q>>>(s->P, C);
-        } else XD_MX_CONTACT(false, 0);
+        else if (s->cmode == 1) k_mx_contact<false, 0, true><<<grid, ct, (ct / 32u) * sizeof(WallBuf), q>>>(s->P, C);
+        else XD_MX_CONTACT(false, 0);
     }
 #undef XD_MX_CONTACT
     st = launch_status("mixed contact");
@@ -3624,7 +3635,7 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
     }
     // the last velocity update, and the call's body reactions
     ph.begin(0, q);
-    k_mx_finish<<<blocks(s->n, 256), 256, 0, q>>>(s->P, s->m[0], s->Fc, s->Mc);
+    k_mx_finish<<<blocks(s->n, 256), 256, 0, q>>>(s->P, s->m[0], s->Fc, s->Mc, s->Fw);
     st = launch_status("mixed finish");
     ph.end(0, q);
     if (st == XD_OK) {
@@ -3640,9 +3651,7 @@ unsigned long long mixed_launches(MixedScene* s, unsigned nsteps)
     if (!s || nsteps == 0 || s->n == 0) return 0;
     // per step: advance + contact; + the last velocity update; a step that
     // re-bins adds mixed_rebuild_launches()
-    // (and the wall pass after a cooperative pair pass)
-    const unsigned long long per = 2 + (s->kinematic && s->ntri ? 3 : 0) +
-                                   (s->cmode == 1 && (s->P.nplanes || s->P.ntri) ? 1 : 0);
+    const unsigned long long per = 2 + (s->kinematic && s->ntri ? 3 : 0);
     unsigned long long total = per * nsteps + 1 + (s->nbodies ? 1 : 0);
     if (!s->cells_clean) total += mixed_rebuild_launches(s);   // the first step re-bins
     return total;
@@ -3694,7 +3703,7 @@ int mixed_eval_contacts(MixedScene* s, double* force, double* moment, cudaStream
         st = cuda_status(cudaMemsetAsync(df, 0, sizeof(double) * 6 * n, q), "eval");
     if (st != XD_OK) return st;
     if (s->n) {
-        k_mx_store_forces<<<blocks(s->n, 256), 256, 0, q>>>(s->P, s->m[s->cur], s->Fc, s->Mc, df, dm);
+        k_mx_store_forces<<<blocks(s->n, 256), 256, 0, q>>>(s->P, s->m[s->cur], s->Fc, s->Mc, s->Fw, df, dm);
         st = launch_status("mixed store forces");
     }
     if (st == XD_OK && force)
@@ -4013,10 +4022,11 @@ __global__ void __launch_bounds__(256) k_batch_advance(const BatchScene* __restr
     __syncthreads();
     const unsigned i = (blockIdx.x - d.adv_block0) * blockDim.x + threadIdx.x;
     if (MODE == 2) {
-        if (i < sP.n) finish_one(sP, d.C.M, d.C.Fc, d.C.Mc, i);
+        if (i < sP.n) finish_one(sP, d.C.M, d.C.Fc, d.C.Mc, d.C.Fw, i);
         return;
     }
-    const bool out = i < sP.n && advance_one<MODE>(sP, d.C.M, d.C.Fc, d.C.Mc, d.pref, d.pf, d.qa, d.qb, d.pr, i);
+    const bool out = i < sP.n && advance_one<MODE>(sP, d.C.M, d.C.Fc, d.C.Mc, d.C.Fw, d.pref, d.pf, d.qa, d.qb,
+                                                              d.pr, i);
     if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) atomicOr(d.C.counters + CN_REBUILD, 1u);
 }
 
@@ -4053,11 +4063,11 @@ __global__ void k_batch_group(const unsigned* __restrict__ flags, unsigned first
 
 // Runs of listed particles per scene, as an exclusive prefix over scenes, of
 // counter word `cw` (CN_HEAVY: every listed particle; CN_HTRI: those with
-// walls in reach) into runs[0, ns]; runs[ns + 1] (the launch's next free run)
-// cleared, and the particles a run holds (run_size of all scenes' together)
-// in runs[ns + 2].
-__device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsigned cw, unsigned* __restrict__ runs,
-                           unsigned* c, unsigned& carry)
+// walls in reach) into runs[0, ns]; runs[ns + 1] (the next free run) cleared,
+// and the particles a run holds (`each`, or with 0 run_size of all scenes'
+// together) in runs[ns + 2].
+__device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsigned cw, unsigned each,
+                           unsigned* __restrict__ runs, unsigned* c, unsigned& carry)
 {
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -4066,7 +4076,7 @@ __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsign
     all = __reduce_add_sync(0xffffffffu, all);
     if ((threadIdx.x & 31u) == 0 && all) atomicAdd(&carry, all);
     __syncthreads();
-    const unsigned run = run_size(carry, kContactWarpsTotal);
+    const unsigned run = each ? each : run_size(carry, kContactWarpsTotal);
     __syncthreads();
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -4095,15 +4105,15 @@ __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsign
     __syncthreads();
 }
 
-// The runs of the contact launch (chunk_start) and of the wall launch
-// (chunk_start + ns + 3).
+// The pair runs (chunk_start; with per_particle, 32 particles each: the
+// per-particle pass's) and the wall runs (chunk_start + ns + 3).
 __global__ void __launch_bounds__(1024) k_batch_chunks(const BatchScene* __restrict__ D, unsigned ns,
-                                                       unsigned* __restrict__ chunk_start)
+                                                       int per_particle, unsigned* __restrict__ chunk_start)
 {
     __shared__ unsigned c[1024];
     __shared__ unsigned carry;
-    batch_runs(D, ns, CN_HEAVY, chunk_start, c, carry);
-    batch_runs(D, ns, CN_HTRI, chunk_start + ns + 3, c, carry);
+    batch_runs(D, ns, CN_HEAVY, per_particle ? 32u : 0u, chunk_start, c, carry);
+    batch_runs(D, ns, CN_HTRI, kWallRun, chunk_start + ns + 3, c, carry);
 }
 
 // The contact pass of every scene: each warp takes the next kBatchGrab runs
@@ -4119,60 +4129,71 @@ __host__ __device__ constexpr unsigned batch_scene_bytes(unsigned nwarps)
     return (unsigned)((nwarps * sizeof(WarpScene) + 15u) / 16u * 16u);
 }
 
-// KIND 0: the per-particle contact pass; 1: the cooperative pair pass; 2:
-// the wall pass (runs over the front of each scene's list).
+// KIND 0: the per-particle contact pass; 1: cooperative pair runs; 2: wall
+// runs (over the front of each scene's list).
 template <int KIND>
-__global__ void __launch_bounds__(kContactMaxThreads) k_batch_contact(const BatchScene* __restrict__ D, unsigned ns,
-                                                                   unsigned* __restrict__ chunk_start)
+__device__ __forceinline__ void batch_runs_of(const BatchScene* __restrict__ D, unsigned ns,
+                                              unsigned* __restrict__ chunk_start, WarpScene& W, WallBuf* B)
 {
-    // dynamic shared memory: one WarpScene per warp of the block, then (the
-    // cooperative kinds) one PairBuf or WallBuf per warp
-    extern __shared__ __align__(16) unsigned char batch_smem[];
-    const unsigned lane = threadIdx.x & 31u, wb = threadIdx.x / 32u, nwarps = blockDim.x / 32u;
-    WarpScene& W = reinterpret_cast<WarpScene*>(batch_smem)[wb];
-    unsigned char* const bufs = batch_smem + batch_scene_bytes(nwarps);
+    const unsigned lane = threadIdx.x & 31u;
     const unsigned total = __ldg(chunk_start + ns);
     unsigned* next = chunk_start + ns + 1;
     const unsigned run = __ldg(chunk_start + ns + 2), grab = run == 32u ? kBatchGrab : 1u;
     unsigned cur = 0xffffffffu, lo = 0, heavy = 0, front = 0;
     for (;;) {
-    unsigned c0 = 0;
-    if (lane == 0) c0 = atomicAdd(next, grab);
-    c0 = __shfl_sync(0xffffffffu, c0, 0);
-    if (c0 >= total) break;
-    const unsigned c1 = min(total, c0 + grab);
-    for (unsigned ch = c0; ch < c1; ++ch) {
-        if (cur == 0xffffffffu || ch >= __ldg(chunk_start + cur + 1)) {
-            // the scene holding run ch: the last s with chunk_start[s] <= ch
-            unsigned a = 0, b = ns;
-            while (b - a > 1u) {
-                const unsigned m = (a + b) / 2u;
-                if (__ldg(chunk_start + m) <= ch) a = m;
-                else b = m;
+        unsigned c0 = 0;
+        if (lane == 0) c0 = atomicAdd(next, grab);
+        c0 = __shfl_sync(0xffffffffu, c0, 0);
+        if (c0 >= total) break;
+        const unsigned c1 = min(total, c0 + grab);
+        for (unsigned ch = c0; ch < c1; ++ch) {
+            if (cur == 0xffffffffu || ch >= __ldg(chunk_start + cur + 1)) {
+                // the scene holding run ch: the last s with chunk_start[s] <= ch
+                unsigned a = 0, b = ns;
+                while (b - a > 1u) {
+                    const unsigned m = (a + b) / 2u;
+                    if (__ldg(chunk_start + m) <= ch) a = m;
+                    else b = m;
+                }
+                cur = a;
+                lo = __ldg(chunk_start + cur);
+                __syncwarp();
+                copy_words(&W.P, &D[cur].P, sizeof(MixParams), lane, 32u);
+                copy_words(&W.C, &D[cur].C, sizeof(ContactArgs), lane, 32u);
+                __syncwarp();
+                heavy = W.C.counters[CN_HEAVY];
+                front = W.C.counters[CN_HTRI];
             }
-            cur = a;
-            lo = __ldg(chunk_start + cur);
-            __syncwarp();
-            copy_words(&W.P, &D[cur].P, sizeof(MixParams), lane, 32u);
-            copy_words(&W.C, &D[cur].C, sizeof(ContactArgs), lane, 32u);
-            __syncwarp();
-            heavy = W.C.counters[CN_HEAVY];
-            front = W.C.counters[CN_HTRI];
-        }
-        const unsigned t = (ch - lo) * run + lane;
-        if (KIND == 1) {
-            const bool valid = lane < run && t < heavy;
-            contact_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + list_index(t, front, W.P.n)) : 0u,
-                               reinterpret_cast<PairBuf*>(bufs)[wb]);
-        } else if (KIND == 2) {
-            const bool valid = lane < run && t < front;
-            walls_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + t) : 0u,
-                             reinterpret_cast<WallBuf*>(bufs)[wb]);
-        } else if (lane < run && t < heavy) {
-            contact_entry<false, 0>(W.P, W.C, __ldg(W.C.hlist + list_index(t, front, W.P.n)));
+            const unsigned t = (ch - lo) * run + lane;
+            if (KIND == 1) {
+                const bool valid = lane < run && t < heavy;
+                contact_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + list_index(t, front, W.P.n)) : 0u,
+                                   t < front, B->c);
+            } else if (KIND == 2) {
+                const bool valid = lane < run && t < front;
+                walls_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + t) : 0u, *B);
+            } else if (t < heavy) {
+                contact_entry<false, 0>(W.P, W.C, __ldg(W.C.hlist + list_index(t, front, W.P.n)));
+            }
         }
     }
-    }
+}
+
+// One contact launch of a batch: KIND as above, or 3: the wall runs, then the
+// pair runs (the step graphs; kernel timing launches them apart).
+template <int KIND>
+__global__ void __launch_bounds__(kContactMaxThreads) k_batch_contact(const BatchScene* __restrict__ D, unsigned ns,
+                                                                   unsigned* __restrict__ chunk_start)
+{
+    // dynamic shared memory: one WarpScene per warp of the block, then (the
+    // cooperative kinds) one WallBuf per warp
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    const unsigned wb = threadIdx.x / 32u, nwarps = blockDim.x / 32u;
+    WarpScene& W = reinterpret_cast<WarpScene*>(batch_smem)[wb];
+    WallBuf* const B = reinterpret_cast<WallBuf*>(batch_smem + batch_scene_bytes(nwarps)) + wb;
+    if (KIND >= 2) batch_runs_of<2>(D, ns, chunk_start + ns + 3, W, B);
+    if (KIND == 1 || KIND == 3) batch_runs_of<1>(D, ns, chunk_start, W, B);
+    if (KIND == 0) batch_runs_of<0>(D, ns, chunk_start, W, nullptr);
 }
 
 }  // namespace
@@ -4203,31 +4224,21 @@ struct MixedBatch {
     unsigned long long launches[3] = {};
 };
 
-// The batch's contact launch: every scene's listed particles.
-static void launch_batch_pairs(const MixedBatch* b, unsigned ns, cudaStream_t q)
+// The batch's contact launches: every scene's listed particles.  KIND 1 and 2
+// apart for kernel timing, 3 both in one.
+template <int KIND>
+static void launch_batch_contact_kind(const MixedBatch* b, unsigned ns, cudaStream_t q)
 {
     const unsigned ct = b->cthreads, grid = kContactWarpsTotal * 32u / ct, w = ct / 32u;
-    if (b->cmode == 1)
-        k_batch_contact<1><<<grid, ct, batch_scene_bytes(w) + w * sizeof(PairBuf), q>>>(b->d_scenes, ns,
-                                                                                         b->d_chunks);
-    else
-        k_batch_contact<0><<<grid, ct, batch_scene_bytes(w), q>>>(b->d_scenes, ns, b->d_chunks);
-}
-
-// The wall pass after a cooperative pair pass (none otherwise: the
-// per-particle pass does its walls itself).
-static void launch_batch_walls(const MixedBatch* b, unsigned ns, cudaStream_t q)
-{
-    const unsigned ct = b->cthreads, grid = kContactWarpsTotal * 32u / ct, w = ct / 32u;
-    if (b->cmode == 1 && b->walls)
-        k_batch_contact<2><<<grid, ct, batch_scene_bytes(w) + w * sizeof(WallBuf), q>>>(b->d_scenes, ns,
-                                                                                         b->d_chunks + ns + 3);
+    const unsigned smem = batch_scene_bytes(w) + (KIND ? w * (unsigned)sizeof(WallBuf) : 0u);
+    k_batch_contact<KIND><<<grid, ct, smem, q>>>(b->d_scenes, ns, b->d_chunks);
 }
 
 static void launch_batch_contact(const MixedBatch* b, unsigned ns, cudaStream_t q)
 {
-    launch_batch_pairs(b, ns, q);
-    launch_batch_walls(b, ns, q);
+    if (b->cmode == 0) launch_batch_contact_kind<0>(b, ns, q);
+    else if (b->walls) launch_batch_contact_kind<3>(b, ns, q);
+    else launch_batch_contact_kind<1>(b, ns, q);
 }
 
 namespace {
@@ -4354,7 +4365,7 @@ int capture_batch_step(MixedBatch* b, int kind)
                                                                  cudaStreamSetCaptureDependencies),
                              "batch capture dependencies");
         if (st == XD_OK) {
-            k_batch_chunks<<<1, 1024, 0, cs>>>(b->d_scenes, ns, b->d_chunks);
+            k_batch_chunks<<<1, 1024, 0, cs>>>(b->d_scenes, ns, b->cmode == 0, b->d_chunks);
             launch_batch_contact(b, ns, cs);
             st = launch_status("batch contact");
         }
@@ -4488,17 +4499,17 @@ int mixed_batch_create(MixedScene* const* scenes, unsigned count, MixedBatch** o
         for (unsigned j = 0; j < k; ++j)
             if (scenes[j] == sc) return set_error(XD_ERR_INVALID, "batch: scene %u given twice", k);
     }
-    // the cooperative kinds' shared memory at the largest block: the wall
-    // pass's is above the 48 KB a launch may take without asking
+    // the cooperative kinds' shared memory at the largest block, above the
+    // 48 KB that a launch may take without asking
     {
         const unsigned w = kContactMaxThreads / 32u;
-        int st = cuda_status(cudaFuncSetAttribute(k_batch_contact<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)(batch_scene_bytes(w) + w * sizeof(PairBuf))),
-                             "batch pair pass shared memory");
-        if (st == XD_OK)
-            st = cuda_status(cudaFuncSetAttribute(k_batch_contact<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)(batch_scene_bytes(w) + w * sizeof(WallBuf))),
-                             "batch wall pass shared memory");
+        const int most = (int)(batch_scene_bytes(w) + w * sizeof(WallBuf));
+        int st = XD_OK;
+        for (const void* k : { (const void*)k_batch_contact<1>, (const void*)k_batch_contact<2>,
+                               (const void*)k_batch_contact<3> })
+            if (st == XD_OK)
+                st = cuda_status(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                                 "batch contact shared memory");
         if (st != XD_OK) return st;
     }
     MixedBatch* b = new (std::nothrow) MixedBatch();
@@ -4565,9 +4576,13 @@ int batch_step_direct(MixedBatch* b, unsigned nsteps, cudaStream_t q)
         for (unsigned k = 0; k < ns && st == XD_OK; ++k)
             if (flags[k]) st = rebuild(b->scenes[k], q);
         if (st != XD_OK) break;
-        k_batch_chunks<<<1, 1024, 0, q>>>(b->d_scenes, ns, b->d_chunks);
-        span(1, [&] { launch_batch_pairs(b, ns, q); });
-        if (b->cmode == 1 && b->walls) span(2, [&] { launch_batch_walls(b, ns, q); });
+        k_batch_chunks<<<1, 1024, 0, q>>>(b->d_scenes, ns, b->cmode == 0, b->d_chunks);
+        if (b->cmode == 0) {
+            span(1, [&] { launch_batch_contact_kind<0>(b, ns, q); });
+        } else {
+            span(1, [&] { launch_batch_contact_kind<1>(b, ns, q); });
+            if (b->walls) span(2, [&] { launch_batch_contact_kind<2>(b, ns, q); });
+        }
         st = launch_status("batch contact");
     }
     if (st == XD_OK) {

@@ -351,8 +351,9 @@ class Batch:
 
     def kernel_times(self) -> dict:
         """{"advance": (ms, launches), "contact": (ms, launches), "walls": (ms, launches)} since
-        timing was enabled: the advance, the pair pass (the whole contact pass in contact_mode
-        0) and the wall pass that follows a cooperative pair pass."""
+        timing was enabled: the advance, the pair runs (the whole contact pass in contact_mode
+        0) and the wall runs, launched after the pair runs while timing is on (the step graphs
+        run both in one launch)."""
         ms = np.zeros(3)
         n = np.zeros(3, np.uint64)
         call("xd_batch_kernel_times", self.handle, ms.ctypes.data, n.ctypes.data)
