@@ -442,8 +442,12 @@ __device__ __forceinline__ dfl q_to_df(long long q)
 // (impl:455), dv = s + t exact, u = dq / |dq| from the exact integer
 // separation (|dq| = d0 + c), the radii from their fixed-point values, the
 // angular velocities from their hi/lo pairs, and the normal speed q0 + q1.
-// Used where the FP32 rotation term's rounding could matter (rolling).
-__device__ __noinline__ f3 slip_pair(const float s[3], const float t[3], const int dq[3], float d0, float c,
+// Used where the FP32 rotation term's rounding could matter (rolling).  Inline,
+// as normal_pair: some lane of nearly every group of 32 contacts needs it, and
+// the two calls cost a 199,583-sphere bed's pass 62 us against 56.  (The pass
+// must stay within 128 registers: 16 warps an SM.  With 130 it takes 250 us on
+// 500,000 spheres against 132.)
+__device__ __forceinline__ f3 slip_pair(const float s[3], const float t[3], const int dq[3], float d0, float c,
                                      float q0, float q1, long long qri, long long qrj, float4 wih, float4 wil,
                                      float4 wjh, float4 wjl)
 {
@@ -510,7 +514,7 @@ __device__ __forceinline__ dfl d_to_df(double x)
 // reference's expression, impl:449-452), getConstant's Req and Meq from the
 // FP64 radii and masses (impl:238-246), the normal speed q0 + q1.  No
 // cohesion (the cohesive recheck is FP64).
-__device__ __noinline__ float normal_pair(const MixParams& P, const Master& M, const double* __restrict__ mass0,
+__device__ __forceinline__ float normal_pair(const MixParams& P, const Master& M, const double* __restrict__ mass0,
                                           unsigned i, unsigned j, unsigned idi, unsigned idj, float q0, float q1)
 {
     const dfl X = d_to_df(__ldg(M.x + j) - __ldg(M.x + i));
@@ -2209,6 +2213,7 @@ constexpr unsigned kCoopSlots = 16;
 // List entries that a lane loads together (a 199,583-sphere bed's pass 62 us;
 // 66 with four at a time and the exact test, three times the bytes, in the scan).
 constexpr unsigned kScanAtOnce = 8;
+constexpr unsigned kRunMin = 4;   // the least particles of a run
 
 struct CoopBuf {
     unsigned cand[32 * kCoopSlots];   // k-major: lane L's k-th candidate at [k * 32 + L]
@@ -2514,13 +2519,16 @@ __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const Conta
 }
 
 // Listed particles that a warp of the cooperative pair pass takes at a time:
-// 32, which fill its lanes with contacts best, or 16 or 8 where `total` of
-// them would leave warps without any -- a run is a chain of loads and of groups
-// of 32 contacts, and a short list's pass lasts as long as one run.  With runs
-// of 32 always, 8,000 spheres' pairs and walls took 24 us a step (16 with this).
+// at most 32, and as many as give every warp the same number of runs -- a run
+// is a chain of loads and of groups of 32 contacts, the pass lasts as long as
+// the warp with the most of them, and a short list's as long as one.  Runs of
+// 32 always, us a step: 8,000 spheres' pairs and walls 24, 199,583 spheres
+// (2.6 runs a warp) 56; with this 12 and 54.
 __host__ __device__ __forceinline__ unsigned run_size(unsigned total, unsigned warps)
 {
-    return total <= warps * 8u ? 8u : (total <= warps * 16u ? 16u : 32u);
+    const unsigned full = 32u * warps, rounds = total > full ? (total + full - 1u) / full : 1u;
+    const unsigned run = (total + rounds * warps - 1u) / (rounds * warps);
+    return run < kRunMin ? kRunMin : run;
 }
 
 // COOP: the warp-cooperative passes (no history, no recording; dynamic shared
@@ -3494,8 +3502,8 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
     s->cells_clean = true;
     ph.begin(3, q);
     // the list holds at most n particles: no more warps than there are runs of
-    // 8 of them (of 32 in the per-particle pass)
-    const unsigned ct = s->cthreads, each = s->cmode == 1 ? ct / 4u : ct;
+    // kRunMin of them (of 32 in the per-particle pass)
+    const unsigned ct = s->cthreads, each = s->cmode == 1 ? ct / 32u * kRunMin : ct;
     const unsigned grid = std::max(1u, std::min(kContactWarpsTotal * 32u / ct, (n + each - 1) / each));
     // tangential springs: updated by a step, read only by the diagnostic evaluation (MODE 3)
     const HistTable ht = history_table(s);
@@ -3981,7 +3989,7 @@ namespace {
 
 constexpr unsigned kBatchGroup = 32;
 constexpr unsigned kBatchGraphSteps = 4;   // later steps captured per graph launch
-constexpr unsigned kBatchGrab = 2;         // runs of 32 listed particles that a contact warp takes at a time
+constexpr unsigned kBatchGrab = 1;         // runs that a contact warp takes at a time
 
 
 // One scene of a batch as the batch kernels read it.
@@ -4138,14 +4146,14 @@ __device__ __forceinline__ void batch_runs_of(const BatchScene* __restrict__ D, 
     const unsigned lane = threadIdx.x & 31u;
     const unsigned total = __ldg(chunk_start + ns);
     unsigned* next = chunk_start + ns + 1;
-    const unsigned run = __ldg(chunk_start + ns + 2), grab = run == 32u ? kBatchGrab : 1u;
+    const unsigned run = __ldg(chunk_start + ns + 2);
     unsigned cur = 0xffffffffu, lo = 0, heavy = 0, front = 0;
     for (;;) {
         unsigned c0 = 0;
-        if (lane == 0) c0 = atomicAdd(next, grab);
+        if (lane == 0) c0 = atomicAdd(next, kBatchGrab);
         c0 = __shfl_sync(0xffffffffu, c0, 0);
         if (c0 >= total) break;
-        const unsigned c1 = min(total, c0 + grab);
+        const unsigned c1 = min(total, c0 + kBatchGrab);
         for (unsigned ch = c0; ch < c1; ++ch) {
             if (cur == 0xffffffffu || ch >= __ldg(chunk_start + cur + 1)) {
                 // the scene holding run ch: the last s with chunk_start[s] <= ch
@@ -4179,10 +4187,17 @@ __device__ __forceinline__ void batch_runs_of(const BatchScene* __restrict__ D, 
     }
 }
 
+// Out of line: the pair runs' registers are then theirs alone.
+__device__ __noinline__ void batch_wall_runs(const BatchScene* __restrict__ D, unsigned ns,
+                                             unsigned* __restrict__ chunk_start, WarpScene& W, WallBuf* B)
+{
+    batch_runs_of<2>(D, ns, chunk_start, W, B);
+}
+
 // One contact launch of a batch: KIND as above, or 3: the wall runs, then the
 // pair runs (the step graphs; kernel timing launches them apart).
 template <int KIND>
-__global__ void __launch_bounds__(kContactMaxThreads) k_batch_contact(const BatchScene* __restrict__ D, unsigned ns,
+__global__ void __launch_bounds__(kContactMaxThreads, KIND ? 4 : 1) k_batch_contact(const BatchScene* __restrict__ D, unsigned ns,
                                                                    unsigned* __restrict__ chunk_start)
 {
     // dynamic shared memory: one WarpScene per warp of the block, then (the
@@ -4191,7 +4206,7 @@ __global__ void __launch_bounds__(kContactMaxThreads) k_batch_contact(const Batc
     const unsigned wb = threadIdx.x / 32u, nwarps = blockDim.x / 32u;
     WarpScene& W = reinterpret_cast<WarpScene*>(batch_smem)[wb];
     WallBuf* const B = reinterpret_cast<WallBuf*>(batch_smem + batch_scene_bytes(nwarps)) + wb;
-    if (KIND >= 2) batch_runs_of<2>(D, ns, chunk_start + ns + 3, W, B);
+    if (KIND >= 2) batch_wall_runs(D, ns, chunk_start + ns + 3, W, B);
     if (KIND == 1 || KIND == 3) batch_runs_of<1>(D, ns, chunk_start, W, B);
     if (KIND == 0) batch_runs_of<0>(D, ns, chunk_start, W, nullptr);
 }
