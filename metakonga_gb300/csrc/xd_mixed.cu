@@ -86,14 +86,17 @@ enum {
     CN_REBUILDS = 7,   // re-binnings (cumulative)
     CN_RXN = 8,        // blocks of k_rxn_sum done (the last one finishes the sum)
     CN_HTRI = 9,       // listed particles with walls (planes, triangles) in reach: hlist[0, CN_HTRI)
-    CN_HBACK = 10,     // the other listed particles: hlist[n - CN_HBACK, n)
+    CN_DMAX = 10,      // largest squared displacement of a particle since the last build (FP32 bits)
     CN_WALLS = 11,     // wall contacts decided by the FP64 region test (cumulative)
     CN_VINC = 12,      // Verlet lists over their capacity at the last build (the pass searches the cells)
     CN_TINC = 13,      // triangle lists over their capacity at the last build
     CN_VSUM = 14,      // Verlet-list entries at the last build
     CN_TSUM = 15,      // triangle-list entries at the last build
-    kCounters = 16
+    CN_BIN = 16,       // listed particles by class at the last build: near walls, then by gap (kGapBins)
+    CN_CUR = 25,       // k_mx_list's cursors of the classes
+    kCounters = 34
 };
+constexpr unsigned kGapBins = 8;
 
 struct Master {
     double *x, *y, *z, *r;   // FP64 positions and radii
@@ -120,6 +123,7 @@ struct MixParams {
                          // in 32 bits (their FP32 values then come from 32-bit conversions)
     float vcut;          // Verlet list: pairs within ri + rj + vcut are listed
     float disp2;         // squared displacement that forces re-binning
+    float gap_bin, inv_gap_bin;   // width of a gap class (vcut / kGapBins)
     float inv_gx, inv_gxy;   // 1 / gx, 1 / (gx gy) for the key decode
     float dtf, hf, half2dtf;
     float gf[3];
@@ -188,7 +192,8 @@ struct MixedScene {
     float4* Mc = nullptr;
     float4* Fw = nullptr;         // wall force (the cooperative pass's wall runs)
     // Verlet lists (slots of the current cell order, rebuilt with the cells)
-    unsigned* hlist = nullptr;    // particles with neighbours or planes in reach
+    unsigned* hlist = nullptr;    // particles with neighbours or walls in reach, by class
+    unsigned char* lclass = nullptr;   // each particle's class (kUnlisted: none)
     unsigned short* wmask = nullptr;   // planes in reach of each particle
     unsigned* vcount = nullptr;   // Verlet neighbours per particle (| kIncomplete: overflow)
     unsigned* vlist = nullptr;    // [vcap][n]: neighbour slots in search order
@@ -607,22 +612,6 @@ __device__ __forceinline__ unsigned cell_key(const MixParams& P, float x, float 
     return ((unsigned)cz * (unsigned)P.gy + (unsigned)cy) * (unsigned)P.gx + (unsigned)cx;
 }
 
-// Appends v to list (counter *cnt) for the lanes where take is set, one
-// atomic per warp.  Every lane of the warp calls it.
-template <typename T>
-__device__ __forceinline__ void warp_append(bool take, const T& v, T* __restrict__ list,
-                                            unsigned* __restrict__ cnt)
-{
-    const unsigned bal = __ballot_sync(0xffffffffu, take);
-    if (!bal) return;
-    const unsigned lane = threadIdx.x & 31u;
-    const int leader = __ffs(bal) - 1;
-    unsigned base = 0;
-    if ((int)lane == leader) base = atomicAdd(cnt, (unsigned)__popc(bal));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (take) list[base + __popc(bal & ((1u << lane) - 1u))] = v;
-}
-
 // Adds one to a diagnostic counter for each lane that calls it, one atomic
 // per group of converged lanes (a shared address would otherwise serialise
 // every lane's increment).
@@ -640,6 +629,14 @@ __device__ __forceinline__ void count_add(unsigned* c, unsigned v)
     if ((threadIdx.x & 31u) == (unsigned)(__ffs(m) - 1) && t) atomicAdd(c, t);
 }
 
+// Loads issued where they stand: the compiler otherwise moves the loads of a
+// batch behind the branches that use them, one after another.
+__device__ __forceinline__ float4 ldg_now(const float4* p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 // ---- integration -----------------------------------------------------------
 //
 // Velocity Verlet as the reference splits it (vv_update_position_kernel
@@ -707,38 +704,40 @@ __device__ __forceinline__ double drift(const MixParams& P, double x, float vhi,
 // that does not sets CN_REBUILD.  The last block to finish passes the flag to
 // the graph's conditional node (use_cond), one caller as the conditional
 // requires.
-// The contact force of slot i: the pairs' and, where its .w says so, the walls'.
-__device__ __forceinline__ float4 contact_sum(const float4* __restrict__ Fc, const float4* __restrict__ Fw, unsigned i)
+// Fc.w: what the contact pass left at a slot (zero: no contact, F = M = 0).
+constexpr float kHasWalls = 1.f, kHasPairs = 2.f;
+
+// The walls' part of slot i's contact force f, where its .w says so.
+__device__ __forceinline__ void add_walls(float4& f, const float4* __restrict__ Fw, unsigned i)
 {
-    float4 f = Fc[i];
-    if (f.w != 0.f) {
+    if (f.w == kHasWalls || f.w == kHasWalls + kHasPairs) {
         const float4 w = Fw[i];
         f.x += w.x;
         f.y += w.y;
         f.z += w.z;
     }
-    return f;
 }
 
 // One slot of the advance (MODE 0: drift; MODE 1: kick with the last
-// contact forces, then drift), its contact view, and whether it has left half
-// the skin since the last build.
+// contact forces, then drift), its contact view, and its squared displacement
+// since the last build.
 template <int MODE>
-__device__ __forceinline__ bool advance_one(const MixParams& P, const Master& M, const float4* __restrict__ Fc,
-                                            const float4* __restrict__ Mc, const float4* __restrict__ Fw,
-                                            const float4* __restrict__ pref,
-                                            float4* __restrict__ pf, longlong2* __restrict__ qa,
-                                            longlong2* __restrict__ qb, float4* __restrict__ pr,
-                                            const unsigned i)
+__device__ __forceinline__ float advance_one(const MixParams& P, const Master& M, const float4* __restrict__ Fc,
+                                             const float4* __restrict__ Mc, const float4* __restrict__ Fw,
+                                             const float4* __restrict__ pref,
+                                             float4* __restrict__ pf, longlong2* __restrict__ qa,
+                                             longlong2* __restrict__ qb, float4* __restrict__ pr,
+                                             const unsigned i)
 {
     double x = M.x[i], y = M.y[i], z = M.z[i];
     const double r = M.r[i];
     if (MODE == 0 || MODE == 1) {
         float4 vh = M.vh[i], vl = M.vl[i], ab = M.ab[i];
         if (MODE == 1) {
-            float4 wh = M.wh[i], wl = M.wl[i];
+            float4 wh = M.wh[i], wl = M.wl[i], f = Fc[i];
             float2 b2 = M.b2[i];
-            kick(P, vh, vl, wh, wl, ab, b2, contact_sum(Fc, Fw, i), Mc[i]);
+            add_walls(f, Fw, i);
+            kick(P, vh, vl, wh, wl, ab, b2, f, Mc[i]);
             M.vh[i] = vh;
             M.vl[i] = vl;
             M.wh[i] = wh;
@@ -756,7 +755,35 @@ __device__ __forceinline__ bool advance_one(const MixParams& P, const Master& M,
     const float4 v = write_view(P, i, x, y, z, r, pf, qa, qb, pr);
     const float4 r0 = pref[i];
     const float dx = v.x - r0.x, dy = v.y - r0.y, dz = v.z - r0.z;
-    return !(dx * dx + dy * dy + dz * dz < P.disp2);
+    return dx * dx + dy * dy + dz * dz;
+}
+
+// A block's part of the skin test, for every thread of a 256-thread block: its
+// largest squared displacement since the last build, to its thread 0 (infinity
+// where a particle has left half the skin or is nowhere).  A reduction and one
+// barrier; an atomic per warp took 28 us where a million spheres had just been
+// listed.
+__device__ __forceinline__ unsigned block_displacement(const MixParams& P, float d2)
+{
+    __shared__ unsigned most[8];
+    const unsigned m = __reduce_max_sync(0xffffffffu, d2 < P.disp2 ? __float_as_uint(d2) : 0x7f800000u);
+    if ((threadIdx.x & 31u) == 0) most[threadIdx.x / 32u] = m;
+    __syncthreads();
+    unsigned a = 0;
+    if (threadIdx.x == 0)
+        for (unsigned w = 0; w < 8u; ++w) a = max(a, most[w]);
+    return a;
+}
+
+// ... and into the counters (thread 0): the displacement that limits which gap
+// classes of the list may touch (listed_now), the flag of a re-binning.
+__device__ __forceinline__ void note_displacement(unsigned a, unsigned* counters)
+{
+    if (a > __ldcg(counters + CN_DMAX)) atomicMax(counters + CN_DMAX, a);
+    if (a == 0x7f800000u) {
+        atomicOr(counters + CN_REBUILD, 1u);
+        __threadfence();   // (before the block counts as done)
+    }
 }
 
 template <int MODE>
@@ -768,26 +795,20 @@ __global__ void __launch_bounds__(256) k_mx_advance(MixParams P, Master M, const
                                                     unsigned* __restrict__ counters,
                                                     cudaGraphConditionalHandle cond, int use_cond)
 {
-    __shared__ bool last;
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool out = i < P.n && advance_one<MODE>(P, M, Fc, Mc, Fw, pref, pf, qa, qb, pr, i);
-    // only the flag must be visible to the last block: the lanes that set it
-    // fence; the state and view writes need no ordering here
-    if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) {
-        atomicOr(counters + CN_REBUILD, 1u);
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counters + CN_DONE, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        const unsigned f = atomicOr(counters + CN_REBUILD, 0u) ? 1u : 0u;
-        // the handle's default (0, assigned at every graph launch) stands
-        // unless a re-binning is due
-        if (use_cond && f) cudaGraphSetConditional(cond, 1u);
-        counters[CN_DONE] = 0;
-    }
+    const unsigned a =
+        block_displacement(P, i < P.n ? advance_one<MODE>(P, M, Fc, Mc, Fw, pref, pf, qa, qb, pr, i) : 0.f);
+    if (threadIdx.x != 0) return;
+    // only the flag must be visible to the last block: the state and view
+    // writes need no ordering here
+    note_displacement(a, counters);
+    if (atomicAdd(counters + CN_DONE, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const unsigned f = atomicOr(counters + CN_REBUILD, 0u) ? 1u : 0u;
+    // the handle's default (0, assigned at every graph launch) stands
+    // unless a re-binning is due
+    if (use_cond && f) cudaGraphSetConditional(cond, 1u);
+    counters[CN_DONE] = 0;
 }
 
 // Re-binning, 1: the cell key of every slot's current position.
@@ -848,7 +869,9 @@ __device__ __forceinline__ void finish_one(const MixParams& P, const Master& M, 
 {
     float4 vh = M.vh[i], vl = M.vl[i], wh = M.wh[i], wl = M.wl[i], ab = M.ab[i];
     float2 b2 = M.b2[i];
-    kick(P, vh, vl, wh, wl, ab, b2, contact_sum(Fc, Fw, i), Mc[i]);
+    float4 f = Fc[i];
+    add_walls(f, Fw, i);
+    kick(P, vh, vl, wh, wl, ab, b2, f, Mc[i]);
     M.vh[i] = vh;
     M.vl[i] = vl;
     M.wh[i] = wh;
@@ -1017,6 +1040,7 @@ __device__ __forceinline__ float near_reach(const MixParams& P, const float4& pi
     return pi.w + ((fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z)) * 3e-7f + (pi.w + P.rmaxf) * 2e-6f + 1e-10f);
 }
 
+constexpr unsigned kUnlisted = 255u;            // lclass of a particle that is not listed
 constexpr unsigned kIncomplete = 0x80000000u;   // vcount flag: the list is not complete
 
 // ---- triangle meshes ---------------------------------------------------------
@@ -1220,14 +1244,16 @@ __global__ void __launch_bounds__(256) k_mx_build(MixParams P, const float4* __r
                                                   unsigned short* __restrict__ wmask,
                                                   const unsigned* __restrict__ tcount,
                                                   double* __restrict__ rxn,
-                                                  unsigned* __restrict__ hlist,
+                                                  unsigned char* __restrict__ lclass,
                                                   float4* __restrict__ Fc, float4* __restrict__ Mc,
                                                   unsigned* __restrict__ counters)
 {
     __shared__ uint2 rows[9][256];
+    __shared__ unsigned found[kGapBins + 1];
     const unsigned tid = threadIdx.x;
     const unsigned i = blockIdx.x * blockDim.x + tid;
-    bool heavy = false, tri = false;
+    if (tid <= kGapBins) found[tid] = 0;
+    __syncthreads();
     if (i < P.n) {
         const float4 pi = __ldg(pf + i);
         pref[i] = pi;
@@ -1265,6 +1291,7 @@ __global__ void __launch_bounds__(256) k_mx_build(MixParams P, const float4* __r
         const unsigned n = P.n;
         const float rt0 = pi.w + P.vcut;
         unsigned nv = 0, r = 0;
+        float gap = 3.0e38f;   // to the nearest listed neighbour
         uint2 b = rows[0][tid];
         unsigned j = b.x;
         for (; left; --left, ++j) {
@@ -1277,32 +1304,79 @@ __global__ void __launch_bounds__(256) k_mx_build(MixParams P, const float4* __r
             const float4 pj = __ldg(pf + j);
             const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
             const float Rt = rt0 + pj.w;
-            if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) >= Rt * Rt || j == i) continue;
+            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            if (d2 >= Rt * Rt || j == i) continue;
+            gap = fminf(gap, sqrtf(d2) - (pi.w + pj.w));
             if (nv < P.vcap) vlist[(size_t)nv * n + i] = j;
             ++nv;
         }
         vcount[i] = nv > P.vcap ? (P.vcap | kIncomplete) : nv;
         if (nv > P.vcap) count_one(counters + CN_VINC);
         count_add(counters + CN_VSUM, min(nv, P.vcap));
-        tri = (P.ntri && __ldg(tcount + i) != 0u) || wm != 0u;   // walls in reach
-        heavy = nv > 0 || tri;
+        // its class: walls (planes or triangles) in reach, or its gap's
+        const bool wall = (P.ntri && __ldg(tcount + i) != 0u) || wm != 0u;
+        unsigned c = kUnlisted;
+        if (wall) c = 0;
+        else if (nv) c = 1u + (unsigned)min(max((int)(gap * P.inv_gap_bin), 0), (int)kGapBins - 1);
+        lclass[i] = (unsigned char)c;
+        if (c != kUnlisted) atomicAdd(&found[c], 1u);
     }
-    // the spheres with walls (planes or triangles) in reach first, the others
-    // from the end: the wall pass takes the front of the list, and in the
-    // per-particle pass the warps run the wall work side by side instead of
-    // on a few lanes each
-    warp_append(heavy && tri, i, hlist, counters + CN_HTRI);
-    const unsigned bal = __ballot_sync(0xffffffffu, heavy && !tri);
-    if (bal) {
-        const unsigned lane = threadIdx.x & 31u;
-        const int leader = __ffs(bal) - 1;
-        unsigned base = 0;
-        if ((int)lane == leader) base = atomicAdd(counters + CN_HBACK, (unsigned)__popc(bal));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (heavy && !tri) hlist[P.n - 1u - (base + __popc(bal & ((1u << lane) - 1u)))] = i;
+    __syncthreads();
+    if (tid <= kGapBins && found[tid]) {
+        atomicAdd(counters + CN_BIN + tid, found[tid]);
+        atomicAdd(counters + CN_HEAVY, found[tid]);
+        if (tid == 0) atomicAdd(counters + CN_HTRI, found[0]);
     }
-    const unsigned hb = __ballot_sync(0xffffffffu, heavy);
-    if (hb && (threadIdx.x & 31u) == 0) atomicAdd(counters + CN_HEAVY, (unsigned)__popc(hb));
+}
+
+// The list of the particles that have neighbours or walls in reach, by class:
+// those with walls first (the wall runs take that front), then the others by
+// the gap to their nearest neighbour.  A particle whose gap exceeds what any
+// two have moved since the build has had no contact and needs no scan
+// (listed_now): in a falling cloud that is most of the list.
+__global__ void __launch_bounds__(256) k_mx_list(MixParams P, const unsigned char* __restrict__ lclass,
+                                                 unsigned* __restrict__ hlist, unsigned* __restrict__ counters)
+{
+    __shared__ unsigned cnt[kGapBins + 1], base[kGapBins + 1];
+    const unsigned tid = threadIdx.x, i = blockIdx.x * blockDim.x + tid;
+    if (tid <= kGapBins) cnt[tid] = 0;
+    __syncthreads();
+    const unsigned c = i < P.n ? (unsigned)lclass[i] : kUnlisted;
+    // rank within the block, in slot order by warps
+    const unsigned peers = __match_any_sync(0xffffffffu, c), before = peers & ((1u << (tid & 31u)) - 1u);
+    unsigned at = 0;
+    for (unsigned w = 0; w < blockDim.x / 32u; ++w) {
+        if (tid / 32u == w && c != kUnlisted) {
+            at = cnt[c] + __popc(before);
+            __syncwarp(peers);
+            if (!before) cnt[c] += __popc(peers);
+        }
+        __syncthreads();
+    }
+    if (tid <= kGapBins) {
+        unsigned first = 0;
+        for (unsigned k = 0; k < tid; ++k) first += counters[CN_BIN + k];
+        base[tid] = first + (cnt[tid] ? atomicAdd(counters + CN_CUR + tid, cnt[tid]) : 0u);
+    }
+    __syncthreads();
+    if (c != kUnlisted) hlist[base[c] + at] = i;
+}
+
+// The listed particles that a contact pass has to visit now: those with walls
+// in reach and the gap classes that may touch, the first of the list.  Two
+// particles have each moved at most the largest displacement since the build;
+// 2 P.tol covers the FP32 positions then and now.
+__device__ __forceinline__ unsigned listed_now(const MixParams& P, const unsigned* __restrict__ counters)
+{
+    unsigned c[kGapBins + 1];
+#pragma unroll
+    for (unsigned k = 0; k <= kGapBins; ++k) c[k] = counters[CN_BIN + k];
+    const float reach = 2.f * sqrtf(__uint_as_float(counters[CN_DMAX])) * 1.0001f + 2.f * P.tol;
+    unsigned t = c[0] + c[1];
+#pragma unroll
+    for (unsigned k = 1; k < kGapBins; ++k)
+        if ((float)k * P.gap_bin <= reach) t += c[k + 1];
+    return t;
 }
 
 // Per-particle contact state carried across the pairs of one particle (the
@@ -1573,13 +1647,6 @@ __device__ __forceinline__ void accumulate(PairAcc& A, const PairOut& o)
 // FP64, in plane order (the others are out of reach and add exactly zero).
 // Block 0 clears CN_REBUILD for the next step's skin test.
 
-
-// Entry t of the listed particles: the ones with triangles in reach fill the
-// list from the front (front of them), the others from the end.
-__device__ __forceinline__ unsigned list_index(unsigned t, unsigned front, unsigned n)
-{
-    return t < front ? t : n - 1u - (t - front);
-}
 
 // The pointers of one scene the contact pass reads and writes.
 struct ContactArgs {
@@ -2025,7 +2092,7 @@ __device__ __forceinline__ void contact_entry(const MixParams& P, const ContactA
         I.qb = __ldg(qb + i);
         for_each_contact<true>(P, M, i, pi, I.qa, I.qb, __ldg(keys + i), pf, qa, qb, lb, counters, add);
     }
-    float4 F = make_float4(A.sumF.x, A.sumF.y, A.sumF.z, 0.f);
+    float4 F = make_float4(A.sumF.x, A.sumF.y, A.sumF.z, kHasPairs);   // its walls are in F
     // planes in reach: an FP32 distance to the supporting plane first (the
     // finite plane is never nearer), the reference's FP64 test after it
     unsigned wm = __ldg(wmask + i);
@@ -2268,15 +2335,6 @@ __device__ __noinline__ bool coop_cells(const MixParams& P, const ContactArgs& C
     return seen > done;
 }
 
-// A read-only load issued where it stands: the compiler otherwise moves the
-// loads of a batch behind the branches that use them, one after another.
-__device__ __forceinline__ float4 load_now(const float4* p)
-{
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-
 // Own data of slot i as contact_force reads it.
 __device__ __forceinline__ Own load_own(const MixParams& P, const ContactArgs& C, unsigned i)
 {
@@ -2334,7 +2392,7 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
                     for (unsigned q = 0; q < kScanAtOnce; ++q)
                         jj[q] = kpos + q < vc ? __ldg(C.vlist + (size_t)(kpos + q) * n + i) : i;
 #pragma unroll
-                    for (unsigned q = 0; q < kScanAtOnce; ++q) pp[q] = load_now(C.pf + jj[q]);
+                    for (unsigned q = 0; q < kScanAtOnce; ++q) pp[q] = ldg_now(C.pf + jj[q]);
 #pragma unroll
                     for (unsigned q = 0; q < kScanAtOnce; ++q) {
                         if (kpos >= vc || cnt >= kCoopSlots) break;
@@ -2346,6 +2404,7 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
                     }
                 }
                 more = kpos < vc;
+                done += cnt;
             } else {
                 more = coop_cells(P, C, i, pi, rt0, done, mine, cnt);
             }
@@ -2402,7 +2461,7 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
     }
     if (!valid) return;
     // the walls' part comes from a wall run (walls_entry_coop), into Fw
-    C.Fc[i] = make_float4(A.sumF.x, A.sumF.y, A.sumF.z, walls ? 1.f : 0.f);
+    C.Fc[i] = make_float4(A.sumF.x, A.sumF.y, A.sumF.z, (done ? kHasPairs : 0.f) + (walls ? kHasWalls : 0.f));
     C.Mc[i] = make_float4(A.sumM.x, A.sumM.y, A.sumM.z, 0.f);
 }
 
@@ -2412,7 +2471,7 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
 // the candidates are spread one per lane in level order (level_order,
 // wall_eval), and each particle's lane adds its results in candidate order
 // (wall_add).  The sum goes to Fw, and whoever reads the contact force adds it
-// to the pairs' (contact_sum), the addition the per-particle pass makes after
+// to the pairs' (add_walls), the addition the per-particle pass makes after
 // its pairs: so pairs and walls need no order between them and share a launch,
 // in which the few wall runs, each a long chain of FP64 region tests, run
 // beside the pairs' instead of after them.
@@ -2540,7 +2599,8 @@ template <bool RECORD, int HIST, bool COOP>
 __global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, ContactArgs C)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) C.counters[CN_REBUILD] = 0;
-    const unsigned total = C.counters[CN_HEAVY], front = C.counters[CN_HTRI];
+    // (with history every listed particle: a contact that has ended frees its entry)
+    const unsigned total = HIST ? C.counters[CN_HEAVY] : listed_now(P, C.counters), front = C.counters[CN_HTRI];
     // runs of consecutive list entries go to the warps of all blocks in turn:
     // every SM gets an equal share however short the list
     const unsigned warps = gridDim.x * (blockDim.x / 32u);
@@ -2558,12 +2618,12 @@ __global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, 
         for (unsigned t0 = (warps - 1u - gw) * run; t0 < total; t0 += warps * run) {
             const unsigned t = t0 + lane;
             const bool valid = lane < run && t < total;
-            contact_entry_coop(P, C, valid, valid ? __ldg(C.hlist + list_index(t, front, P.n)) : 0u, t < front, B.c);
+            contact_entry_coop(P, C, valid, valid ? __ldg(C.hlist + t) : 0u, t < front, B.c);
         }
         return;
     }
     for (unsigned t = gw * 32u + (threadIdx.x & 31u); t < total; t += warps * 32u)
-        contact_entry<RECORD, HIST>(P, C, __ldg(C.hlist + list_index(t, front, P.n)));
+        contact_entry<RECORD, HIST>(P, C, __ldg(C.hlist + t));
 }
 
 // Body reactions: rxn[(b * 6 + q) * n + i] summed over i in a fixed order,
@@ -2717,7 +2777,9 @@ __global__ void __launch_bounds__(256) k_mx_store_forces(MixParams P, Master M,
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
     const size_t o = __float_as_uint(M.wl[i].w);
-    const float4 f = contact_sum(Fc, Fw, i), t = Mc[i];
+    float4 f = Fc[i];
+    add_walls(f, Fw, i);
+    const float4 t = Mc[i];
     force[3 * o + 0] = f.x;
     force[3 * o + 1] = f.y;
     force[3 * o + 2] = f.z;
@@ -2866,6 +2928,8 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
     // skin less the FP32 position error, so no unlisted pair can touch.
     P.vcut = (float)skin + P.tol;
     P.disp2 = (float)((0.5 * skin - P.tol) * (0.5 * skin - P.tol));
+    P.gap_bin = P.vcut / (float)kGapBins;
+    P.inv_gap_bin = 1.0f / P.gap_bin;
     P.wall_tol = (float)(1e-5 + extent * 0x1p-20);
     const xd_contact_property& cp = d.cp_pp;
     double Eeq = (cp.Ei * cp.Ej) / (cp.Ei * (1 - cp.prj * cp.prj) + cp.Ej * (1 - cp.pri * cp.pri));
@@ -2939,6 +3003,7 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
     A(alloc(s, &s->Mc, n));
     A(alloc(s, &s->Fw, n));
     A(alloc(s, &s->hlist, n));
+    A(alloc(s, &s->lclass, n));
     A(alloc(s, &s->wmask, n));
     A(alloc(s, &s->vcount, n));
     A(alloc(s, &s->vlist, n * s->vcap));
@@ -3321,6 +3386,8 @@ static int rebuild(MixedScene* s, cudaStream_t q)
     if (st == XD_OK)
         st = cuda_status(cudaMemsetAsync(s->counters + CN_HTRI, 0, 2 * sizeof(unsigned), q), "mixed re-binning");
     if (st == XD_OK)
+        st = cuda_status(cudaMemsetAsync(s->counters + CN_BIN, 0, (kCounters - CN_BIN) * sizeof(unsigned), q), "mixed re-binning");
+    if (st == XD_OK)
         st = cuda_status(cudaMemsetAsync(s->counters + CN_VINC, 0, 4 * sizeof(unsigned), q), "mixed re-binning");
     if (st != XD_OK) return st;
     k_mx_keys<<<blocks(n, 256), 256, 0, q>>>(s->P, s->pf, s->keys, s->vals);
@@ -3351,8 +3418,9 @@ static int rebuild(MixedScene* s, cudaStream_t q)
     }
     if (st != XD_OK) return st;
     k_mx_build<<<blocks(n, 256), 256, 0, q>>>(s->P, s->pf, s->prev_keys, s->lb, s->vcount, s->vlist, s->pref,
-                                              s->wmask, s->tcount, s->rxn, s->hlist, s->Fc, s->Mc,
+                                              s->wmask, s->tcount, s->rxn, s->lclass, s->Fc, s->Mc,
                                               s->counters);
+    k_mx_list<<<blocks(n, 256), 256, 0, q>>>(s->P, s->lclass, s->hlist, s->counters);
     return launch_status("mixed re-binning");
 }
 
@@ -3668,10 +3736,10 @@ unsigned long long mixed_launches(MixedScene* s, unsigned nsteps)
 unsigned long long mixed_rebuild_launches(MixedScene* s)
 {
     if (!s || s->n == 0) return 0;
-    // keys, sort, permute, copy back, cell bounds (2), list build; with
+    // keys, sort, permute, copy back, cell bounds (2), list build (2); with
     // triangles also their lists, and for a mesh that moves on the device
     // its cell table (count, scan, fill, pad and their sort)
-    unsigned long long k = radix_sort_launches(s->n, key_bits_for(s->ncell)) + 6ull;
+    unsigned long long k = radix_sort_launches(s->n, key_bits_for(s->ncell)) + 7ull;
     if (s->ntri)
         k += 1 + (s->kinematic ? 4ull + radix_sort_launches(s->tpair_cap, key_bits_for(s->ncell + 1)) : 0ull);
     if (s->nbodies) k += 1;   // the reactions flushed first
@@ -4033,9 +4101,10 @@ __global__ void __launch_bounds__(256) k_batch_advance(const BatchScene* __restr
         if (i < sP.n) finish_one(sP, d.C.M, d.C.Fc, d.C.Mc, d.C.Fw, i);
         return;
     }
-    const bool out = i < sP.n && advance_one<MODE>(sP, d.C.M, d.C.Fc, d.C.Mc, d.C.Fw, d.pref, d.pf, d.qa, d.qb,
-                                                              d.pr, i);
-    if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) atomicOr(d.C.counters + CN_REBUILD, 1u);
+    const unsigned a = block_displacement(sP, i < sP.n ? advance_one<MODE>(sP, d.C.M, d.C.Fc, d.C.Mc, d.C.Fw, d.pref,
+                                                                           d.pf, d.qa, d.qb, d.pr, i)
+                                                       : 0.f);
+    if (threadIdx.x == 0) note_displacement(a, d.C.counters);
 }
 
 // Each scene's re-binning flag into flags[] (and cleared for the next step);
@@ -4069,18 +4138,24 @@ __global__ void k_batch_group(const unsigned* __restrict__ flags, unsigned first
     if (t < count && flags[first + t]) cudaGraphSetConditional(hs[first + t], 1u);
 }
 
+// A scene's particles for the wall runs (those with walls in reach) or the
+// pair runs.
+__device__ __forceinline__ unsigned batch_list(const BatchScene& d, bool walls)
+{
+    return walls ? d.C.counters[CN_HTRI] : listed_now(d.P, d.C.counters);
+}
+
 // Runs of listed particles per scene, as an exclusive prefix over scenes, of
-// counter word `cw` (CN_HEAVY: every listed particle; CN_HTRI: those with
-// walls in reach) into runs[0, ns]; runs[ns + 1] (the next free run) cleared,
+// the wall runs' or the pair runs' lists, into runs[0, ns]; runs[ns + 1] (the next free run) cleared,
 // and the particles a run holds (`each`, or with 0 run_size of all scenes'
 // together) in runs[ns + 2].
-__device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsigned cw, unsigned each,
+__device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, bool walls, unsigned each,
                            unsigned* __restrict__ runs, unsigned* c, unsigned& carry)
 {
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     unsigned all = 0;
-    for (unsigned sc = threadIdx.x; sc < ns; sc += 1024u) all += D[sc].C.counters[cw];
+    for (unsigned sc = threadIdx.x; sc < ns; sc += 1024u) all += batch_list(D[sc], walls);
     all = __reduce_add_sync(0xffffffffu, all);
     if ((threadIdx.x & 31u) == 0 && all) atomicAdd(&carry, all);
     __syncthreads();
@@ -4090,7 +4165,7 @@ __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, unsign
     __syncthreads();
     for (unsigned base = 0; base < ns; base += 1024u) {
         const unsigned sc = base + threadIdx.x;
-        const unsigned h = sc < ns ? D[sc].C.counters[cw] : 0u;
+        const unsigned h = sc < ns ? batch_list(D[sc], walls) : 0u;
         c[threadIdx.x] = (h + run - 1u) / run;
         __syncthreads();
         // inclusive scan (Hillis-Steele)
@@ -4120,8 +4195,8 @@ __global__ void __launch_bounds__(1024) k_batch_chunks(const BatchScene* __restr
 {
     __shared__ unsigned c[1024];
     __shared__ unsigned carry;
-    batch_runs(D, ns, CN_HEAVY, per_particle ? 32u : 0u, chunk_start, c, carry);
-    batch_runs(D, ns, CN_HTRI, kWallRun, chunk_start + ns + 3, c, carry);
+    batch_runs(D, ns, false, per_particle ? 32u : 0u, chunk_start, c, carry);
+    batch_runs(D, ns, true, kWallRun, chunk_start + ns + 3, c, carry);
 }
 
 // The contact pass of every scene: each warp takes the next kBatchGrab runs
@@ -4169,19 +4244,19 @@ __device__ __forceinline__ void batch_runs_of(const BatchScene* __restrict__ D, 
                 copy_words(&W.P, &D[cur].P, sizeof(MixParams), lane, 32u);
                 copy_words(&W.C, &D[cur].C, sizeof(ContactArgs), lane, 32u);
                 __syncwarp();
-                heavy = W.C.counters[CN_HEAVY];
+                heavy = listed_now(W.P, W.C.counters);
                 front = W.C.counters[CN_HTRI];
             }
             const unsigned t = (ch - lo) * run + lane;
             if (KIND == 1) {
                 const bool valid = lane < run && t < heavy;
-                contact_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + list_index(t, front, W.P.n)) : 0u,
+                contact_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + t) : 0u,
                                    t < front, B->c);
             } else if (KIND == 2) {
                 const bool valid = lane < run && t < front;
                 walls_entry_coop(W.P, W.C, valid, valid ? __ldg(W.C.hlist + t) : 0u, *B);
             } else if (t < heavy) {
-                contact_entry<false, 0>(W.P, W.C, __ldg(W.C.hlist + list_index(t, front, W.P.n)));
+                contact_entry<false, 0>(W.P, W.C, __ldg(W.C.hlist + t));
             }
         }
     }
