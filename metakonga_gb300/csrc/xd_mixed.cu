@@ -549,21 +549,61 @@ __device__ __forceinline__ long long fixed_q(double x, double off)
     return __double_as_longlong(__fma_rn(x, kQ, off)) - __double_as_longlong(kMagic);
 }
 
-// FP32 value of a fixed-point coordinate (|q| < 2^51), from two exact 32-bit
-// conversions (the 64-bit integer conversions run on the FP64 pipe).
-__device__ __forceinline__ float q_to_f(long long q)
+// Conversions in integer and FP32 instructions: the conversion instructions
+// issue on the FP64 pipe.  An integer in [-2^22, 2^22) added to the bits of
+// 1.5 * 2^23 is that float plus the integer; a normal float's exponent and
+// mantissa moved to a double's places.
+__device__ __forceinline__ float tiny_i2f(int a) { return __fsub_rn(__int_as_float(0x4B400000 + a), 12582912.0f); }
+__device__ __forceinline__ float small_i2f(int a)
 {
-    return __fmaf_rn(__int2float_rn((int)(q >> 20)), 0x1p-16f,
-                     __fmul_rn(__int2float_rn((int)(q & 0xfffff)), 0x1p-36f));
+    return (unsigned)(a + 0x400000) < 0x800000u ? tiny_i2f(a) : __int2float_rn(a);
+}
+__device__ __forceinline__ double f2d(float f)
+{
+    const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu;
+    if (a - 0x00800000u < 0x7f000000u)
+        return __hiloint2double((int)((b & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(b << 29));
+    return (double)f;
 }
 
-// The quantisation residual x - (wo + q 2^-36) in metres of a fixed-point
-// coordinate formed as t = fma(x, 2^36, off): the FMA's rounding error,
-// recovered by a second FMA (off - t is exact: both lie in [2^52, 2^53)).
-__device__ __forceinline__ float fixed_residual(double x, double off, long long q)
+// FP32 value of a fixed-point coordinate (|q| < 2^51), from two exact 32-bit
+// conversions (the low part has 20 bits).
+__device__ __forceinline__ float q_to_f(long long q)
 {
-    const double t = __longlong_as_double(q + __double_as_longlong(kMagic));
-    return (float)__fma_rn(x, kQ, off - t) * 0x1p-36f;
+    return __fmaf_rn(small_i2f((int)(q >> 20)), 0x1p-16f, __fmul_rn(tiny_i2f((int)(q & 0xfffff)), 0x1p-36f));
+}
+
+// fixed_q, and the quantisation residual x - (wo + q 2^-36) in metres as FP32:
+// the FMA's rounding error, which a second FMA recovers (t = the rounded sum;
+// off - t is exact: both lie in [2^52, 2^53)).
+//
+// A normal x whose last mantissa bit is worth 2^-1 to 2^-31 of the fixed-point
+// unit (2^-15 m <= |x| < 2^16 m) needs neither FMA: its mantissa, shifted by
+// that much, is the integer and the remainder, off is an integer (wo is a
+// multiple of the unit), and the remainder's FP32 value is one rounding of two
+// exact parts.  About 30 integer instructions for 4 of the FP64 pipe, where a
+// warp instruction takes 16 cycles of an SM; with the view's 16 and the 6
+// conversions of the drift the pipe bounded the advance (62 -> 55 us for
+// 1,000,000 spheres, 33 -> 27 for 500,000, 7.7 -> 6.4 for 20,000).
+__device__ __forceinline__ long long fixed_split(double x, double off, float& residual)
+{
+    const int hi = __double2hiint(x), s = 1039 - ((hi >> 20) & 0x7ff);
+    if (s >= 1 && s <= 31) {
+        const long long a = ((long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x);
+        const long long m = hi < 0 ? -a : a;
+        const long long base = (m >> s) + (__double_as_longlong(off) - __double_as_longlong(kMagic));
+        if ((unsigned)((int)(base >> 32) + 0x80000) < 0x100000u) {   // in fixed_q's range
+            const unsigned rest = (unsigned)m & ((1u << s) - 1u), half = 1u << (s - 1);
+            const unsigned up = rest + ((unsigned)base & 1u) > half ? 1u : 0u;   // ties to even
+            const int r = (int)(rest - (up << s));                               // |r| <= 2^30
+            residual = __fmul_rn(__fmaf_rn(tiny_i2f(r >> 12), 4096.f, tiny_i2f(r & 0xfff)),
+                                 __int_as_float((91 - s) << 23));
+            return base + up;
+        }
+    }
+    const long long q = fixed_q(x, off);
+    residual = (float)__fma_rn(x, kQ, off - __longlong_as_double(q + __double_as_longlong(kMagic))) * 0x1p-36f;
+    return q;
 }
 
 // The contact view of slot i: FP32 position and radius (pf), the int64 fixed
@@ -575,12 +615,12 @@ __device__ __forceinline__ float4 write_view(const MixParams& P, unsigned i, dou
                                              longlong2* __restrict__ qa, longlong2* __restrict__ qb,
                                              float4* __restrict__ pr)
 {
-    const long long qx = fixed_q(x, P.qoff[0]), qy = fixed_q(y, P.qoff[1]), qz = fixed_q(z, P.qoff[2]);
-    const long long qr = fixed_q(r, kMagic);
+    float4 e;
+    const long long qx = fixed_split(x, P.qoff[0], e.x), qy = fixed_split(y, P.qoff[1], e.y);
+    const long long qz = fixed_split(z, P.qoff[2], e.z), qr = fixed_split(r, kMagic, e.w);
     qa[i] = make_longlong2(qx, qy);
     qb[i] = make_longlong2(qz, qr);
-    pr[i] = make_float4(fixed_residual(x, P.qoff[0], qx), fixed_residual(y, P.qoff[1], qy),
-                        fixed_residual(z, P.qoff[2], qz), fixed_residual(r, kMagic, qr));
+    pr[i] = e;
     const float4 v = make_float4(q_to_f(qx), q_to_f(qy), q_to_f(qz), (float)r);
     pf[i] = v;
     return v;
@@ -695,15 +735,9 @@ __device__ __forceinline__ double drift(const MixParams& P, double x, float vhi,
     dfl inc = df_mul(df_of(P.dt_df), dfl{ vhi, vlo });
     inc = df_add(inc, df_of(P.G2[k]));
     inc = df_add_f(inc, P.half2dtf * ac);
-    return __dadd_rn(x, __dadd_rn((double)inc.hi, (double)inc.lo));
+    return __dadd_rn(x, __dadd_rn(f2d(inc.hi), f2d(inc.lo)));
 }
 
-// k_mx_advance: one step of the state in place (MODE as above), the contact
-// view, then the skin test on the new position: every particle must stay
-// within half the skin of its position at the last list build (pref); one
-// that does not sets CN_REBUILD.  The last block to finish passes the flag to
-// the graph's conditional node (use_cond), one caller as the conditional
-// requires.
 // Fc.w: what the contact pass left at a slot (zero: no contact, F = M = 0).
 constexpr float kHasWalls = 1.f, kHasPairs = 2.f;
 
@@ -786,6 +820,15 @@ __device__ __forceinline__ void note_displacement(unsigned a, unsigned* counters
     }
 }
 
+// k_mx_advance: one step of the state in place (MODE as above), the contact
+// view, then the skin test on the new position: every particle must stay
+// within half the skin of its position at the last list build (pref); one
+// that does not sets CN_REBUILD.  The last block to finish passes the flag to
+// the graph's conditional node (use_cond), one caller as the conditional
+// requires.
+//
+// 344 bytes a particle: 51 us for 1,000,000 at the copy rate, 55 measured (60
+// when the view came from the FP64 pipe, fixed_split).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_mx_advance(MixParams P, Master M, const float4* __restrict__ Fc,
                                                     const float4* __restrict__ Mc, const float4* __restrict__ Fw,
@@ -4086,8 +4129,12 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, unsigned 
 }
 
 // MODE 0: drift; MODE 1: kick then drift; MODE 2: kick only (the finish).
+//
+// 5 blocks an SM: 12 hoppers of 50,000 spheres take 35.5 us, with 4 blocks 37.3
+// (k_mx_advance spills at 48 registers and gains nothing: 55.9 us against 54.9
+// for 1,000,000 spheres).
 template <int MODE>
-__global__ void __launch_bounds__(256) k_batch_advance(const BatchScene* __restrict__ D,
+__global__ void __launch_bounds__(256, 5) k_batch_advance(const BatchScene* __restrict__ D,
                                                        const unsigned* __restrict__ block_scene, unsigned nblocks)
 {
     __shared__ MixParams sP;
