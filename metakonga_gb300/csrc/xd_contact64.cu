@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(256) k_update_polygon(const xd_polygon_mass_in
     unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= ntri) return;
     d3 Pv, Qv, Rv;
-    update_polygon_one(dpmi, vlist, sphere, dpi, id, Pv, Qv, Rv);
+    update_polygon_one(dpmi, nullptr, vlist, sphere, dpi, id, Pv, Qv, Rv);
 }
 
 // ----------------------------------------------------------- reductionD3
@@ -1002,54 +1002,80 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
 // One step of prescribed body motion (an extension; the reference moves its
 // bodies through the multibody solver on the host): origin += dt vel, the
 // Euler parameters p <- q (x) p with q the rotation of angle |omega| dt about
-// omega, normalised.  One thread per body.
-__global__ void k_body_advance(xd_polygon_mass_info* __restrict__ pmi, unsigned nbodies, double dt)
+// omega, normalised.  One thread per body.  The pose reached goes to pose (the
+// mixed form's, which the mesh update then takes and gives to the body: the
+// pose is computed while a contact pass still reads the body's), or in place.
+__global__ void k_body_advance(xd_polygon_mass_info* __restrict__ pmi, unsigned nbodies, double dt,
+                               double* __restrict__ pose, StepGate g)
 {
     const unsigned b = threadIdx.x;
-    if (b >= nbodies) return;
+    if (b >= nbodies || (g.words && !step_moves(g, step_todo(g.words)))) return;
     xd_polygon_mass_info* m = pmi + b;
-    for (int a = 0; a < 3; ++a) m->origin[a] = m->origin[a] + dt * m->vel[a];
+    double* o = pose ? pose + kPose * b : m->origin;
+    double* ep = pose ? pose + kPose * b + 3 : m->ep;
+    for (int a = 0; a < 3; ++a) o[a] = m->origin[a] + dt * m->vel[a];
+    const double p0 = m->ep[0], p1 = m->ep[1], p2 = m->ep[2], p3 = m->ep[3];
     const double wx = m->omega[0], wy = m->omega[1], wz = m->omega[2];
     const double w = sqrt(wx * wx + wy * wy + wz * wz);
     if (w > 0.0) {
         const double h = 0.5 * w * dt;
         const double c = cos(h), sn = sin(h) / w;
         const double a0 = c, a1 = sn * wx, a2 = sn * wy, a3 = sn * wz;
-        const double p0 = m->ep[0], p1 = m->ep[1], p2 = m->ep[2], p3 = m->ep[3];
         const double r0 = a0 * p0 - (a1 * p1 + a2 * p2 + a3 * p3);
         const double r1 = a0 * p1 + p0 * a1 + (a2 * p3 - a3 * p2);
         const double r2 = a0 * p2 + p0 * a2 + (a3 * p1 - a1 * p3);
         const double r3 = a0 * p3 + p0 * a3 + (a1 * p2 - a2 * p1);
         const double nr = sqrt(r0 * r0 + r1 * r1 + r2 * r2 + r3 * r3);
-        m->ep[0] = r0 / nr;
-        m->ep[1] = r1 / nr;
-        m->ep[2] = r2 / nr;
-        m->ep[3] = r3 / nr;
+        ep[0] = r0 / nr;
+        ep[1] = r1 / nr;
+        ep[2] = r2 / nr;
+        ep[3] = r3 / nr;
+    } else if (pose) {
+        ep[0] = p0;
+        ep[1] = p1;
+        ep[2] = p2;
+        ep[3] = p3;
     }
 }
 
-int launch_body_advance(xd_polygon_mass_info* pmi, unsigned nbodies, double dt, cudaStream_t s)
+int launch_body_advance(xd_polygon_mass_info* pmi, unsigned nbodies, double dt, cudaStream_t s, double* pose,
+                        const StepGate& g)
 {
     if (nbodies == 0) return XD_OK;
-    k_body_advance<<<1, 32, 0, s>>>(pmi, nbodies, dt);
+    k_body_advance<<<1, 32, 0, s>>>(pmi, nbodies, dt, pose, g);
     return launch_status("kinematic bodies");
 }
 
 // The mesh update and, for the mixed form, whether a vertex has moved from
 // its position at the last list build (ref: FP32, relative to the grid origin
 // wo) by disp2 or more: *flag is raised then.  rec (the mixed form's
-// triangle records) is rewritten from the new vertices.
-__global__ void __launch_bounds__(64) k_mesh_move(const xd_polygon_mass_info* __restrict__ dpmi,
-                                                  const double* __restrict__ vlist, double* __restrict__ sphere,
-                                                  xd_polygon_info* __restrict__ dpi, unsigned ntri,
-                                                  const float* __restrict__ ref, double wo0, double wo1, double wo2,
-                                                  float disp2, unsigned* __restrict__ flag, TriRec* __restrict__ rec)
+// triangle records) is rewritten from the new vertices.  pose (nullable): the
+// poses to place it at, which the bodies take over.  In a graph (g) it is
+// part of a step: it runs beside the advance, and its blocks count with the
+// advance's.
+constexpr unsigned kMeshThreads = 64;
+
+__global__ void __launch_bounds__(kMeshThreads) k_mesh_move(xd_polygon_mass_info* __restrict__ dpmi,
+                                                            const double* __restrict__ pose, unsigned nbodies,
+                                                            const double* __restrict__ vlist,
+                                                            double* __restrict__ sphere,
+                                                            xd_polygon_info* __restrict__ dpi, unsigned ntri,
+                                                            const float* __restrict__ ref, double wo0, double wo1,
+                                                            double wo2, float disp2, unsigned* __restrict__ flag,
+                                                            TriRec* __restrict__ rec, StepGate g)
 {
     const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned todo = g.words ? step_todo(g.words) : 0u;
+    if (g.words && todo == 0) return;
     bool out = false;
-    if (id < ntri) {
+    const bool moves = !g.words || step_moves(g, todo);
+    if (moves && pose && id < nbodies) {   // (nobody else reads the bodies' poses here)
+        for (int a = 0; a < 3; ++a) dpmi[id].origin[a] = pose[kPose * id + a];
+        for (int a = 0; a < 4; ++a) dpmi[id].ep[a] = pose[kPose * id + 3 + a];
+    }
+    if (id < ntri && moves) {
         d3 V[3];
-        update_polygon_one(dpmi, vlist, sphere, dpi, id, V[0], V[1], V[2]);
+        update_polygon_one(dpmi, pose, vlist, sphere, dpi, id, V[0], V[1], V[2]);
         if (rec) write_tri_rec(rec + id, V[0], V[1], V[2], (unsigned)dpi[id].id);
         const double wo[3] = { wo0, wo1, wo2 };
         for (int k = 0; k < 3; ++k) {
@@ -1062,16 +1088,25 @@ __global__ void __launch_bounds__(64) k_mesh_move(const xd_polygon_mass_info* __
             out |= !(d2 < disp2);
         }
     }
-    if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) atomicOr(flag, 1u);
+    if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) {
+        atomicOr(flag, 1u);
+        __threadfence();   // (before the block counts as done)
+    }
+    if (!g.words) return;
+    __syncthreads();
+    if (threadIdx.x == 0) step_end(g, todo);
 }
 
-int launch_mesh_move(const xd_polygon_mass_info* dpmi, const double* vlist, double* sphere, xd_polygon_info* dpi,
+unsigned mesh_move_blocks(unsigned ntri) { return div_up(ntri, kMeshThreads); }
+
+int launch_mesh_move(xd_polygon_mass_info* dpmi, const double* pose, unsigned nbodies, const double* vlist,
+                     double* sphere, xd_polygon_info* dpi,
                      unsigned ntri, const float* ref, const double wo[3], float disp2, unsigned* flag,
-                     TriRec* rec, cudaStream_t s)
+                     TriRec* rec, cudaStream_t s, const StepGate& g)
 {
     if (ntri == 0) return XD_OK;
-    k_mesh_move<<<div_up(ntri, 64), 64, 0, s>>>(dpmi, vlist, sphere, dpi, ntri, ref, wo[0], wo[1], wo[2], disp2,
-                                               flag, rec);
+    k_mesh_move<<<mesh_move_blocks(ntri), kMeshThreads, 0, s>>>(dpmi, pose, nbodies, vlist, sphere, dpi, ntri, ref,
+                                                                wo[0], wo[1], wo[2], disp2, flag, rec, g);
     return launch_status("mesh move");
 }
 

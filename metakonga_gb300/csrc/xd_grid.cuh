@@ -54,16 +54,71 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
                    double* moment, const double* mass, const unsigned* sidx,
                    const unsigned* cstart, const unsigned* cend, const xd_contact_property* cp,
                    unsigned nbodies, void* scratch, cudaStream_t s, const HistTable* ht = nullptr);
-int launch_body_advance(xd_polygon_mass_info* pmi, unsigned nbodies, double dt, cudaStream_t s);
+// The end of a graph step of the mixed form (its advance and, beside it, the
+// mesh update): blocks of both that have to finish, and the words they share
+// (nullptr: launched directly, nothing to gate).
+//   words[kStepDone]  blocks done (reset by the last one)
+//   words[kStepFlag]  a re-binning is due (raised by either)
+//   words[kStepStop]  the flag as the last finished step left it: the steps
+//                     that follow in the graph do nothing until it is cleared
+//   words[kStepTodo]  contact passes left in the call
+// first: the call's first advance (no contact pass precedes it).  tail: the
+// graph ends with this step: rebin is set where a re-binning is due, more (if
+// loop) where passes are left.
+enum { kStepFlag = 0, kStepDone = 1, kStepStop = 34, kStepTodo = 35 };   // (the last two in one 8-byte word)
+struct StepGate {
+    unsigned* words = nullptr;
+    unsigned blocks = 0;
+    int first = 0, tail = 0, loop = 0;
+    cudaGraphConditionalHandle rebin = 0, more = 0;
+};
+#ifdef __CUDACC__
+// Passes left as a kernel of the step finds them (0: nothing to do); an
+// advance moves something if step_moves.
+__device__ __forceinline__ unsigned step_todo(const unsigned* words)
+{
+    const uint2 w = __ldcg(reinterpret_cast<const uint2*>(words + kStepStop));   // one load: the kernel waits for it
+    return w.x ? 0u : w.y;
+}
+__device__ __forceinline__ bool step_moves(const StepGate& g, unsigned todo) { return todo >= (g.first ? 1u : 2u); }
+
+__device__ __forceinline__ void step_set(const StepGate& g, unsigned flag, unsigned left)
+{
+    // (the value is set either way: a loop's body does not reset it)
+    cudaGraphSetConditional(g.rebin, flag ? 1u : 0u);
+    if (g.loop) cudaGraphSetConditional(g.more, left ? 1u : 0u);
+}
+// A step that does nothing (step_todo 0), by one thread of it, at a graph's end.
+__device__ __forceinline__ void step_skip(const StepGate& g)
+{
+    if (g.tail) step_set(g, __ldcg(g.words + kStepStop), __ldcg(g.words + kStepTodo));
+}
+// One block of the step has finished (its thread 0; a flag it raised is visible):
+// the last one closes the step.
+__device__ __forceinline__ void step_end(const StepGate& g, unsigned todo)
+{
+    if (atomicAdd(g.words + kStepDone, 1u) != g.blocks - 1u) return;
+    __threadfence();
+    const unsigned flag = atomicOr(g.words + kStepFlag, 0u), left = g.first ? todo : todo - 1u;
+    g.words[kStepDone] = 0;
+    g.words[kStepStop] = flag ? 1u : 0u;
+    g.words[kStepTodo] = left;
+    if (g.tail) step_set(g, flag, left);
+}
+#endif
+int launch_body_advance(xd_polygon_mass_info* pmi, unsigned nbodies, double dt, cudaStream_t s,
+                        double* pose = nullptr, const StepGate& g = StepGate());
+unsigned mesh_move_blocks(unsigned ntri);
 int launch_update_polygon(const xd_polygon_mass_info* dpmi, const double* vlist, double* sphere,
                           xd_polygon_info* dpi, unsigned ntri, cudaStream_t s);
 // The mesh update with the mixed form's moved check in one launch (see
 // k_mesh_move): *flag raised when a vertex moved disp2 or more from ref; rec
 // (nullable) receives the triangle records of the new pose.
 struct TriRec;
-int launch_mesh_move(const xd_polygon_mass_info* dpmi, const double* vlist, double* sphere, xd_polygon_info* dpi,
+int launch_mesh_move(xd_polygon_mass_info* dpmi, const double* pose, unsigned nbodies, const double* vlist,
+                     double* sphere, xd_polygon_info* dpi,
                      unsigned ntri, const float* ref, const double wo[3], float disp2, unsigned* flag,
-                     TriRec* rec, cudaStream_t s);
+                     TriRec* rec, cudaStream_t s, const StepGate& g = StepGate());
 // The mixed form's triangle records of a mesh as it stands.
 int launch_tri_records(const xd_polygon_info* dpi, unsigned ntri, TriRec* rec, cudaStream_t s);
 int reduction_d3(const double* in, unsigned n, double out[3], void* scratch, cudaStream_t s);

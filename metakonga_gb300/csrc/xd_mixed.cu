@@ -22,8 +22,9 @@
 //                 particle's Verlet list holds the slots within ri + rj + skin
 //                 of it at the list build, so both stay valid while no
 //                 particle has moved half the skin since;
-//   re-binning    only when one has (a CUDA graph conditional node, or the
-//                 host between direct launches): cell keys, stable radix sort,
+//   re-binning    only when one has (a conditional node at the end of a CUDA
+//                 graph of up to eight steps, the rest of which is skipped, or
+//                 the host between direct launches): cell keys, stable radix sort,
 //                 the state permuted into the new cell order, k_lb_fill
 //                 (lb[c] = first slot whose key is >= c, for every cell, so a
 //                 row of three cells is the slot range [lb[c0], lb[c0 + 3])),
@@ -76,8 +77,8 @@ constexpr int kMaxBodies = 8;                  // polygon bodies of a mixed scen
 
 // Counter words.
 enum {
-    CN_REBUILD = 0,    // nonzero: this step re-bins (set by k_mx_advance, cleared by k_mx_contact)
-    CN_DONE = 1,       // blocks of k_mx_advance finished (last-block hand-off; reset by the last)
+    CN_REBUILD = kStepFlag,   // nonzero: a re-binning is due (set by k_mx_advance, cleared by the re-binning)
+    CN_DONE = kStepDone,      // blocks of a graph step's advance and mesh update finished (StepGate)
     CN_GAPS = 2,       // long gaps of the cell lower-bound array (re-binning)
     CN_HEAVY = 3,      // particles with Verlet neighbours or planes in reach (since the last build)
     CN_DECISIONS = 4,  // FP64 contact decisions (cumulative)
@@ -94,7 +95,9 @@ enum {
     CN_TSUM = 15,      // triangle-list entries at the last build
     CN_BIN = 16,       // listed particles by class at the last build: near walls, then by gap (kGapBins)
     CN_CUR = 25,       // k_mx_list's cursors of the classes
-    kCounters = 34
+    CN_STOP = kStepStop,   // a graph's later steps wait for a re-binning (StepGate)
+    CN_TODO = kStepTodo,   // contact passes left in the call (StepGate)
+    kCounters = 36
 };
 constexpr unsigned kGapBins = 8;
 
@@ -201,9 +204,9 @@ struct MixedScene {
     // triangle meshes (FP64, world frame) and their polygon bodies
     unsigned ntri = 0, nbodies = 0;
     xd_polygon_info* poly = nullptr;
-    double* sphere = nullptr;     // circumcentres (written by the mesh update)
     double* vlist_body = nullptr; // body-frame vertices [ntri][9]
     xd_polygon_mass_info* pmi = nullptr;
+    double* pose = nullptr;       // the bodies' next poses (k_body_advance), kPose words each
     float* tri_ref = nullptr;     // vertices at the last build, FP32 relative to the grid origin
     float4* tbound = nullptr;     // bounding sphere of each triangle at the last build (same frame)
     TriRec* trec = nullptr;       // the contact pass's triangle records of the current pose
@@ -244,7 +247,7 @@ struct MixedScene {
     // host-order transfer buffers
     double* xfer = nullptr;
     bool ready = false;                // grid and buffers set up (first upload)
-    cudaGraphExec_t graph[5] = {};   // first step; 1, 2, 4 and 8 middle steps
+    cudaGraphExec_t graph[6] = {};   // step graphs (kFirstStep to kLoop)
     // tangential-spring history (an extension): [s * n + slot] tables in the
     // state's slot order, permuted with the particles at re-binning
     unsigned hslots = 0;
@@ -823,9 +826,8 @@ __device__ __forceinline__ void note_displacement(unsigned a, unsigned* counters
 // k_mx_advance: one step of the state in place (MODE as above), the contact
 // view, then the skin test on the new position: every particle must stay
 // within half the skin of its position at the last list build (pref); one
-// that does not sets CN_REBUILD.  The last block to finish passes the flag to
-// the graph's conditional node (use_cond), one caller as the conditional
-// requires.
+// that does not sets CN_REBUILD.  In a graph the last block of the step closes
+// it (StepGate).
 //
 // 344 bytes a particle: 51 us for 1,000,000 at the copy rate, 55 measured (60
 // when the view came from the FP64 pipe, fixed_split).
@@ -835,30 +837,49 @@ __global__ void __launch_bounds__(256) k_mx_advance(MixParams P, Master M, const
                                                     const float4* __restrict__ pref,
                                                     float4* __restrict__ pf, longlong2* __restrict__ qa,
                                                     longlong2* __restrict__ qb, float4* __restrict__ pr,
-                                                    unsigned* __restrict__ counters,
-                                                    cudaGraphConditionalHandle cond, int use_cond)
+                                                    unsigned* __restrict__ counters, StepGate g)
 {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned todo = g.words ? step_todo(g.words) : 0u;
+    if (g.words && todo == 0) {
+        if (i == 0) step_skip(g);
+        return;
+    }
+    const bool moves = i < P.n && (!g.words || step_moves(g, todo));
     const unsigned a =
-        block_displacement(P, i < P.n ? advance_one<MODE>(P, M, Fc, Mc, Fw, pref, pf, qa, qb, pr, i) : 0.f);
+        block_displacement(P, moves ? advance_one<MODE>(P, M, Fc, Mc, Fw, pref, pf, qa, qb, pr, i) : 0.f);
     if (threadIdx.x != 0) return;
     // only the flag must be visible to the last block: the state and view
     // writes need no ordering here
     note_displacement(a, counters);
-    if (atomicAdd(counters + CN_DONE, 1u) != gridDim.x - 1) return;
-    __threadfence();
-    const unsigned f = atomicOr(counters + CN_REBUILD, 0u) ? 1u : 0u;
-    // the handle's default (0, assigned at every graph launch) stands
-    // unless a re-binning is due
-    if (use_cond && f) cudaGraphSetConditional(cond, 1u);
-    counters[CN_DONE] = 0;
+    if (g.words) step_end(g, todo);
 }
 
-// Re-binning, 1: the cell key of every slot's current position.
+// The first kernel of a call of `todo` steps in graphs.
+__global__ void k_call_begin(unsigned* __restrict__ words, unsigned todo, int rebin)
+{
+    words[kStepTodo] = todo;
+    words[kStepStop] = 0;
+    words[kStepDone] = 0;
+    if (rebin) words[kStepFlag] = 1;
+}
+
+// Ahead of the loop over what a call's graphs have left.
+__global__ void k_call_left(const unsigned* __restrict__ words, cudaGraphConditionalHandle more)
+{
+    if (__ldcg(words + kStepTodo)) cudaGraphSetConditional(more, 1u);
+}
+
+// Re-binning, 1: the cell key of every slot's current position; the words that
+// the re-binning fills, cleared.
 __global__ void __launch_bounds__(256) k_mx_keys(MixParams P, const float4* __restrict__ pf,
-                                                 unsigned* __restrict__ keys, unsigned* __restrict__ vals)
+                                                 unsigned* __restrict__ keys, unsigned* __restrict__ vals,
+                                                 unsigned* __restrict__ counters)
 {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kCounters && (i == CN_GAPS || i == CN_HEAVY || i == CN_HTRI || i == CN_DMAX ||
+                          (i >= CN_VINC && i <= CN_TSUM) || (i >= CN_BIN && i < CN_BIN + 2 * (kGapBins + 1))))
+        counters[i] = 0;
     if (i >= P.n) return;
     const float4 p = pf[i];
     keys[i] = cell_key(P, p.x, p.y, p.z);
@@ -1382,6 +1403,7 @@ __global__ void __launch_bounds__(256) k_mx_list(MixParams P, const unsigned cha
 {
     __shared__ unsigned cnt[kGapBins + 1], base[kGapBins + 1];
     const unsigned tid = threadIdx.x, i = blockIdx.x * blockDim.x + tid;
+    if (i == 0) counters[CN_REBUILD] = counters[CN_STOP] = 0;   // the re-binning's last kernel
     if (tid <= kGapBins) cnt[tid] = 0;
     __syncthreads();
     const unsigned c = i < P.n ? (unsigned)lclass[i] : kUnlisted;
@@ -1688,8 +1710,6 @@ __device__ __forceinline__ void accumulate(PairAcc& A, const PairOut& o)
 // prefilter, exact integer test, FP64 guard band, FP32 Hertz-Mindlin -- then
 // plane_contact_force_kernel<1> (impl:572-621) for the planes in reach, in
 // FP64, in plane order (the others are out of reach and add exactly zero).
-// Block 0 clears CN_REBUILD for the next step's skin test.
-
 
 // The pointers of one scene the contact pass reads and writes.
 struct ContactArgs {
@@ -2633,21 +2653,26 @@ __host__ __device__ __forceinline__ unsigned run_size(unsigned total, unsigned w
     return run < kRunMin ? kRunMin : run;
 }
 
+// gate: the scene's counters in a graph, where nothing is done while a
+// re-binning is due or once the call's passes are done (StepGate).
+//
 // COOP: the warp-cooperative passes (no history, no recording; dynamic shared
 // memory of one WallBuf per warp): the wall runs first, from the first warp
 // on, and the pair runs from the last warp on, so that the warps with a wall
 // run are those with the fewest pair runs.  A 199,583-sphere hopper 62 us a
 // step (62 and, after them, 16.5 with the walls in a launch of their own).
 template <bool RECORD, int HIST, bool COOP>
-__global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, ContactArgs C)
+__global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, ContactArgs C,
+                                                                  const unsigned* __restrict__ gate)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) C.counters[CN_REBUILD] = 0;
+    const bool skip = gate && step_todo(gate) == 0;
     // (with history every listed particle: a contact that has ended frees its entry)
     const unsigned total = HIST ? C.counters[CN_HEAVY] : listed_now(P, C.counters), front = C.counters[CN_HTRI];
     // runs of consecutive list entries go to the warps of all blocks in turn:
     // every SM gets an equal share however short the list
     const unsigned warps = gridDim.x * (blockDim.x / 32u);
     const unsigned gw = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
+    if (skip) return;
     if (COOP) {
         extern __shared__ WallBuf wall_buf[];
         WallBuf& B = wall_buf[threadIdx.x / 32u];
@@ -3104,9 +3129,9 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
                              span * span * span);
         s->tpair_cap = (unsigned)cap;
         A(alloc(s, &s->poly, s->ntri));
-        A(alloc(s, &s->sphere, 4 * (size_t)s->ntri));
         A(alloc(s, &s->vlist_body, 9 * (size_t)s->ntri));
         A(alloc(s, &s->pmi, s->nbodies));
+        A(alloc(s, &s->pose, kPose * (size_t)s->nbodies));
         A(alloc(s, &s->tri_ref, 9 * (size_t)s->ntri));
         A(alloc(s, &s->tbound, (size_t)s->ntri));
         A(alloc(s, &s->trec, (size_t)s->ntri));
@@ -3122,7 +3147,6 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
         A(alloc(s, &s->rxn_part, (size_t)6 * s->nbodies * kRxnBlocks));
         if (st == XD_OK) {
             A(cuda_status(cudaMemcpy(s->poly, d.poly, sizeof(xd_polygon_info) * s->ntri, cudaMemcpyHostToDevice), "mixed mesh"));
-            A(cuda_status(cudaMemcpy(s->sphere, d.sphere, sizeof(double) * 4 * s->ntri, cudaMemcpyHostToDevice), "mixed mesh"));
             A(cuda_status(cudaMemcpy(s->vlist_body, d.vlist, sizeof(double) * 9 * s->ntri, cudaMemcpyHostToDevice), "mixed mesh"));
             A(cuda_status(cudaMemcpy(s->pmi, d.pmi, sizeof(xd_polygon_mass_info) * s->nbodies, cudaMemcpyHostToDevice), "mixed mesh"));
             A(launch_tri_records(s->poly, s->ntri, s->trec, 0));
@@ -3445,15 +3469,7 @@ static int rebuild(MixedScene* s, cudaStream_t q)
     const unsigned n = s->n;
     int st = flush_reactions(s, q);
     if (st != XD_OK) return st;
-    st = cuda_status(cudaMemsetAsync(s->counters + CN_GAPS, 0, 2 * sizeof(unsigned), q), "mixed re-binning");
-    if (st == XD_OK)
-        st = cuda_status(cudaMemsetAsync(s->counters + CN_HTRI, 0, 2 * sizeof(unsigned), q), "mixed re-binning");
-    if (st == XD_OK)
-        st = cuda_status(cudaMemsetAsync(s->counters + CN_BIN, 0, (kCounters - CN_BIN) * sizeof(unsigned), q), "mixed re-binning");
-    if (st == XD_OK)
-        st = cuda_status(cudaMemsetAsync(s->counters + CN_VINC, 0, 4 * sizeof(unsigned), q), "mixed re-binning");
-    if (st != XD_OK) return st;
-    k_mx_keys<<<blocks(n, 256), 256, 0, q>>>(s->P, s->pf, s->keys, s->vals);
+    k_mx_keys<<<blocks(n, 256), 256, 0, q>>>(s->P, s->pf, s->keys, s->vals, s->counters);
     st = launch_status("mixed keys");
     if (st != XD_OK) return st;
     unsigned *sk = nullptr, *sv = nullptr;
@@ -3495,7 +3511,7 @@ static int update_mesh(MixedScene* s, cudaStream_t q)
     if (!s->ntri) return XD_OK;
     int st = XD_OK;
     if (s->bodies_dirty) {
-        st = launch_mesh_move(s->pmi, s->vlist_body, s->sphere, s->poly, s->ntri, s->tri_ref, s->P.wo,
+        st = launch_mesh_move(s->pmi, nullptr, 0, s->vlist_body, nullptr, s->poly, s->ntri, s->tri_ref, s->P.wo,
                               s->P.disp2, s->counters + CN_REBUILD, s->trec, q);
         if (st != XD_OK) return st;
         s->bodies_dirty = false;
@@ -3515,9 +3531,10 @@ static int update_mesh(MixedScene* s, cudaStream_t q)
 }
 
 // Inside a stream capture: a conditional node that runs body(s, stream) when
-// the handle is set (by k_mx_keys); the capture continues after it.
+// (or, as a loop, while) the handle is set; the capture continues after it.
 template <typename Body>
-static int capture_conditional(MixedScene* s, cudaStream_t q, cudaGraphConditionalHandle h, Body body)
+static int capture_conditional(MixedScene* s, cudaStream_t q, cudaGraphConditionalHandle h, Body body,
+                               cudaGraphConditionalNodeType type = cudaGraphCondTypeIf)
 {
     cudaStreamCaptureStatus cst;
     cudaGraph_t g = nullptr;
@@ -3527,7 +3544,7 @@ static int capture_conditional(MixedScene* s, cudaStream_t q, cudaGraphCondition
     if (st != XD_OK) return st;
     cudaGraphNodeParams np = { cudaGraphNodeTypeConditional };
     np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeIf;
+    np.conditional.type = type;
     np.conditional.size = 1;
     cudaGraphNode_t node = nullptr;
     st = cuda_status(cudaGraphAddNode(&node, g, deps, nullptr, nd, &np), "mixed conditional node");
@@ -3549,10 +3566,6 @@ static int capture_conditional(MixedScene* s, cudaStream_t q, cudaGraphCondition
                        "mixed capture dependencies");
 }
 
-// One step: the state advanced in place with the skin test, re-binning when
-// a particle has left its skin (or the cells are not set up), then the
-// contact forces.  cond: the conditional handle when capturing into a graph
-// (nullptr for direct launches, where the host reads the flag).
 static ContactArgs contact_args(MixedScene* s, unsigned* rc, unsigned* rp, unsigned rec_cap, const HistTable& ht,
                                 int rxn_on)
 {
@@ -3592,45 +3605,62 @@ static ContactArgs contact_args(MixedScene* s, unsigned* rc, unsigned* rp, unsig
     return C;
 }
 
+// The state advanced in place with the skin test and, for a mesh that moves on
+// the device, the pose and the triangles; the flag is raised once a particle or
+// a vertex has left half the skin.  gate: the step's part in a graph (its
+// blocks are filled in here), where the mesh moves on a branch beside the
+// advance, and its next pose is computed beside the contact pass before
+// (capture_chunk): of a 500,000-sphere drum's step the pose took 9 us, the mesh
+// 21 and then the advance 27; mesh and advance together take 31, the step
+// 217 -> 187.
+struct MeshBranch {
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+
+// In a capture: what follows on b comes after a.
+static int after(cudaStream_t a, cudaStream_t b, cudaEvent_t ev)
+{
+    const int st = cuda_status(cudaEventRecord(ev, a), "mixed mesh branch");
+    return st == XD_OK ? cuda_status(cudaStreamWaitEvent(b, ev, 0), "mixed mesh branch") : st;
+}
+
 template <int MODE>
-static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool record, unsigned rec_cap,
-                     const cudaGraphConditionalHandle* cond)
+static int advance_step(MixedScene* s, cudaStream_t q, const Phases& ph, StepGate g, const MeshBranch& mb)
 {
     const unsigned n = s->n;
-    const Master& M = s->m[0];
+    const bool mesh = s->kinematic && s->ntri && MODE != 3;
+    g.blocks = blocks(n, 256) + (mesh ? mesh_move_blocks(s->ntri) : 0u);
     int st = XD_OK;
-    if (s->kinematic && s->ntri && MODE != 3) {
-        // prescribed body motion: pose, triangles, and the re-binning flag
-        // once a vertex has moved half the skin since the last build
-        st = launch_body_advance(s->pmi, s->nbodies, s->P.dt, q);
+    if (mesh) {
+        cudaStream_t mq = q;
+        if (g.words) {
+            mq = mb.side;
+            st = after(q, mq, mb.fork);
+            if (st == XD_OK && g.first) st = launch_body_advance(s->pmi, s->nbodies, s->P.dt, mq, s->pose, g);
+        } else {
+            st = launch_body_advance(s->pmi, s->nbodies, s->P.dt, mq, s->pose);
+        }
         if (st == XD_OK)
-            st = launch_mesh_move(s->pmi, s->vlist_body, s->sphere, s->poly, s->ntri, s->tri_ref, s->P.wo,
-                                  s->P.disp2, s->counters + CN_REBUILD, s->trec, q);
+            st = launch_mesh_move(s->pmi, s->pose, s->nbodies, s->vlist_body, nullptr, s->poly, s->ntri, s->tri_ref,
+                                  s->P.wo, s->P.disp2, s->counters + CN_REBUILD, s->trec, mq, g);
         if (st != XD_OK) return st;
     }
     ph.begin(0, q);
-    k_mx_advance<MODE><<<blocks(n, 256), 256, 0, q>>>(s->P, M, s->Fc, s->Mc, s->Fw, s->pref, s->pf, s->qa, s->qb, s->pr,
-                                                      s->counters, cond ? *cond : 0, cond ? 1 : 0);
+    k_mx_advance<MODE><<<blocks(n, 256), 256, 0, q>>>(s->P, s->m[0], s->Fc, s->Mc, s->Fw, s->pref, s->pf, s->qa, s->qb,
+                                                      s->pr, s->counters, g);
     st = launch_status("mixed advance");
     ph.end(0, q);
-    if (st != XD_OK) return st;
-    ph.begin(2, q);
-    if (cond) {
-        st = capture_conditional(s, q, *cond, rebuild);
-    } else {
-        bool need = !s->cells_clean;
-        if (!need) {
-            unsigned flag = 0;
-            st = cuda_status(cudaMemcpyAsync(&flag, s->counters + CN_REBUILD, sizeof(unsigned),
-                                             cudaMemcpyDeviceToHost, q), "mixed re-binning flag");
-            if (st == XD_OK) st = cuda_status(cudaStreamSynchronize(q), "mixed re-binning flag");
-            need = flag != 0;
-        }
-        if (st == XD_OK && need) st = rebuild(s, q);
-    }
-    ph.end(2, q);
-    if (st != XD_OK) return st;
-    s->cells_clean = true;
+    if (st == XD_OK && mesh && g.words) st = after(mb.side, q, mb.join);
+    return st;
+}
+
+// The contact forces of the current state.
+template <int MODE>
+static int contact_step(MixedScene* s, cudaStream_t q, const Phases& ph, bool record, unsigned rec_cap, bool gated)
+{
+    const unsigned n = s->n;
+    int st = XD_OK;
     ph.begin(3, q);
     // the list holds at most n particles: no more warps than there are runs of
     // kRunMin of them (of 32 in the per-particle pass)
@@ -3648,7 +3678,8 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
         rp = s->rec_pairs;
     }
     const ContactArgs C = contact_args(s, rc, rp, record ? rec_cap : 0u, ht, MODE == 3 ? 0 : 1);
-#define XD_MX_CONTACT(REC, H) k_mx_contact<REC, H, false><<<grid, ct, 0, q>>>(s->P, C)
+    const unsigned* gate = gated ? s->counters : nullptr;
+#define XD_MX_CONTACT(REC, H) k_mx_contact<REC, H, false><<<grid, ct, 0, q>>>(s->P, C, gate)
     if (record) {
         if (hist == 2) XD_MX_CONTACT(true, 2);
         else if (hist == 1) XD_MX_CONTACT(true, 1);
@@ -3656,7 +3687,7 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
     } else {
         if (hist == 2) XD_MX_CONTACT(false, 2);
         else if (hist == 1) XD_MX_CONTACT(false, 1);
-        else if (s->cmode == 1) k_mx_contact<false, 0, true><<<grid, ct, (ct / 32u) * sizeof(WallBuf), q>>>(s->P, C);
+        else if (s->cmode == 1) k_mx_contact<false, 0, true><<<grid, ct, (ct / 32u) * sizeof(WallBuf), q>>>(s->P, C, gate);
         else XD_MX_CONTACT(false, 0);
     }
 #undef XD_MX_CONTACT
@@ -3665,13 +3696,43 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
     return st;
 }
 
-// Step graphs of a scene: kFirstStep (the first step of a call, MODE 0) and
-// graphs of 1, 2, 4 and 8 middle steps (MODE 1), each step with its own
-// conditional re-binning node; a call replays the first step, then runs of
-// eight, then the binary digits of what is left.
-enum { kFirstStep = 0, kSteps1 = 1, kSteps2 = 2, kSteps4 = 3, kSteps8 = 4, kGraphKinds = 5 };
+// One directly launched step: the host reads the flag and re-bins where a
+// particle has left its skin (or the cells are not set up).
+template <int MODE>
+static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool record, unsigned rec_cap)
+{
+    int st = advance_step<MODE>(s, q, ph, StepGate(), MeshBranch());
+    if (st != XD_OK) return st;
+    ph.begin(2, q);
+    bool need = !s->cells_clean;
+    if (!need) {
+        unsigned flag = 0;
+        st = cuda_status(cudaMemcpyAsync(&flag, s->counters + CN_REBUILD, sizeof(unsigned), cudaMemcpyDeviceToHost, q),
+                         "mixed re-binning flag");
+        if (st == XD_OK) st = cuda_status(cudaStreamSynchronize(q), "mixed re-binning flag");
+        need = flag != 0;
+    }
+    if (st == XD_OK && need) st = rebuild(s, q);
+    ph.end(2, q);
+    if (st != XD_OK) return st;
+    s->cells_clean = true;
+    return contact_step<MODE>(s, q, ph, record, rec_cap, false);
+}
 
-static unsigned graph_steps(int kind) { return kind == kFirstStep ? 1u : 1u << (kind - 1); }
+// Step graphs of a scene.  kFirstStep is the call's first advance (MODE 0),
+// kSteps1 to kSteps8 are 1, 2, 4 and 8 times a contact pass and the advance to
+// the next step, and each ends with a conditional node that re-bins.  Where an
+// advance inside a graph finds that a re-binning is due, the rest of the graph's
+// kernels do nothing (StepGate) and the node at its end re-bins; kLoop runs
+// eight-step graphs while passes are left, so a call takes all its steps and
+// never waits for the GPU.
+//
+// A conditional node between an advance and its contact pass costs 7 us (a
+// kernel after a kernel 0.4).  One in eight steps instead of one a step: 8,000
+// spheres 25 -> 18 us a step, 199,583 80 -> 75, 1,000,000 115 -> 108.  A skipped
+// kernel costs 1 to 2 us, so what eight steps save, a re-binning amid them loses
+// again in part; scenes that re-bin on every step take about as long as before.
+enum { kFirstStep = 0, kSteps1 = 1, kSteps2 = 2, kSteps4 = 3, kSteps8 = 4, kLoop = 5, kGraphKinds = 6 };
 
 constexpr unsigned kGraphMinSteps = 16;
 
@@ -3685,33 +3746,93 @@ static void destroy_graphs(MixedScene* s)
         }
 }
 
+// `steps` contact passes with the advance to the next step (0: the call's first
+// advance) and the re-binning node, into the capture on q.
+static int capture_chunk(MixedScene* s, cudaStream_t q, unsigned steps, const MeshBranch& mb,
+                         const cudaGraphConditionalHandle* more)
+{
+    cudaStreamCaptureStatus cst;
+    cudaGraph_t cg = nullptr;
+    StepGate g;
+    int st = cuda_status(cudaStreamGetCaptureInfo(q, &cst, nullptr, &cg), "mixed capture info");
+    if (st == XD_OK)
+        st = cuda_status(cudaGraphConditionalHandleCreate(&g.rebin, cg, 0, cudaGraphCondAssignDefault),
+                         "mixed conditional handle");
+    if (st != XD_OK) return st;
+    g.words = s->counters;
+    g.first = steps == 0;
+    if (more) {
+        g.loop = 1;
+        g.more = *more;
+    }
+    Phases none;
+    if (steps == 0) {
+        g.tail = 1;
+        st = advance_step<0>(s, q, none, g, mb);
+    }
+    for (unsigned k = 0; k < steps && st == XD_OK; ++k) {
+        g.tail = k + 1 == steps;
+        if (s->kinematic && s->ntri) {
+            st = after(q, mb.side, mb.fork);
+            if (st == XD_OK) st = launch_body_advance(s->pmi, s->nbodies, s->P.dt, mb.side, s->pose, g);
+            if (st != XD_OK) break;
+        }
+        st = contact_step<1>(s, q, none, false, 0, true);
+        if (st == XD_OK) st = advance_step<1>(s, q, none, g, mb);
+    }
+    return st == XD_OK ? capture_conditional(s, q, g.rebin, rebuild) : st;
+}
+
 static int capture_steps(MixedScene* s, int kind)
 {
     cudaStream_t cs = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_status(e, "mixed graph stream");
-    e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    int st = cuda_status(e, "mixed graph capture");
-    cudaGraph_t cg = nullptr;
-    cudaGraphConditionalHandle h[8] = {};
-    if (st == XD_OK) {
-        cudaStreamCaptureStatus cst;
-        st = cuda_status(cudaStreamGetCaptureInfo(cs, &cst, nullptr, &cg), "mixed capture info");
+    MeshBranch mb;
+    int st = XD_OK;
+    if (s->kinematic && s->ntri) {
+        // (the mesh's blocks ahead of the advance's, which fill every SM)
+        int low = 0, high = 0;
+        st = cuda_status(cudaDeviceGetStreamPriorityRange(&low, &high), "mixed mesh branch");
+        if (st == XD_OK)
+            st = cuda_status(cudaStreamCreateWithPriority(&mb.side, cudaStreamNonBlocking, high), "mixed mesh branch");
+        if (st == XD_OK) st = cuda_status(cudaEventCreateWithFlags(&mb.fork, cudaEventDisableTiming), "mixed mesh branch");
+        if (st == XD_OK) st = cuda_status(cudaEventCreateWithFlags(&mb.join, cudaEventDisableTiming), "mixed mesh branch");
     }
-    const unsigned nh = graph_steps(kind);
-    for (unsigned k = 0; k < nh && st == XD_OK; ++k)
-        st = cuda_status(cudaGraphConditionalHandleCreate(&h[k], cg, 0, cudaGraphCondAssignDefault),
-                         "mixed conditional handle");
-    const bool clean = s->cells_clean;
-    Phases none;
-    for (unsigned k = 0; k < nh && st == XD_OK; ++k)
-        st = kind == kFirstStep ? step_once<0>(s, cs, none, false, 0, &h[k]) : step_once<1>(s, cs, none, false, 0, &h[k]);
-    s->cells_clean = clean;   // capture only recorded the launches
+    bool capturing = false;
+    if (st == XD_OK) {
+        st = cuda_status(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "mixed graph capture");
+        capturing = st == XD_OK;
+    }
+    if (st == XD_OK && kind == kLoop) {
+        cudaStreamCaptureStatus cst;
+        cudaGraph_t cg = nullptr;
+        cudaGraphConditionalHandle more = 0;
+        st = cuda_status(cudaStreamGetCaptureInfo(cs, &cst, nullptr, &cg), "mixed capture info");
+        if (st == XD_OK)
+            st = cuda_status(cudaGraphConditionalHandleCreate(&more, cg, 0, cudaGraphCondAssignDefault),
+                             "mixed conditional handle");
+        if (st == XD_OK) {
+            k_call_left<<<1, 1, 0, cs>>>(s->counters, more);
+            st = launch_status("mixed loop");
+        }
+        if (st == XD_OK)
+            st = capture_conditional(
+                s, cs, more, [&](MixedScene* sc, cudaStream_t q) { return capture_chunk(sc, q, 8, mb, &more); },
+                cudaGraphCondTypeWhile);
+    } else if (st == XD_OK) {
+        st = capture_chunk(s, cs, kind == kFirstStep ? 0u : 1u << (kind - 1), mb, nullptr);
+    }
     cudaGraph_t g = nullptr;
-    e = cudaStreamEndCapture(cs, &g);
-    if (st == XD_OK) st = cuda_status(e, "mixed graph capture");
+    if (capturing) {
+        e = cudaStreamEndCapture(cs, &g);
+        if (st == XD_OK) st = cuda_status(e, "mixed graph capture");
+    }
     if (st == XD_OK) st = cuda_status(cudaGraphInstantiate(&s->graph[kind], g, 0), "mixed graph instantiate");
     if (g) cudaGraphDestroy(g);
+    if (mb.fork) cudaEventDestroy(mb.fork);
+    if (mb.join) cudaEventDestroy(mb.join);
+    if (mb.side) cudaStreamDestroy(mb.side);
     cudaStreamDestroy(cs);
     return st;
 }
@@ -3736,7 +3857,7 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
         int st = XD_OK;
         for (unsigned t = 0; t < nsteps && st == XD_OK; ++t) {
             st = launch_body_advance(s->pmi, s->nbodies, s->P.dt, q);
-            if (st == XD_OK) st = launch_update_polygon(s->pmi, s->vlist_body, s->sphere, s->poly, s->ntri, q);
+            if (st == XD_OK) st = launch_update_polygon(s->pmi, s->vlist_body, nullptr, s->poly, s->ntri, q);
         }
         if (st == XD_OK) st = launch_tri_records(s->poly, s->ntri, s->trec, q);
         s->cells_clean = false;
@@ -3757,19 +3878,22 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
         // of any length only replay
         for (int kind = 0; kind < kGraphKinds && st == XD_OK; ++kind)
             if (!s->graph[kind]) st = capture_steps(s, kind);
-        if (st == XD_OK && !s->cells_clean)
-            st = cuda_status(cudaMemsetAsync(s->counters + CN_REBUILD, 1, 1, q), "mixed re-binning flag");
+        if (st != XD_OK) return st;
+        k_call_begin<<<1, 1, 0, q>>>(s->counters, nsteps, s->cells_clean ? 0 : 1);
+        st = launch_status("mixed call");
         if (st == XD_OK) st = launch_steps(s, kFirstStep, q);
-        unsigned left = nsteps - 1;
+        unsigned left = nsteps;
         for (; st == XD_OK && left >= 8; left -= 8) st = launch_steps(s, kSteps8, q);
         for (int kind = kSteps4; kind >= kSteps1 && st == XD_OK; --kind)
-            if (left & graph_steps(kind)) st = launch_steps(s, kind, q);
+            if (left & (1u << (kind - 1))) st = launch_steps(s, kind, q);
+        // (single steps never fall short)
+        if (st == XD_OK && nsteps > 1) st = launch_steps(s, kLoop, q);
         if (st != XD_OK) return st;
         s->cells_clean = true;
     } else {
         // direct launches (phase timing): the host reads the re-binning flag
-        st = step_once<0>(s, q, ph, false, 0, nullptr);
-        for (unsigned t = 1; t < nsteps && st == XD_OK; ++t) st = step_once<1>(s, q, ph, false, 0, nullptr);
+        st = step_once<0>(s, q, ph, false, 0);
+        for (unsigned t = 1; t < nsteps && st == XD_OK; ++t) st = step_once<1>(s, q, ph, false, 0);
         if (st != XD_OK) return st;
     }
     // the last velocity update, and the call's body reactions
@@ -3788,10 +3912,11 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
 unsigned long long mixed_launches(MixedScene* s, unsigned nsteps)
 {
     if (!s || nsteps == 0 || s->n == 0) return 0;
-    // per step: advance + contact; + the last velocity update; a step that
-    // re-bins adds mixed_rebuild_launches()
-    const unsigned long long per = 2 + (s->kinematic && s->ntri ? 3 : 0);
-    unsigned long long total = per * nsteps + 1 + (s->nbodies ? 1 : 0);
+    // per step: advance + contact (and pose + mesh); + the first kernel of the
+    // call and the last velocity update; a step that re-bins adds
+    // mixed_rebuild_launches() (launches that skip are not counted)
+    const unsigned long long per = 2 + (s->kinematic && s->ntri ? 2 : 0);
+    unsigned long long total = per * nsteps + 2 + (s->nbodies ? 1 : 0);
     if (!s->cells_clean) total += mixed_rebuild_launches(s);   // the first step re-bins
     return total;
 }
@@ -3827,7 +3952,7 @@ static int current_contacts(MixedScene* s, cudaStream_t q, bool record, unsigned
     Phases none;
     int st = update_mesh(s, q);
     if (st != XD_OK) return st;
-    return step_once<3>(s, q, none, record, rec_cap, nullptr);
+    return step_once<3>(s, q, none, record, rec_cap);
 }
 
 int mixed_eval_contacts(MixedScene* s, double* force, double* moment, cudaStream_t q)
