@@ -1088,13 +1088,12 @@ __global__ void __launch_bounds__(kMeshThreads) k_mesh_move(xd_polygon_mass_info
             out |= !(d2 < disp2);
         }
     }
-    if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) {
-        atomicOr(flag, 1u);
-        __threadfence();   // (before the block counts as done)
+    if (!g.words) {
+        if (__any_sync(0xffffffffu, out) && (threadIdx.x & 31u) == 0) atomicOr(flag, 1u);
+        return;
     }
-    if (!g.words) return;
-    __syncthreads();
-    if (threadIdx.x == 0) step_end(g, todo);
+    const int raised = __syncthreads_or(out);
+    if (threadIdx.x == 0) step_end(g, todo, raised != 0);
 }
 
 unsigned mesh_move_blocks(unsigned ntri) { return div_up(ntri, kMeshThreads); }

@@ -57,15 +57,18 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
 // The end of a graph step of the mixed form (its advance and, beside it, the
 // mesh update): blocks of both that have to finish, and the words they share
 // (nullptr: launched directly, nothing to gate).
-//   words[kStepDone]  blocks done (reset by the last one)
-//   words[kStepFlag]  a re-binning is due (raised by either)
+//   words[kStepDone]  blocks done and, in the next word, those that raised the
+//                     flag (one 8-byte word, reset by the last block: what it
+//                     needs to know comes with its own atomic)
+//   words[kStepFlag]  a re-binning is due (raised ahead of the call, and by
+//                     direct launches)
 //   words[kStepStop]  the flag as the last finished step left it: the steps
 //                     that follow in the graph do nothing until it is cleared
 //   words[kStepTodo]  contact passes left in the call
 // first: the call's first advance (no contact pass precedes it).  tail: the
 // graph ends with this step: rebin is set where a re-binning is due, more (if
 // loop) where passes are left.
-enum { kStepFlag = 0, kStepDone = 1, kStepStop = 34, kStepTodo = 35 };   // (the last two in one 8-byte word)
+enum { kStepFlag = 0, kStepStop = 34, kStepTodo = 35, kStepDone = 36 };   // (stop and todo in one 8-byte word)
 struct StepGate {
     unsigned* words = nullptr;
     unsigned blocks = 0;
@@ -93,16 +96,16 @@ __device__ __forceinline__ void step_skip(const StepGate& g)
 {
     if (g.tail) step_set(g, __ldcg(g.words + kStepStop), __ldcg(g.words + kStepTodo));
 }
-// One block of the step has finished (its thread 0; a flag it raised is visible):
-// the last one closes the step.
-__device__ __forceinline__ void step_end(const StepGate& g, unsigned todo)
+// One block of the step has finished (its thread 0): the last one closes the step.
+__device__ __forceinline__ void step_end(const StepGate& g, unsigned todo, bool raised)
 {
-    if (atomicAdd(g.words + kStepDone, 1u) != g.blocks - 1u) return;
-    __threadfence();
-    const unsigned flag = atomicOr(g.words + kStepFlag, 0u), left = g.first ? todo : todo - 1u;
-    g.words[kStepDone] = 0;
-    g.words[kStepStop] = flag ? 1u : 0u;
-    g.words[kStepTodo] = left;
+    unsigned long long* done = reinterpret_cast<unsigned long long*>(g.words + kStepDone);
+    const unsigned long long old = atomicAdd(done, raised ? 0x100000001ull : 1ull);
+    if ((unsigned)old != g.blocks - 1u) return;
+    const unsigned flag = raised || (old >> 32) != 0ull || (g.first && __ldcg(g.words + kStepFlag)) ? 1u : 0u;
+    const unsigned left = g.first ? todo : todo - 1u;
+    *done = 0;
+    *reinterpret_cast<uint2*>(g.words + kStepStop) = make_uint2(flag, left);
     if (g.tail) step_set(g, flag, left);
 }
 #endif
