@@ -820,6 +820,15 @@ __device__ __forceinline__ void note_displacement(unsigned a, unsigned* counters
 {
     if (a != 0u) atomicMax(counters + CN_DMAX, a);
 }
+// A kernel launched by launch_overlapped may start while the one before it ends:
+// from here on that one has finished and its writes are there; then the next
+// may be brought up.  (Nothing to wait for in a plain launch.)
+__device__ __forceinline__ void wait_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
 // k_mx_advance: one step of the state in place (MODE as above), the contact
 // view, then the skin test on the new position: every particle must stay
 // within half the skin of its position at the last list build (pref); one
@@ -839,6 +848,7 @@ __global__ void __launch_bounds__(256) k_mx_advance(MixParams P, Master M, const
                                                     longlong2* __restrict__ qb, float4* __restrict__ pr,
                                                     unsigned* __restrict__ counters, StepGate g)
 {
+    wait_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned todo = g.words ? step_todo(g.words) : 0u;
     if (g.words && todo == 0) {
@@ -2664,6 +2674,7 @@ template <bool RECORD, int HIST, bool COOP>
 __global__ void __launch_bounds__(kContactMaxThreads) k_mx_contact(MixParams P, ContactArgs C,
                                                                   const unsigned* __restrict__ gate)
 {
+    wait_previous();
     const bool skip = gate && step_todo(gate) == 0;
     // (with history every listed particle: a contact that has ended frees its entry)
     const unsigned total = HIST ? C.counters[CN_HEAVY] : listed_now(P, C.counters), front = C.counters[CN_HTRI];
@@ -3604,6 +3615,25 @@ static ContactArgs contact_args(MixedScene* s, unsigned* rc, unsigned* rp, unsig
     return C;
 }
 
+// A launch that, in a graph, may be brought up while the kernel before it on
+// the stream ends (wait_previous): 1 us of each of a step's two.
+template <typename... K, typename... A>
+static int launch_overlapped(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t q,
+                             bool overlap, const char* what, const A&... args)
+{
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = q;
+    c.attrs = &at;
+    c.numAttrs = overlap ? 1 : 0;
+    return cuda_status(cudaLaunchKernelEx(&c, kernel, K(args)...), what);
+}
+
 // The state advanced in place with the skin test and, for a mesh that moves on
 // the device, the pose and the triangles; the flag is raised once a particle or
 // a vertex has left half the skin.  gate: the step's part in a graph (its
@@ -3646,9 +3676,9 @@ static int advance_step(MixedScene* s, cudaStream_t q, const Phases& ph, StepGat
         if (st != XD_OK) return st;
     }
     ph.begin(0, q);
-    k_mx_advance<MODE><<<blocks(n, 256), 256, 0, q>>>(s->P, s->m[0], s->Fc, s->Mc, s->Fw, s->pref, s->pf, s->qa, s->qb,
-                                                      s->pr, s->counters, g);
-    st = launch_status("mixed advance");
+    // (with a mesh branch the step's kernels join events, not one another)
+    st = launch_overlapped(k_mx_advance<MODE>, blocks(n, 256), 256, 0, q, g.words && !mesh && !g.first, "mixed advance",
+                           s->P, s->m[0], s->Fc, s->Mc, s->Fw, s->pref, s->pf, s->qa, s->qb, s->pr, s->counters, g);
     ph.end(0, q);
     if (st == XD_OK && mesh && g.words) st = after(mb.side, q, mb.join);
     return st;
@@ -3678,19 +3708,20 @@ static int contact_step(MixedScene* s, cudaStream_t q, const Phases& ph, bool re
     }
     const ContactArgs C = contact_args(s, rc, rp, record ? rec_cap : 0u, ht, MODE == 3 ? 0 : 1);
     const unsigned* gate = gated ? s->counters : nullptr;
-#define XD_MX_CONTACT(REC, H) k_mx_contact<REC, H, false><<<grid, ct, 0, q>>>(s->P, C, gate)
+    const bool overlap = gated && !(s->kinematic && s->ntri);
+#define XD_MX_CONTACT(REC, H, COOP, SMEM) \
+    st = launch_overlapped(k_mx_contact<REC, H, COOP>, grid, ct, SMEM, q, overlap, "mixed contact", s->P, C, gate)
     if (record) {
-        if (hist == 2) XD_MX_CONTACT(true, 2);
-        else if (hist == 1) XD_MX_CONTACT(true, 1);
-        else XD_MX_CONTACT(true, 0);
+        if (hist == 2) XD_MX_CONTACT(true, 2, false, 0);
+        else if (hist == 1) XD_MX_CONTACT(true, 1, false, 0);
+        else XD_MX_CONTACT(true, 0, false, 0);
     } else {
-        if (hist == 2) XD_MX_CONTACT(false, 2);
-        else if (hist == 1) XD_MX_CONTACT(false, 1);
-        else if (s->cmode == 1) k_mx_contact<false, 0, true><<<grid, ct, (ct / 32u) * sizeof(WallBuf), q>>>(s->P, C, gate);
-        else XD_MX_CONTACT(false, 0);
+        if (hist == 2) XD_MX_CONTACT(false, 2, false, 0);
+        else if (hist == 1) XD_MX_CONTACT(false, 1, false, 0);
+        else if (s->cmode == 1) XD_MX_CONTACT(false, 0, true, (ct / 32u) * sizeof(WallBuf));
+        else XD_MX_CONTACT(false, 0, false, 0);
     }
 #undef XD_MX_CONTACT
-    st = launch_status("mixed contact");
     ph.end(3, q);
     return st;
 }
