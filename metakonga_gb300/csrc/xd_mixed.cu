@@ -126,7 +126,7 @@ struct MixParams {
                          // in 32 bits (their FP32 values then come from 32-bit conversions)
     float vcut;          // Verlet list: pairs within ri + rj + vcut are listed
     float disp2;         // squared displacement that forces re-binning
-    float gap_bin, inv_gap_bin;   // width of a gap class (vcut / kGapBins)
+    float gap_bin, inv_gap_bin;   // gap class k begins at k^2 gap_bin; class kGapBins would at vcut
     float inv_gx, inv_gxy;   // 1 / gx, 1 / (gx gy) for the key decode
     float dtf, hf, half2dtf;
     float gf[3];
@@ -1390,7 +1390,7 @@ __global__ void __launch_bounds__(256) k_mx_build(MixParams P, const float4* __r
         const bool wall = (P.ntri && __ldg(tcount + i) != 0u) || wm != 0u;
         unsigned c = kUnlisted;
         if (wall) c = 0;
-        else if (nv) c = 1u + (unsigned)min(max((int)(gap * P.inv_gap_bin), 0), (int)kGapBins - 1);
+        else if (nv) c = 1u + min((unsigned)sqrtf(fmaxf(gap, 0.f) * P.inv_gap_bin), kGapBins - 1u);
         lclass[i] = (unsigned char)c;
         if (c != kUnlisted) atomicAdd(&found[c], 1u);
     }
@@ -1449,7 +1449,7 @@ __device__ __forceinline__ unsigned listed_now(const MixParams& P, const unsigne
     unsigned t = c[0] + c[1];
 #pragma unroll
     for (unsigned k = 1; k < kGapBins; ++k)
-        if ((float)k * P.gap_bin <= reach) t += c[k + 1];
+        if ((float)(k * k) * P.gap_bin <= reach) t += c[k + 1];
     return t;
 }
 
@@ -3026,7 +3026,7 @@ static int mixed_setup(MixedScene* s, const xd_scene_desc& d, const double* pos_
     // skin less the FP32 position error, so no unlisted pair can touch.
     P.vcut = (float)skin + P.tol;
     P.disp2 = (float)((0.5 * skin - P.tol) * (0.5 * skin - P.tol));
-    P.gap_bin = P.vcut / (float)kGapBins;
+    P.gap_bin = P.vcut / (float)(kGapBins * kGapBins);
     P.inv_gap_bin = 1.0f / P.gap_bin;
     P.wall_tol = (float)(1e-5 + extent * 0x1p-20);
     const xd_contact_property& cp = d.cp_pp;
