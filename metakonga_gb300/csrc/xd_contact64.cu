@@ -31,17 +31,19 @@ namespace xd {
 
 // ------------------------------------------------------- particle-particle
 
-// Results of a warp's contacts in its ScanBuf (9 values): T = Fn + Ft (the
+// Results of contacts in the block's ScanBuf (9 values): T = Fn + Ft (the
 // normal force alone when the slip is zero), Ft, M.
 enum { kContact = 1u, kSlip = 2u };
 
-__device__ __forceinline__ void put3(double (*res)[32], int a, unsigned lane, d3 v)
+template <unsigned L>
+__device__ __forceinline__ void put3(double (*res)[L], int a, unsigned lane, d3 v)
 {
     res[a][lane] = v.x;
     res[a + 1][lane] = v.y;
     res[a + 2][lane] = v.z;
 }
-__device__ __forceinline__ d3 get3(const double (*res)[32], int a, unsigned lane)
+template <unsigned L>
+__device__ __forceinline__ d3 get3(const double (*res)[L], int a, unsigned lane)
 {
     return mk(res[a][lane], res[a + 1][lane], res[a + 2][lane]);
 }
@@ -81,7 +83,7 @@ __device__ __forceinline__ bool spheres_near(const Near4& a, const Near4& b)
 // with the law evaluated where a thread found a contact; 8,000 spheres 50 us
 // (438), 17,159 on a mesh's cells of 2.5 cm 212 us (2,527).
 template <int LP>
-__global__ void __launch_bounds__(64, 8) k_p2p(Params P, const double* __restrict__ pos,
+__global__ void __launch_bounds__(32 * kPoolWarps<LP>, 16 / kPoolWarps<LP>) k_p2p(Params P, const double* __restrict__ pos,
                                                const double* __restrict__ vel, const double* __restrict__ omega,
                                                double* __restrict__ force, double* __restrict__ moment,
                                                const double* __restrict__ mass, const unsigned* __restrict__ sorted,
@@ -89,16 +91,13 @@ __global__ void __launch_bounds__(64, 8) k_p2p(Params P, const double* __restric
                                                const xd_contact_property* __restrict__ cp, unsigned np)
 {
     using Buf = ScanBuf<LP, double, 9>;
-    __shared__ Buf bufs[2];
+    __shared__ Buf B;
     __shared__ PairConst pc;
-    if (threadIdx.x == 0) pc = load_pair_const(cp);
-    __syncthreads();
-    Buf& B = bufs[threadIdx.x / 32u];
-    constexpr unsigned NP = 32 / LP;
+    if (threadIdx.x == 0) pc = load_pair_const(cp);   // (scan_contacts' barriers before the first use)
+    constexpr unsigned NP = 32 / LP, NB = NP * kPoolWarps<LP>;
     const unsigned lane = threadIdx.x & 31u;
-    const unsigned groups = (np + NP - 1u) / NP;
-    for (unsigned g = blockIdx.x * 2u + threadIdx.x / 32u; g < groups; g += gridDim.x * 2u) {
-        const unsigned id0 = g * NP, id = id0 + lane / LP;
+    for (unsigned b0 = blockIdx.x * NB; b0 < np; b0 += gridDim.x * NB) {
+        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
         const bool valid = id < np;
         d4 ip = d4{ 0, 0, 0, 0 };
         int3 gp = make_int3(0, 0, 0);
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(64, 8) k_p2p(Params P, const double* __restric
             B, runs, sorted,
             [&](unsigned k, unsigned) { return k != id && k < np && spheres_near(mine, near_of(ld4(pos, k))); },
             [&](unsigned o, unsigned k, unsigned l) {
-                const unsigned i = id0 + o;
+                const unsigned i = b0 + o;
                 const d4 a = ld4(pos, i), b = ld4(pos, k);
                 const d3 rp = mk(b.x - a.x, b.y - a.y, b.z - a.z);
                 const double dist = length(rp);
@@ -498,7 +497,7 @@ __device__ __forceinline__ bool triangle_near(const Near4& p, const xd_polygon_i
 enum { kMoment = 4u, kBodyShift = 3u };
 
 template <int NB, int LP>
-__global__ void __launch_bounds__(64) k_polygon(Params P, const xd_polygon_info* __restrict__ dpi,
+__global__ void __launch_bounds__(32 * kPoolWarps<LP>) k_polygon(Params P, const xd_polygon_info* __restrict__ dpi,
                                                 xd_polygon_mass_info* __restrict__ dpmi,
                                                 const double* __restrict__ pos, const double* __restrict__ vel,
                                                 const double* __restrict__ omega, double* __restrict__ force,
@@ -510,10 +509,9 @@ __global__ void __launch_bounds__(64) k_polygon(Params P, const xd_polygon_info*
                                                 double* __restrict__ partials)
 {
     using Buf = ScanBuf<LP, double, 12>;
-    __shared__ Buf bufs[2];
-    Buf& B = bufs[threadIdx.x / 32u];
+    __shared__ Buf B;
     constexpr int NBR = NB > 0 ? NB : 1;
-    constexpr unsigned NP = 32 / LP;
+    constexpr unsigned NP = 32 / LP, NW = kPoolWarps<LP>;
     double react[NBR][6];
 #pragma unroll
     for (int b = 0; b < NBR; ++b)
@@ -521,10 +519,9 @@ __global__ void __launch_bounds__(64) k_polygon(Params P, const xd_polygon_info*
         for (int q = 0; q < 6; ++q) react[b][q] = 0.0;
     bool reacted = false;
     const unsigned cnp = P.np, lane = threadIdx.x & 31u;
-    const unsigned warp = blockIdx.x * 2u + threadIdx.x / 32u;
-    const unsigned groups = (cnp + NP - 1u) / NP;
-    for (unsigned g = warp; g < groups; g += gridDim.x * 2u) {
-        const unsigned id0 = g * NP, id = id0 + lane / LP;
+    const unsigned warp = blockIdx.x * NW + threadIdx.x / 32u;
+    for (unsigned b0 = blockIdx.x * NP * NW; b0 < cnp; b0 += gridDim.x * NP * NW) {
+        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
         const bool valid = id < cnp;
         d4 ip = d4{ 0, 0, 0, 0 };
         int3 gp = make_int3(0, 0, 0);
@@ -543,7 +540,7 @@ __global__ void __launch_bounds__(64) k_polygon(Params P, const xd_polygon_info*
             // values: Fn + Ft, Ft and the reaction's moment, or without slip Fn, -- and the contact point
             // from the body's origin; then M, where it is not zero (a normal that is not a number)
             [&](unsigned o, unsigned k, unsigned l) {
-                const unsigned i = id0 + o;
+                const unsigned i = b0 + o;
                 const xd_polygon_info* tri = dpi + (k - cnp);
                 const d4 a = ld4(pos, i);
                 const d3 ipos = xyz(a);
@@ -918,8 +915,9 @@ int launch_p2p(const Params& P, const double* pos, const double* vel, const doub
         return launch_status("calculate_p2p");
     }
     const int lp = scan_lanes(np);
-    const unsigned nb = scan_blocks(np, lp);
-#define XD_P2P(LP) k_p2p<LP><<<nb, 64, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart, cend, cp, np)
+#define XD_P2P(LP)                                                                                              \
+    k_p2p<LP><<<scan_blocks<LP>(np), 32 * kPoolWarps<LP>, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, \
+                                                                  cstart, cend, cp, np)
     if (lp == 1) XD_P2P(1);
     else if (lp == 4) XD_P2P(4);
     else XD_P2P(8);
@@ -970,11 +968,15 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
     if (np == 0) return XD_OK;
     const unsigned nbr = nbr_for(nbodies);
     const int lp = scan_lanes(np);
-    const unsigned nb = ht ? div_up(np, 128) : scan_blocks(np, lp);
+    unsigned nb = div_up(np, 128), parts = nb;
     double* part = static_cast<double*>(scratch);
-#define XD_POLY_LP(NBV, LP)                                                                                   \
-    k_polygon<NBV, LP><<<nb, 64, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, sidx, cstart, cend, \
-                                         cp, part)
+#define XD_POLY_LP(NBV, LP)                                                                                       \
+    do {                                                                                                          \
+        nb = scan_blocks<LP>(np);                                                                                 \
+        parts = nb * kPoolWarps<LP>;                                                                              \
+        k_polygon<NBV, LP><<<nb, 32 * kPoolWarps<LP>, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, \
+                                                              sidx, cstart, cend, cp, part);                      \
+    } while (0)
 #define XD_POLY(NBV)                                                                                          \
     do {                                                                                                      \
         if (ht)                                                                                               \
@@ -995,7 +997,7 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
 #undef XD_POLY_LP
     int st = launch_status("particle_polygon_collision");
     if (st != XD_OK || nbr == 0) return st;
-    k_polygon_reaction_final<<<6 * nbodies, 128, 0, s>>>(part, ht ? nb : 2u * nb, nbr, dpmi);
+    k_polygon_reaction_final<<<6 * nbodies, 128, 0, s>>>(part, parts, nbr, dpmi);
     return launch_status("particle_polygon_collision (reaction)");
 }
 

@@ -49,19 +49,24 @@ __device__ __forceinline__ int3 grid_pos_fast(const Params& P, double x, double 
     return make_int3(cell_of(P, x, 0), cell_of(P, y, 1), cell_of(P, z, 2));
 }
 
-// One warp's buffer for P particles of 32 / P lanes each: the runs of sorted
-// slots that their cells cover, the partners found (k-th of particle o at
-// [k * P + o]), the order in which they are taken, and NR values of result
-// per lane.
+// A block's warps in the search, whose contacts it pools, by lanes per particle.
+template <int LP>
+constexpr int kPoolWarps = LP == 8 ? 8 : (LP == 4 ? 4 : 2);
+
+// A block's buffer, NP = 32 / LP particles a warp: the runs of sorted slots
+// that their cells cover, the partners found (k-th of a warp's particle o at
+// [k * NP + o] of the warp's kEach), where each comes in the pooled order and
+// that order, and NR values of result per lane.
 template <int LP, typename Real, int NR>
 struct ScanBuf {
-    static constexpr int kParticles = 32 / LP;
-    static constexpr int kSlots = LP == 1 ? 16 : 24;
-    uint2 run[27][kParticles];
-    Real res[NR][32];
-    unsigned cand[kSlots * kParticles];
-    unsigned short slot[kSlots * kParticles];
-    unsigned short pos[kSlots * kParticles];
+    static constexpr unsigned kWarps = kPoolWarps<LP>, kParticles = 32 / LP, kSlots = LP == 1 ? 16 : 24;
+    static constexpr unsigned kEach = kSlots * kParticles, kLanes = 32 * kWarps;
+    uint2 run[kWarps][27][kParticles];
+    Real res[NR][kLanes];
+    unsigned cand[kWarps * kEach];
+    unsigned short slot[kWarps * kEach];
+    unsigned short pos[kWarps * kEach];
+    unsigned total[kWarps];
 };
 
 // The cells of lane group o's particle (cell gp, when valid) into run[][o]:
@@ -73,6 +78,7 @@ __device__ __forceinline__ unsigned stage_runs(Buf& B, bool valid, int3 gp, cons
                                                const unsigned* __restrict__ cend, Hash hash)
 {
     const unsigned lane = threadIdx.x & 31u, o = lane / LP, sub = lane % LP;
+    auto& run = B.run[threadIdx.x / 32u];
     constexpr int kEach = (27 + LP - 1) / LP;
 #pragma unroll
     for (int q = 0; q < kEach; ++q) {
@@ -80,7 +86,7 @@ __device__ __forceinline__ unsigned stage_runs(Buf& B, bool valid, int3 gp, cons
         if (valid && c < 27) {
             const unsigned h = hash(gp.x + c % 3 - 1, gp.y + (c / 3) % 3 - 1, gp.z + c / 9 - 1);
             const unsigned st = __ldg(cstart + h);
-            B.run[c][o] = make_uint2(st, st == 0xffffffffu ? st : __ldg(cend + h));
+            run[c][o] = make_uint2(st, st == 0xffffffffu ? st : __ldg(cend + h));
         }
     }
     __syncwarp();
@@ -88,43 +94,50 @@ __device__ __forceinline__ unsigned stage_runs(Buf& B, bool valid, int3 gp, cons
     if (valid && sub == 0) {
         uint2 cur = make_uint2(0u, 0u);
         for (int c = 0; c < 27; ++c) {
-            const uint2 b = B.run[c][o];
+            const uint2 b = run[c][o];
             if (b.x >= b.y) continue;
             if (b.x == cur.y && cur.x != cur.y) {
                 cur.y = b.y;
             } else {
-                if (cur.x != cur.y) B.run[n++][o] = cur;
+                if (cur.x != cur.y) run[n++][o] = cur;
                 cur = b;
             }
         }
-        if (cur.x != cur.y) B.run[n++][o] = cur;
+        if (cur.x != cur.y) run[n++][o] = cur;
     }
     n = __shfl_sync(kFullWarp, n, (int)(o * LP));
     __syncwarp();
     return n;
 }
 
-// The warp's contacts.  near(k, o): whether entry k of the sorted list may
-// touch particle o (never false for one that does).  eval(o, k, lane): the
-// law of that pair, its result into B.res[][lane]; returns a code, 0 for no
-// contact.  add(code, lane): the result in B.res[][lane] to the sums of the
-// calling lane's particle; lane o adds particle o's, in search order.
+// The block's contacts (every thread of it calls).  near(k, o): whether entry
+// k of the sorted list may touch particle o of the warp (never false for one
+// that does).  eval(o, k, l): the law of that pair, o counted through the
+// block's warps, its result into B.res[][l]; returns a code, 0 for no contact.
+// add(code, l): the result in B.res[][l] to the sums of the calling lane's
+// particle; lane o of a warp adds its particle o's, in search order.
 //
 // Each round collects partners until a particle's slots could overflow, then
-// takes them level by level (every particle's first, then every particle's
-// second, ...), 32 at a time: a group of 32 then holds one or two of most
-// particles and the adding runs on most lanes.
+// takes a warp's level by level (every particle's first, then every
+// particle's second, ...), 32 a warp at a time: a group of 32 then holds one
+// or two of most particles and the adding runs on most lanes.  The groups run
+// on across the block's warps: the FP64 pipe takes as long for a group of
+// three contacts as for one of 32, and a warp's own last group was half empty
+// (us a call: P2P_FIGURES).
 template <int LP, typename Buf, typename Near, typename Eval, typename Add>
 __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsigned* __restrict__ sorted, Near near,
                                               Eval eval, Add add)
 {
-    constexpr unsigned P = 32 / LP, U = LP == 1 ? 4u : (LP == 4 ? 2u : 1u), S = Buf::kSlots;
-    const unsigned lane = threadIdx.x & 31u, o = lane / LP, sub = lane % LP;
+    constexpr unsigned P = 32 / LP, U = LP == 1 ? 4u : (LP == 4 ? 2u : 1u), S = Buf::kSlots, E = Buf::kEach;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x / 32u, o = lane / LP, sub = lane % LP;
     const unsigned group = LP == 32 ? kFullWarp : ((1u << LP) - 1u) << (o * LP);
+    unsigned* const cand = B.cand + warp * E;
+    unsigned short* const pos = B.pos + warp * E;
+    const auto& run = B.run[warp];
     unsigned r = 0, j = 0, e = 0;
     bool more = nruns != 0u;
     if (more) {
-        const uint2 b = B.run[0][o];
+        const uint2 b = run[0][o];
         j = b.x;
         e = b.y;
     }
@@ -146,10 +159,10 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
 #pragma unroll
             for (unsigned u = 0; u < U; ++u) {
                 if (LP == 1) {
-                    if (in[u]) B.cand[cnt++ * P + o] = k[u];
+                    if (in[u]) cand[cnt++ * P + o] = k[u];
                 } else {
                     const unsigned b = __ballot_sync(kFullWarp, in[u]) & group;
-                    if (in[u]) B.cand[(cnt + __popc(b & ((1u << lane) - 1u))) * P + o] = k[u];
+                    if (in[u]) cand[(cnt + __popc(b & ((1u << lane) - 1u))) * P + o] = k[u];
                     cnt += __popc(b);
                 }
             }
@@ -158,7 +171,7 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
                 if (j >= e) {
                     more = ++r < nruns;
                     if (more) {
-                        const uint2 b = B.run[r][o];
+                        const uint2 b = run[r][o];
                         j = b.x;
                         e = b.y;
                     }
@@ -168,34 +181,42 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
         // lane o < P owns particle o
         const unsigned mine = LP == 1 ? cnt : __shfl_sync(kFullWarp, cnt, (int)((lane * LP) & 31u));
         const unsigned own = lane < P ? mine : 0u;
-        const unsigned levels = __reduce_max_sync(kFullWarp, own);
-        unsigned total = 0;
+        const unsigned levels = __reduce_max_sync(kFullWarp, own), found = __reduce_add_sync(kFullWarp, own);
+        if (lane == 0) B.total[warp] = found;
+        __syncthreads();
+        unsigned at = 0, total = 0;
+#pragma unroll
+        for (unsigned w = 0; w < Buf::kWarps; ++w) {
+            const unsigned t = B.total[w];
+            at += w < warp ? t : 0u;
+            total += t;
+        }
         for (unsigned l = 0; l < levels; ++l) {
             const unsigned b = __ballot_sync(kFullWarp, own > l);
             if (own > l) {
-                const unsigned p = total + __popc(b & ((1u << lane) - 1u));
-                B.slot[p] = (unsigned short)(l * P + lane);
-                B.pos[l * P + lane] = (unsigned short)p;
+                const unsigned p = at + __popc(b & ((1u << lane) - 1u));
+                B.slot[p] = (unsigned short)(warp * E + l * P + lane);
+                pos[l * P + lane] = (unsigned short)p;
             }
-            total += __popc(b);
+            at += __popc(b);
         }
-        __syncwarp();
+        __syncthreads();
         unsigned done = 0;
-        for (unsigned base = 0; base < total; base += 32u) {
-            if (base + lane < total) {
-                const unsigned s = B.slot[base + lane];
-                B.cand[s] = eval(s % P, B.cand[s], lane);
+        for (unsigned base = 0; base < total; base += Buf::kLanes) {
+            if (base + threadIdx.x < total) {
+                const unsigned s = B.slot[base + threadIdx.x];
+                B.cand[s] = eval(s / E * P + s % P, B.cand[s], threadIdx.x);
             }
-            __syncwarp();
+            __syncthreads();
             for (; done < own; ++done) {
-                const unsigned p = B.pos[done * P + lane];
-                if (p >= base + 32u) break;
-                const unsigned code = B.cand[done * P + lane];
+                const unsigned p = pos[done * P + lane];
+                if (p >= base + Buf::kLanes) break;
+                const unsigned code = cand[done * P + lane];
                 if (code) add(code, p - base);
             }
-            __syncwarp();
+            if (base + Buf::kLanes < total) __syncthreads();
         }
-        if (!__any_sync(kFullWarp, more)) return;
+        if (!__syncthreads_or(more)) return;
     }
 }
 
@@ -209,14 +230,14 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
 // which the upper line lies above where a bed alone would put it (30,000).
 inline int scan_lanes(unsigned np) { return np >= 48000u ? 1 : (np >= 10000u ? 4 : 8); }
 
-// Blocks of two warps for it: at most one wave (eight blocks an SM), whose
-// warps then take several groups of particles and form the contact
-// property's constants once.
+// Blocks for it: at most one wave (16 warps an SM), whose blocks then take
+// several groups of particles and form the contact property's constants once.
 constexpr unsigned kScanWarps = 152u * 8u * 2u;
-inline unsigned scan_blocks(unsigned np, int lp)
+template <int LP>
+inline unsigned scan_blocks(unsigned np)
 {
-    const unsigned groups = div_up(np, 32u / (unsigned)lp), blocks = div_up(groups, 2u);
-    return blocks < kScanWarps / 2u ? blocks : kScanWarps / 2u;
+    const unsigned blocks = div_up(np, 32u / LP * kPoolWarps<LP>), most = kScanWarps / kPoolWarps<LP>;
+    return blocks < most ? blocks : most;
 }
 
 }  // namespace xd

@@ -223,19 +223,21 @@ __global__ void __launch_bounds__(256) k_hash_f(ParamsF P, unsigned* __restrict_
 // root: 100,003 spheres in a bed took 242 us with it evaluated where a thread
 // found a contact, and the partners' velocities read for every candidate;
 // they take 81 us here.
-__device__ __forceinline__ void put3f(float (*res)[32], int a, unsigned lane, f3 v)
+template <unsigned L>
+__device__ __forceinline__ void put3f(float (*res)[L], int a, unsigned lane, f3 v)
 {
     res[a][lane] = v.x;
     res[a + 1][lane] = v.y;
     res[a + 2][lane] = v.z;
 }
-__device__ __forceinline__ f3 get3f(const float (*res)[32], int a, unsigned lane)
+template <unsigned L>
+__device__ __forceinline__ f3 get3f(const float (*res)[L], int a, unsigned lane)
 {
     return mkf(res[a][lane], res[a + 1][lane], res[a + 2][lane]);
 }
 
 template <int LP>
-__global__ void __launch_bounds__(64) k_p2p_f(ParamsF P, const float4* __restrict__ pos,
+__global__ void __launch_bounds__(32 * kPoolWarps<LP>) k_p2p_f(ParamsF P, const float4* __restrict__ pos,
                                               const float* __restrict__ vel, const float* __restrict__ omega,
                                               float* __restrict__ force, float* __restrict__ moment,
                                               const float* __restrict__ mass, const unsigned* __restrict__ sorted,
@@ -244,17 +246,14 @@ __global__ void __launch_bounds__(64) k_p2p_f(ParamsF P, const float4* __restric
                                               const xd_contact_property_f* __restrict__ cpp, unsigned np)
 {
     using Buf = ScanBuf<LP, float, 9>;
-    __shared__ Buf bufs[2];
+    __shared__ Buf B;
     __shared__ PairConstF pc;
-    if (threadIdx.x == 0) pc = pair_const_f(*cpp);
-    __syncthreads();
-    Buf& B = bufs[threadIdx.x / 32u];
-    constexpr unsigned NP = 32 / LP;
+    if (threadIdx.x == 0) pc = pair_const_f(*cpp);   // (scan_contacts' barriers before the first use)
+    constexpr unsigned NP = 32 / LP, NB = NP * kPoolWarps<LP>;
     const xd_contact_property_f cp = *cpp;
     const unsigned lane = threadIdx.x & 31u;
-    const unsigned groups = (np + NP - 1u) / NP;
-    for (unsigned g = blockIdx.x * 2u + threadIdx.x / 32u; g < groups; g += gridDim.x * 2u) {
-        const unsigned id0 = g * NP, id = id0 + lane / LP;
+    for (unsigned b0 = blockIdx.x * NB; b0 < np; b0 += gridDim.x * NB) {
+        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
         const bool valid = id < np;
         float4 ip = make_float4(0.f, 0.f, 0.f, 0.f);
         int3 gp = make_int3(0, 0, 0);
@@ -275,7 +274,7 @@ __global__ void __launch_bounds__(64) k_p2p_f(ParamsF P, const float4* __restric
                 return !(d2 > lim * lim && d2 > 1e-30f);
             },
             [&](unsigned o, unsigned k, unsigned l) {
-                const unsigned i = id0 + o;
+                const unsigned i = b0 + o;
                 const float4 a = __ldg(pos + i), b = __ldg(pos + k);
                 const f3 rp = mkf(b.x - a.x, b.y - a.y, b.z - a.z);
                 const float dist = lenf(rp);
@@ -715,10 +714,9 @@ int xd_calculate_p2p_f(int tcm, const float* pos, const float* vel, const float*
                  "calculate_p2p_f: null pointer");
     XD_REQUIRE_F(aligned16(pos), "calculate_p2p_f: pos must be 16-byte aligned");
     const int lp = scan_lanes(np);
-    const unsigned nb = scan_blocks(np, lp);
-#define XD_P2P_F(LP)                                                                                            \
-    k_p2p_f<LP><<<nb, 64, 0, S(s)>>>(PF, reinterpret_cast<const float4*>(pos), vel, omega, force, moment, mass, \
-                                     sorted_index, cstart, cend, cp, np)
+#define XD_P2P_F(LP)                                                                                       \
+    k_p2p_f<LP><<<scan_blocks<LP>(np), 32 * kPoolWarps<LP>, 0, S(s)>>>(                                    \
+        PF, reinterpret_cast<const float4*>(pos), vel, omega, force, moment, mass, sorted_index, cstart, cend, cp, np)
     if (lp == 1) XD_P2P_F(1);
     else if (lp == 4) XD_P2P_F(4);
     else XD_P2P_F(8);
