@@ -82,19 +82,19 @@ __device__ __forceinline__ bool spheres_near(const Near4& a, const Near4& b)
 // the results are the same bits.  A bed of 120,989 spheres: 0.4 ms, 3.5 ms
 // with the law evaluated where a thread found a contact; 8,000 spheres 50 us
 // (438), 17,159 on a mesh's cells of 2.5 cm 212 us (2,527).
-template <int LP>
-__global__ void __launch_bounds__(32 * kPoolWarps<LP>, 16 / kPoolWarps<LP>) k_p2p(Params P, const double* __restrict__ pos,
+template <int LP, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW) k_p2p(Params P, const double* __restrict__ pos,
                                                const double* __restrict__ vel, const double* __restrict__ omega,
                                                double* __restrict__ force, double* __restrict__ moment,
                                                const double* __restrict__ mass, const unsigned* __restrict__ sorted,
                                                const unsigned* __restrict__ cstart, const unsigned* __restrict__ cend,
                                                const xd_contact_property* __restrict__ cp, unsigned np)
 {
-    using Buf = ScanBuf<LP, double, 9>;
+    using Buf = ScanBuf<LP, NW, double, 9>;
     __shared__ Buf B;
     __shared__ PairConst pc;
     if (threadIdx.x == 0) pc = load_pair_const(cp);   // (scan_contacts' barriers before the first use)
-    constexpr unsigned NP = 32 / LP, NB = NP * kPoolWarps<LP>;
+    constexpr unsigned NP = 32 / LP, NB = NP * NW;
     const unsigned lane = threadIdx.x & 31u;
     for (unsigned b0 = blockIdx.x * NB; b0 < np; b0 += gridDim.x * NB) {
         const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
@@ -496,8 +496,8 @@ __device__ __forceinline__ bool triangle_near(const Near4& p, const xd_polygon_i
 // does not say how many bodies there are).
 enum { kMoment = 4u, kBodyShift = 3u };
 
-template <int NB, int LP>
-__global__ void __launch_bounds__(32 * kPoolWarps<LP>) k_polygon(Params P, const xd_polygon_info* __restrict__ dpi,
+template <int NB, int LP, int NW>
+__global__ void __launch_bounds__(32 * NW) k_polygon(Params P, const xd_polygon_info* __restrict__ dpi,
                                                 xd_polygon_mass_info* __restrict__ dpmi,
                                                 const double* __restrict__ pos, const double* __restrict__ vel,
                                                 const double* __restrict__ omega, double* __restrict__ force,
@@ -508,10 +508,10 @@ __global__ void __launch_bounds__(32 * kPoolWarps<LP>) k_polygon(Params P, const
                                                 const xd_contact_property* __restrict__ cp,
                                                 double* __restrict__ partials)
 {
-    using Buf = ScanBuf<LP, double, 12>;
+    using Buf = ScanBuf<LP, NW, double, 12>;
     __shared__ Buf B;
     constexpr int NBR = NB > 0 ? NB : 1;
-    constexpr unsigned NP = 32 / LP, NW = kPoolWarps<LP>;
+    constexpr unsigned NP = 32 / LP;
     double react[NBR][6];
 #pragma unroll
     for (int b = 0; b < NBR; ++b)
@@ -914,14 +914,11 @@ int launch_p2p(const Params& P, const double* pos, const double* vel, const doub
                                                    cp, np, *ht);
         return launch_status("calculate_p2p");
     }
-    const int lp = scan_lanes(np);
-#define XD_P2P(LP)                                                                                              \
-    k_p2p<LP><<<scan_blocks<LP>(np), 32 * kPoolWarps<LP>, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, \
-                                                                  cstart, cend, cp, np)
-    if (lp == 1) XD_P2P(1);
-    else if (lp == 4) XD_P2P(4);
-    else XD_P2P(8);
-#undef XD_P2P
+    scan_shape(np, [&](auto lp, auto nw) {
+        constexpr int LP = decltype(lp)::value, NW = decltype(nw)::value;
+        k_p2p<LP, NW><<<scan_blocks(np, LP, NW), 32 * NW, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart,
+                                                                  cend, cp, np);
+    });
     return launch_status("calculate_p2p");
 }
 
@@ -967,24 +964,23 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
     unsigned np = P.np;
     if (np == 0) return XD_OK;
     const unsigned nbr = nbr_for(nbodies);
-    const int lp = scan_lanes(np);
-    unsigned nb = div_up(np, 128), parts = nb;
+    const unsigned nb = div_up(np, 128);
+    unsigned parts = nb;   // of the reaction
     double* part = static_cast<double*>(scratch);
-#define XD_POLY_LP(NBV, LP)                                                                                       \
+#define XD_POLY(NBV)                                                                                              \
     do {                                                                                                          \
-        nb = scan_blocks<LP>(np);                                                                                 \
-        parts = nb * kPoolWarps<LP>;                                                                              \
-        k_polygon<NBV, LP><<<nb, 32 * kPoolWarps<LP>, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, \
-                                                              sidx, cstart, cend, cp, part);                      \
-    } while (0)
-#define XD_POLY(NBV)                                                                                          \
-    do {                                                                                                      \
-        if (ht)                                                                                               \
-            k_polygon_hist<NBV><<<nb, 128, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, sidx,   \
-                                                   cstart, cend, cp, part, *ht);                              \
-        else if (lp == 1) XD_POLY_LP(NBV, 1);                                                                 \
-        else if (lp == 4) XD_POLY_LP(NBV, 4);                                                                 \
-        else XD_POLY_LP(NBV, 8);                                                                              \
+        if (ht) {                                                                                                 \
+            k_polygon_hist<NBV><<<nb, 128, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, mass, sidx,      \
+                                                   cstart, cend, cp, part, *ht);                                  \
+        } else {                                                                                                  \
+            scan_shape(np, [&](auto lp, auto nw) {                                                                \
+                constexpr int LP = decltype(lp)::value, NW = decltype(nw)::value;                                 \
+                const unsigned grid = scan_blocks(np, LP, NW);                                                    \
+                parts = grid * NW;                                                                                \
+                k_polygon<NBV, LP, NW><<<grid, 32 * NW, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment,     \
+                                                                mass, sidx, cstart, cend, cp, part);              \
+            });                                                                                                   \
+        }                                                                                                         \
     } while (0)
     switch (nbr) {
     case 0: XD_POLY(0); break;
@@ -994,7 +990,6 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
     default: XD_POLY(8); break;
     }
 #undef XD_POLY
-#undef XD_POLY_LP
     int st = launch_status("particle_polygon_collision");
     if (st != XD_OK || nbr == 0) return st;
     k_polygon_reaction_final<<<6 * nbodies, 128, 0, s>>>(part, parts, nbr, dpmi);

@@ -49,17 +49,13 @@ __device__ __forceinline__ int3 grid_pos_fast(const Params& P, double x, double 
     return make_int3(cell_of(P, x, 0), cell_of(P, y, 1), cell_of(P, z, 2));
 }
 
-// A block's warps in the search, whose contacts it pools, by lanes per particle.
-template <int LP>
-constexpr int kPoolWarps = LP == 8 ? 8 : (LP == 4 ? 4 : 2);
-
-// A block's buffer, NP = 32 / LP particles a warp: the runs of sorted slots
+// The buffer of a block of NW warps, NP = 32 / LP particles a warp: the runs of sorted slots
 // that their cells cover, the partners found (k-th of a warp's particle o at
 // [k * NP + o] of the warp's kEach), where each comes in the pooled order and
 // that order, and NR values of result per lane.
-template <int LP, typename Real, int NR>
+template <int LP, int NW, typename Real, int NR>
 struct ScanBuf {
-    static constexpr unsigned kWarps = kPoolWarps<LP>, kParticles = 32 / LP, kSlots = LP == 1 ? 16 : 24;
+    static constexpr unsigned kWarps = NW, kParticles = 32 / LP, kSlots = LP == 1 ? 16 : 24;
     static constexpr unsigned kEach = kSlots * kParticles, kLanes = 32 * kWarps;
     uint2 run[kWarps][27][kParticles];
     Real res[NR][kLanes];
@@ -224,19 +220,38 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
 // fills its lanes best (131 contacts of a bed in five groups); with few
 // particles the chip is not full and more lanes shorten the chain of loads
 // and contacts that one warp goes through.  FP64 pairs, us with 1 / 4 / 8
-// lanes: a bed of 2,000 spheres 77 / 35 / 26, 8,000 77 / 54 / 54, 17,000
-// 97 / 85 / 94, 60,000 197 / 238 / 285, 120,989 349 / 461 / 556; on a mesh's
-// wide cells 17,159 591 / 216 / 251 and 60,000 2,018 / 1,809 / 2,253, for
-// which the upper line lies above where a bed alone would put it (30,000).
-inline int scan_lanes(unsigned np) { return np >= 48000u ? 1 : (np >= 10000u ? 4 : 8); }
+// lanes: a bed of 2,000 spheres 70 / 37 / 25, 8,000 79 / 46 / 46, 17,000
+// 99 / 73 / 85, 40,000 144 / 139 / 163, 60,000 184 / 210 / 226, 120,989
+// 339 / 400 / 427; on a mesh's wide cells 17,159 581 / 218 / 255 and 60,000
+// 2,025 / 1,858 / 2,303.
+//
+// Warps whose contacts a block pools: for the FP64 law 2, 4 or 8 by lanes per
+// particle, about 32 to 64 particles a block, but with fewer than 152 blocks of
+// 8 warps half as many (2,000 spheres: 8 warps 31 us, 4 25, 2 27; 8,000: 46, 48
+// and 54).  The FP32 law gains from full groups only where there are many: 2
+// warps (8,000 spheres: 8 warps 20.8 us, 2 18.6), and 1 lane a particle from
+// 28,000 on (30,000: 35.3 us, with 4 lanes 37.3; 100,003: 70 and 94).
+//
+// f(lanes, warps), each as a type's value, for np particles.
+template <int V>
+struct IntC {
+    static constexpr int value = V;
+};
+template <bool FP64 = true, typename F>
+inline void scan_shape(unsigned np, F f)
+{
+    if (np >= (FP64 ? 48000u : 28000u)) f(IntC<1>(), IntC<2>());
+    else if (np >= 10000u) f(IntC<4>(), IntC<FP64 ? 4 : 2>());
+    else if (FP64 && np >= 152u * 32u) f(IntC<8>(), IntC<8>());
+    else f(IntC<8>(), IntC<FP64 ? 4 : 2>());
+}
 
 // Blocks for it: at most one wave (16 warps an SM), whose blocks then take
 // several groups of particles and form the contact property's constants once.
 constexpr unsigned kScanWarps = 152u * 8u * 2u;
-template <int LP>
-inline unsigned scan_blocks(unsigned np)
+inline unsigned scan_blocks(unsigned np, unsigned lp, unsigned nw)
 {
-    const unsigned blocks = div_up(np, 32u / LP * kPoolWarps<LP>), most = kScanWarps / kPoolWarps<LP>;
+    const unsigned blocks = div_up(np, 32u / lp * nw), most = kScanWarps / nw;
     return blocks < most ? blocks : most;
 }
 

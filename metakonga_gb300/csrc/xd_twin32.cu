@@ -236,8 +236,8 @@ __device__ __forceinline__ f3 get3f(const float (*res)[L], int a, unsigned lane)
     return mkf(res[a][lane], res[a + 1][lane], res[a + 2][lane]);
 }
 
-template <int LP>
-__global__ void __launch_bounds__(32 * kPoolWarps<LP>) k_p2p_f(ParamsF P, const float4* __restrict__ pos,
+template <int LP, int NW>
+__global__ void __launch_bounds__(32 * NW) k_p2p_f(ParamsF P, const float4* __restrict__ pos,
                                               const float* __restrict__ vel, const float* __restrict__ omega,
                                               float* __restrict__ force, float* __restrict__ moment,
                                               const float* __restrict__ mass, const unsigned* __restrict__ sorted,
@@ -245,11 +245,11 @@ __global__ void __launch_bounds__(32 * kPoolWarps<LP>) k_p2p_f(ParamsF P, const 
                                               const unsigned* __restrict__ cend,
                                               const xd_contact_property_f* __restrict__ cpp, unsigned np)
 {
-    using Buf = ScanBuf<LP, float, 9>;
+    using Buf = ScanBuf<LP, NW, float, 9>;
     __shared__ Buf B;
     __shared__ PairConstF pc;
     if (threadIdx.x == 0) pc = pair_const_f(*cpp);   // (scan_contacts' barriers before the first use)
-    constexpr unsigned NP = 32 / LP, NB = NP * kPoolWarps<LP>;
+    constexpr unsigned NP = 32 / LP, NB = NP * NW;
     const xd_contact_property_f cp = *cpp;
     const unsigned lane = threadIdx.x & 31u;
     for (unsigned b0 = blockIdx.x * NB; b0 < np; b0 += gridDim.x * NB) {
@@ -713,14 +713,12 @@ int xd_calculate_p2p_f(int tcm, const float* pos, const float* vel, const float*
     XD_REQUIRE_F(pos && vel && omega && force && moment && mass && sorted_index && cstart && cend && cp,
                  "calculate_p2p_f: null pointer");
     XD_REQUIRE_F(aligned16(pos), "calculate_p2p_f: pos must be 16-byte aligned");
-    const int lp = scan_lanes(np);
-#define XD_P2P_F(LP)                                                                                       \
-    k_p2p_f<LP><<<scan_blocks<LP>(np), 32 * kPoolWarps<LP>, 0, S(s)>>>(                                    \
-        PF, reinterpret_cast<const float4*>(pos), vel, omega, force, moment, mass, sorted_index, cstart, cend, cp, np)
-    if (lp == 1) XD_P2P_F(1);
-    else if (lp == 4) XD_P2P_F(4);
-    else XD_P2P_F(8);
-#undef XD_P2P_F
+    scan_shape<false>(np, [&](auto lp, auto nw) {
+        constexpr int LP = decltype(lp)::value, NW = decltype(nw)::value;
+        k_p2p_f<LP, NW><<<scan_blocks(np, LP, NW), 32 * NW, 0, S(s)>>>(PF, reinterpret_cast<const float4*>(pos), vel, omega,
+                                                                       force, moment, mass, sorted_index, cstart, cend,
+                                                                       cp, np);
+    });
     return launch_status("calculate_p2p_f");
 }
 
