@@ -675,7 +675,8 @@ int xd_batch_destroy(xd_batch* batch);
  * and around every contact launch.  xd_batch_kernel_times returns their
  * summed milliseconds and launch counts, [0] advance, [1] pair pass (the
  * whole contact pass in contact_mode 0) and [2] wall pass, since timing was
- * enabled.  XDEM_NO_GRAPHS=1 in the environment also makes a batch
+ * enabled; the two passes run one after the other while it is, and in one
+ * launch otherwise.  XDEM_NO_GRAPHS=1 in the environment also makes a batch
  * launch directly (profilers list no kernel inside a graph with conditional
  * nodes). */
 int xd_batch_set_timing(xd_batch* batch, int enable);

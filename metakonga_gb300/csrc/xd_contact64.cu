@@ -88,17 +88,18 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_p2p(Params P, const double
                                                double* __restrict__ force, double* __restrict__ moment,
                                                const double* __restrict__ mass, const unsigned* __restrict__ sorted,
                                                const unsigned* __restrict__ cstart, const unsigned* __restrict__ cend,
-                                               const xd_contact_property* __restrict__ cp, unsigned np)
+                                               const xd_contact_property* __restrict__ cp, unsigned np,
+                                               unsigned each)
 {
     using Buf = ScanBuf<LP, NW, double, 9>;
     __shared__ Buf B;
     __shared__ PairConst pc;
     if (threadIdx.x == 0) pc = load_pair_const(cp);   // (scan_contacts' barriers before the first use)
-    constexpr unsigned NP = 32 / LP, NB = NP * NW;
+    constexpr unsigned NP = 32 / LP;
     const unsigned lane = threadIdx.x & 31u;
-    for (unsigned b0 = blockIdx.x * NB; b0 < np; b0 += gridDim.x * NB) {
-        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
-        const bool valid = id < np;
+    for (unsigned b0 = blockIdx.x * each; b0 < np; b0 += gridDim.x * each) {
+        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP, end = min(np, b0 + each);
+        const bool valid = id < end;
         d4 ip = d4{ 0, 0, 0, 0 };
         int3 gp = make_int3(0, 0, 0);
         if (valid) {
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_p2p(Params P, const double
                 sumM += M;
             });
         const unsigned me = id0 + lane;
-        if (lane < NP && me < np) {
+        if (lane < NP && me < end) {
             st3(force, me, ld3rw(force, me) + sumF);
             st3(moment, me, ld3rw(moment, me) + sumM);
         }
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(32 * NW) k_polygon(Params P, const xd_polygon_
                                                 const unsigned* __restrict__ cstart,
                                                 const unsigned* __restrict__ cend,
                                                 const xd_contact_property* __restrict__ cp,
-                                                double* __restrict__ partials)
+                                                double* __restrict__ partials, unsigned each)
 {
     using Buf = ScanBuf<LP, NW, double, 12>;
     __shared__ Buf B;
@@ -520,9 +521,9 @@ __global__ void __launch_bounds__(32 * NW) k_polygon(Params P, const xd_polygon_
     bool reacted = false;
     const unsigned cnp = P.np, lane = threadIdx.x & 31u;
     const unsigned warp = blockIdx.x * NW + threadIdx.x / 32u;
-    for (unsigned b0 = blockIdx.x * NP * NW; b0 < cnp; b0 += gridDim.x * NP * NW) {
-        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
-        const bool valid = id < cnp;
+    for (unsigned b0 = blockIdx.x * each; b0 < cnp; b0 += gridDim.x * each) {
+        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP, end = min(cnp, b0 + each);
+        const bool valid = id < end;
         d4 ip = d4{ 0, 0, 0, 0 };
         int3 gp = make_int3(0, 0, 0);
         if (valid) {
@@ -916,8 +917,9 @@ int launch_p2p(const Params& P, const double* pos, const double* vel, const doub
     }
     scan_shape(np, [&](auto lp, auto nw) {
         constexpr int LP = decltype(lp)::value, NW = decltype(nw)::value;
-        k_p2p<LP, NW><<<scan_blocks(np, LP, NW), 32 * NW, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart,
-                                                                  cend, cp, np);
+        const ScanGrid g = scan_grid(np, LP, NW);
+        k_p2p<LP, NW><<<g.blocks, 32 * NW, 0, s>>>(P, pos, vel, omega, force, moment, mass, sorted, cstart, cend, cp, np,
+                                                   g.each);
     });
     return launch_status("calculate_p2p");
 }
@@ -975,10 +977,10 @@ int launch_polygon(const Params& P, const xd_polygon_info* dpi, xd_polygon_mass_
         } else {                                                                                                  \
             scan_shape(np, [&](auto lp, auto nw) {                                                                \
                 constexpr int LP = decltype(lp)::value, NW = decltype(nw)::value;                                 \
-                const unsigned grid = scan_blocks(np, LP, NW);                                                    \
-                parts = grid * NW;                                                                                \
-                k_polygon<NBV, LP, NW><<<grid, 32 * NW, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment,     \
-                                                                mass, sidx, cstart, cend, cp, part);              \
+                const ScanGrid g = scan_grid(np, LP, NW);                                                         \
+                parts = g.blocks * NW;                                                                            \
+                k_polygon<NBV, LP, NW><<<g.blocks, 32 * NW, 0, s>>>(P, dpi, dpmi, pos, vel, omega, force, moment, \
+                                                                    mass, sidx, cstart, cend, cp, part, g.each);  \
             });                                                                                                   \
         }                                                                                                         \
     } while (0)

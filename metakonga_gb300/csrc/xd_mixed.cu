@@ -11,8 +11,8 @@
 //   accelerations           FP32: the contact part a - g, and alpha
 //   1/m, 1/I                FP32 (the FP64 mass, by particle id, serves the
 //                           FP64 rechecks, the walls and the download)
-// The only FP64 operations per particle and step are the position update
-// (two adds per axis) and the fixed-point conversion (one FMA per axis).
+// The only FP64 operations per particle and step are the position update's
+// adds (two per axis); the fixed point comes from the mantissa (fixed_split).
 //
 // Per step (dem_simulation::oneStepAnalysis order, dem_simulation.cpp:447-469):
 //   k_mx_advance  the velocity-Verlet update in place (velocity of step t from

@@ -243,18 +243,19 @@ __global__ void __launch_bounds__(32 * NW) k_p2p_f(ParamsF P, const float4* __re
                                               const float* __restrict__ mass, const unsigned* __restrict__ sorted,
                                               const unsigned* __restrict__ cstart,
                                               const unsigned* __restrict__ cend,
-                                              const xd_contact_property_f* __restrict__ cpp, unsigned np)
+                                              const xd_contact_property_f* __restrict__ cpp, unsigned np,
+                                              unsigned each)
 {
     using Buf = ScanBuf<LP, NW, float, 9>;
     __shared__ Buf B;
     __shared__ PairConstF pc;
     if (threadIdx.x == 0) pc = pair_const_f(*cpp);   // (scan_contacts' barriers before the first use)
-    constexpr unsigned NP = 32 / LP, NB = NP * NW;
+    constexpr unsigned NP = 32 / LP;
     const xd_contact_property_f cp = *cpp;
     const unsigned lane = threadIdx.x & 31u;
-    for (unsigned b0 = blockIdx.x * NB; b0 < np; b0 += gridDim.x * NB) {
-        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP;
-        const bool valid = id < np;
+    for (unsigned b0 = blockIdx.x * each; b0 < np; b0 += gridDim.x * each) {
+        const unsigned id0 = b0 + threadIdx.x / 32u * NP, id = id0 + lane / LP, end = min(np, b0 + each);
+        const bool valid = id < end;
         float4 ip = make_float4(0.f, 0.f, 0.f, 0.f);
         int3 gp = make_int3(0, 0, 0);
         if (valid) {
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(32 * NW) k_p2p_f(ParamsF P, const float4* __re
                 sumM += M;
             });
         const unsigned me = id0 + lane;
-        if (lane < NP && me < np) {
+        if (lane < NP && me < end) {
             stf3(force, me, ldf3(force, me) + sumF);
             stf3(moment, me, ldf3(moment, me) + sumM);
         }
@@ -715,9 +716,9 @@ int xd_calculate_p2p_f(int tcm, const float* pos, const float* vel, const float*
     XD_REQUIRE_F(aligned16(pos), "calculate_p2p_f: pos must be 16-byte aligned");
     scan_shape<false>(np, [&](auto lp, auto nw) {
         constexpr int LP = decltype(lp)::value, NW = decltype(nw)::value;
-        k_p2p_f<LP, NW><<<scan_blocks(np, LP, NW), 32 * NW, 0, S(s)>>>(PF, reinterpret_cast<const float4*>(pos), vel, omega,
-                                                                       force, moment, mass, sorted_index, cstart, cend,
-                                                                       cp, np);
+        const ScanGrid g = scan_grid(np, LP, NW);
+        k_p2p_f<LP, NW><<<g.blocks, 32 * NW, 0, S(s)>>>(PF, reinterpret_cast<const float4*>(pos), vel, omega, force, moment,
+                                                        mass, sorted_index, cstart, cend, cp, np, g.each);
     });
     return launch_status("calculate_p2p_f");
 }

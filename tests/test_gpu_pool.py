@@ -9,7 +9,7 @@ from .test_gpu_search import test_triangles as triangles_match
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [15, 16, 17, 32, 33, 4_863, 4_864, 4_895, 4_897])
+@pytest.mark.parametrize("n", [15, 16, 17, 32, 33, 4_863, 4_864, 4_865, 4_895, 4_897, 9_728, 9_729])
 def test_pool_edges(cuda, oracle, n):
     _both(_bed(n, seed=n), oracle)
 
