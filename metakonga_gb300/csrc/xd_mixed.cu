@@ -2548,17 +2548,31 @@ __device__ __forceinline__ void contact_entry_coop(const MixParams& P, const Con
 // in which the few wall runs, each a long chain of FP64 region tests, run
 // beside the pairs' instead of after them.
 //
-// A wall run holds kWallRun particles, whose data their lanes write to shared
-// memory once for all their candidates.
-constexpr unsigned kWallRun = 8;
+// A wall run holds 8 particles, whose data their lanes write to shared memory
+// once for all their candidates; in a batch with a long front (several runs a
+// warp) 16.  A short front is done when its longest run is; a long one is
+// bound by how full the groups of 32 candidates are: 256 hoppers of 11.56 M
+// spheres 6,140 us a step with 8 (the walls 1,527), 5,620 with 16 (1,046), 6,180
+// with 32 (904: their data takes the pair runs' L1).  A scene's own pass keeps
+// the buffer of 8: with 16 a hopper of 199,583 spheres takes 65 us against 60.
+constexpr unsigned kWallRun = 8, kBatchWallRun = 16;
 
-struct WallBuf {
+__device__ __forceinline__ unsigned batch_wall_run(unsigned front)
+{
+    return front > 4u * kWallRun * kContactWarpsTotal ? kBatchWallRun : kWallRun;
+}
+
+template <unsigned N>
+struct WallBufOf {
     PairBuf c;
-    WallOwn own[kWallRun];
+    WallOwn own[N];
 };
+using WallBuf = WallBufOf<kWallRun>;
+using BatchWallBuf = WallBufOf<kBatchWallRun>;
 
+template <unsigned N>
 __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const ContactArgs& C, bool valid, unsigned i,
-                                                 WallBuf& WB)
+                                                 WallBufOf<N>& WB)
 {
     CoopBuf& B = WB.c.c;
     const unsigned lane = threadIdx.x & 31u;
@@ -2584,7 +2598,7 @@ __device__ __forceinline__ void walls_entry_coop(const MixParams& P, const Conta
         }
     }
     const bool any = wm || kb < ke;
-    if (any) WB.own[lane] = load_wall_own(P, C, i);   // lane < kWallRun
+    if (any) WB.own[lane] = load_wall_own(P, C, i);   // lane < N
     f3 f = fk(0.f, 0.f, 0.f), Ftri = fk(0.f, 0.f, 0.f);
     RxnAcc ra;
     ra.b = 0xffffffffu;
@@ -4371,8 +4385,8 @@ __device__ __forceinline__ unsigned batch_list(const BatchScene& d, bool walls)
 
 // Runs of listed particles per scene, as an exclusive prefix over scenes, of
 // the wall runs' or the pair runs' lists, into runs[0, ns]; runs[ns + 1] (the next free run) cleared,
-// and the particles a run holds (`each`, or with 0 run_size of all scenes'
-// together) in runs[ns + 2].
+// and the particles a run holds (`each`, or with 0 the run size of all scenes'
+// lists together) in runs[ns + 2].
 __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, bool walls, unsigned each,
                            unsigned* __restrict__ runs, unsigned* c, unsigned& carry)
 {
@@ -4383,7 +4397,9 @@ __device__ void batch_runs(const BatchScene* __restrict__ D, unsigned ns, bool w
     all = __reduce_add_sync(0xffffffffu, all);
     if ((threadIdx.x & 31u) == 0 && all) atomicAdd(&carry, all);
     __syncthreads();
-    const unsigned run = each ? each : run_size(carry, kContactWarpsTotal);
+    const unsigned run = each    ? each
+                         : walls ? batch_wall_run(carry)
+                                 : run_size(carry, kContactWarpsTotal);
     __syncthreads();
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -4420,7 +4436,7 @@ __global__ void __launch_bounds__(1024) k_batch_chunks(const BatchScene* __restr
     __shared__ unsigned c[1024];
     __shared__ unsigned carry;
     batch_runs(D, ns, false, per_particle ? 32u : 0u, chunk_start, c, carry);
-    batch_runs(D, ns, true, kWallRun, chunk_start + ns + 3, c, carry);
+    batch_runs(D, ns, true, 0u, chunk_start + ns + 3, c, carry);
 }
 
 // The contact pass of every scene: each warp takes the next kBatchGrab runs
@@ -4440,7 +4456,7 @@ __host__ __device__ constexpr unsigned batch_scene_bytes(unsigned nwarps)
 // runs (over the front of each scene's list).
 template <int KIND>
 __device__ __forceinline__ void batch_runs_of(const BatchScene* __restrict__ D, unsigned ns,
-                                              unsigned* __restrict__ chunk_start, WarpScene& W, WallBuf* B)
+                                              unsigned* __restrict__ chunk_start, WarpScene& W, BatchWallBuf* B)
 {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned total = __ldg(chunk_start + ns);
@@ -4488,7 +4504,7 @@ __device__ __forceinline__ void batch_runs_of(const BatchScene* __restrict__ D, 
 
 // Out of line: the pair runs' registers are then theirs alone.
 __device__ __noinline__ void batch_wall_runs(const BatchScene* __restrict__ D, unsigned ns,
-                                             unsigned* __restrict__ chunk_start, WarpScene& W, WallBuf* B)
+                                             unsigned* __restrict__ chunk_start, WarpScene& W, BatchWallBuf* B)
 {
     batch_runs_of<2>(D, ns, chunk_start, W, B);
 }
@@ -4500,11 +4516,11 @@ __global__ void __launch_bounds__(kContactMaxThreads, KIND ? 4 : 1) k_batch_cont
                                                                    unsigned* __restrict__ chunk_start)
 {
     // dynamic shared memory: one WarpScene per warp of the block, then (the
-    // cooperative kinds) one WallBuf per warp
+    // cooperative kinds) one BatchWallBuf per warp
     extern __shared__ __align__(16) unsigned char batch_smem[];
     const unsigned wb = threadIdx.x / 32u, nwarps = blockDim.x / 32u;
     WarpScene& W = reinterpret_cast<WarpScene*>(batch_smem)[wb];
-    WallBuf* const B = reinterpret_cast<WallBuf*>(batch_smem + batch_scene_bytes(nwarps)) + wb;
+    BatchWallBuf* const B = reinterpret_cast<BatchWallBuf*>(batch_smem + batch_scene_bytes(nwarps)) + wb;
     if (KIND >= 2) batch_wall_runs(D, ns, chunk_start + ns + 3, W, B);
     if (KIND == 1 || KIND == 3) batch_runs_of<1>(D, ns, chunk_start, W, B);
     if (KIND == 0) batch_runs_of<0>(D, ns, chunk_start, W, nullptr);
@@ -4544,7 +4560,7 @@ template <int KIND>
 static void launch_batch_contact_kind(const MixedBatch* b, unsigned ns, cudaStream_t q)
 {
     const unsigned ct = b->cthreads, grid = kContactWarpsTotal * 32u / ct, w = ct / 32u;
-    const unsigned smem = batch_scene_bytes(w) + (KIND ? w * (unsigned)sizeof(WallBuf) : 0u);
+    const unsigned smem = batch_scene_bytes(w) + (KIND ? w * (unsigned)sizeof(BatchWallBuf) : 0u);
     k_batch_contact<KIND><<<grid, ct, smem, q>>>(b->d_scenes, ns, b->d_chunks);
 }
 
@@ -4817,7 +4833,7 @@ int mixed_batch_create(MixedScene* const* scenes, unsigned count, MixedBatch** o
     // 48 KB that a launch may take without asking
     {
         const unsigned w = kContactMaxThreads / 32u;
-        const int most = (int)(batch_scene_bytes(w) + w * sizeof(WallBuf));
+        const int most = (int)(batch_scene_bytes(w) + w * sizeof(BatchWallBuf));
         int st = XD_OK;
         for (const void* k : { (const void*)k_batch_contact<1>, (const void*)k_batch_contact<2>,
                                (const void*)k_batch_contact<3> })
