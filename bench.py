@@ -576,11 +576,6 @@ def run_ours(a):
                 "d2h_bytes_per_step": d2h},
         "gpu_launches": launches,
         "cell_rebinnings_in_timed_steps": rebuilds,
-        "autotune": tuned,
-        "step_beyond_kernels_ms": {"value": other_ms, "of_step": other_ms / (ms / a.steps),
-                                   "note": "ms per batch step minus the advance and contact launches' live "
-                                           "times: re-binnings, the decision kernel, run prefix, graph and "
-                                           "conditional nodes -- the most a persistent kernel could save"},
         "roofline": roof,
         "phase_ms_per_launch": phase_ms,
         "other_form": plain,
