@@ -139,13 +139,23 @@ void* workspace(size_t bytes, int* status);
 
 inline unsigned div_up(unsigned a, unsigned b) { return (a + b - 1) / b; }
 
-// radix sort (xd_sort.cu): keys per tile, so that a sort has 65 to 128 tiles
+// radix sort (xd_sort.cu): keys per tile, so that a sort has 64 to 128 tiles
 // from 2^16 to 2^20 keys: enough to fill the chip, and few enough that their
 // digit counts (2,048 a tile, 1 MB up to 2^20 keys) stay small beside the keys.
 __host__ __device__ constexpr unsigned sort_tile(unsigned n)
 {
     return n <= (1u << 17) ? 1024u : (n <= (1u << 18) ? 2048u : (n <= (1u << 19) ? 4096u : 8192u));
 }
+// The most tiles that a sort of n keys or fewer has.  131,072 keys make 128
+// tiles and 131,073 make 65, so a buffer made for the larger count must be
+// sized by this: scenes with an emitter, or with a grid of their own for the
+// particles, sort fewer keys than they have room for.
+constexpr unsigned sort_tiles_within(unsigned n)
+{
+    const unsigned own = n / sort_tile(n) + (n % sort_tile(n) ? 1u : 0u);
+    return n > (1u << 17) && own < 128u ? 128u : own;
+}
+// Bytes that a sort of n keys or fewer needs; never less for a larger n.
 size_t radix_sort_scratch_bytes(unsigned n);
 // Kernel launches of one sort.
 unsigned radix_sort_launches(unsigned n, unsigned key_bits);

@@ -39,15 +39,13 @@
 
 namespace {
 
-// Same layout as xd_grid.cu / xd_sort.cu, at its largest over the sizes up to
-// n = XD_NOALLOC_MAX_ENTRIES: error word (256 B) + alternate keys + alternate
-// values + per-tile digit counts (2,048 x tiles) + the digits' totals, each
-// rounded up to 256 bytes.
+// Same layout as xd_grid.cu / xd_sort.cu for n = XD_NOALLOC_MAX_ENTRIES, which
+// holds every smaller sort as well: error word (256 B) + alternate keys +
+// alternate values + per-tile digit counts (2,048 x tiles) + the digits'
+// totals, each rounded up to 256 bytes.
 constexpr size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 constexpr size_t kMax = XD_NOALLOC_MAX_ENTRIES;
-constexpr size_t tiles_of(size_t n) { return (n + xd::sort_tile((unsigned)n) - 1) / xd::sort_tile((unsigned)n); }
-constexpr size_t max3(size_t a, size_t b, size_t c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
-constexpr size_t kTiles = max3(tiles_of(1u << 17), tiles_of(1u << 19), tiles_of(kMax));
+constexpr size_t kTiles = xd::sort_tiles_within((unsigned)kMax);
 constexpr size_t kScratchBytes = 256 + al256(4 * kMax) + al256(4 * kMax) + al256(4 * 2048 * kTiles) +
                                  al256(4 * 2048);
 

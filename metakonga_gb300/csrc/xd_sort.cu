@@ -267,15 +267,16 @@ __global__ void __launch_bounds__(kRankThreads) k_rank(const unsigned* __restric
     }
 }
 
+// Every part is at least as large as for any smaller n, and so is the whole:
+// a sort of fewer keys fits the scratch of a sort of more.
 struct SortLayout {
     size_t keys_alt, vals_alt, hist, total, bytes;
 };
 
-
 SortLayout layout(unsigned n)
 {
     SortLayout L;
-    const size_t ntiles = div_up(n ? n : 1u, sort_tile(n));
+    const size_t ntiles = n ? sort_tiles_within(n) : 1u;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     L.keys_alt = 0;
     L.vals_alt = L.keys_alt + al(sizeof(unsigned) * (size_t)n);
