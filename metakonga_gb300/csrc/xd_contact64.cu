@@ -453,31 +453,11 @@ int launch_cylinder(const Params& P, const xd_cylinder_info* cyl, const xd_conta
 
 __device__ __forceinline__ d3 ldp(const double* a) { return mk(__ldg(a), __ldg(a + 1), __ldg(a + 2)); }
 
-// Whether a sphere may touch triangle t: its box, then its FP32 distance,
-// each against the radius with a margin above the rounding of the world
-// coordinates (2^-23 of each) and of the region test.  A triangle so thin that the FP32 region test could go astray
-// (sin^2 of the angle at P below 1e-3) counts as near, as does a value that
-// is not finite.
 __device__ __forceinline__ bool triangle_near(const Near4& p, const xd_polygon_info* __restrict__ t)
 {
-    const float ax = f32_of(__ldg(t->P)), ay = f32_of(__ldg(t->P + 1)), az = f32_of(__ldg(t->P + 2));
-    const float bx = f32_of(__ldg(t->Q)), by = f32_of(__ldg(t->Q + 1)), bz = f32_of(__ldg(t->Q + 2));
-    const float cx = f32_of(__ldg(t->R)), cy = f32_of(__ldg(t->R + 1)), cz = f32_of(__ldg(t->R + 2));
-    const float size = fabsf(ax) + fabsf(ay) + fabsf(az) + fabsf(bx) + fabsf(by) + fabsf(bz) + fabsf(cx) +
-                       fabsf(cy) + fabsf(cz);
-    const float reach = p.r * 1.00001f + (size + p.size) * 1e-6f + 1e-15f;
-    if (fminf(ax, fminf(bx, cx)) - p.x > reach || p.x - fmaxf(ax, fmaxf(bx, cx)) > reach) return false;
-    if (fminf(ay, fminf(by, cy)) - p.y > reach || p.y - fmaxf(ay, fmaxf(by, cy)) > reach) return false;
-    if (fminf(az, fminf(bz, cz)) - p.z > reach || p.z - fmaxf(az, fmaxf(bz, cz)) > reach) return false;
-    const float ux = bx - ax, uy = by - ay, uz = bz - az, vx = cx - ax, vy = cy - ay, vz = cz - az;
-    const float uu = ux * ux + uy * uy + uz * uz, vv = vx * vx + vy * vy + vz * vz;
-    const float uv = ux * vx + uy * vy + uz * vz;
-    if (!(uu * vv - uv * uv > 1e-3f * uu * vv && uu * vv > 1e-30f)) return true;
-    bool face;
-    const float d2 = tri_dist2_f(ax - p.x, ay - p.y, az - p.z, bx - p.x, by - p.y, bz - p.z, cx - p.x, cy - p.y,
-                                 cz - p.z, face);
-    const float lim = reach + 1e-4f * (sqrtf(uu) + sqrtf(vv));
-    return !(d2 > lim * lim);
+    return tri_near(p.x, p.y, p.z, p.r, p.size, f32_of(__ldg(t->P)), f32_of(__ldg(t->P + 1)), f32_of(__ldg(t->P + 2)),
+                    f32_of(__ldg(t->Q)), f32_of(__ldg(t->Q + 1)), f32_of(__ldg(t->Q + 2)), f32_of(__ldg(t->R)),
+                    f32_of(__ldg(t->R + 1)), f32_of(__ldg(t->R + 2)));
 }
 
 // particle_polygonObject_collision_kernel<1> (impl:923-1021), a warp for
@@ -485,7 +465,7 @@ __device__ __forceinline__ bool triangle_near(const Near4& p, const xd_polygon_i
 //
 // A mesh's cells are as large as its triangles: here a particle's 27 cells
 // hold a thousand particles and a hundred triangles or none, and few
-// triangles touch it.  Entries are tested in FP32 (triangle_near) and the
+// triangles touch it.  Entries are tested in FP32 (tri_near) and the
 // FP64 closest point and law run on those that pass, one per lane, each
 // particle adding its own in search order (xd_scan.cuh).  A bed of 17,159
 // spheres on a cone of 4,096 triangles: 136 us, 3,512 with the closest point

@@ -5,6 +5,7 @@
 #pragma once
 
 #include "xd_internal.cuh"
+#include "xd_triangle.cuh"
 
 namespace xd {
 
@@ -386,59 +387,6 @@ __device__ __forceinline__ d3 closest_pt_triangle(d3 a, d3 b, d3 c, d3 p)
 {
     int region;
     return closest_pt_triangle_region(a, b, c, p, region);
-}
-
-// Squared distance from the origin to triangle abc in FP32 (the closest-point
-// regions of Ericson, Real-Time Collision Detection 5.1.5, with the query
-// point at the origin).  The distance is continuous across the regions, so a
-// region misjudged by rounding moves it by rounding only.  face: the closest
-// point is inside the face with every barycentric coordinate above 1e-5, far
-// beyond the FP32 rounding, so the FP64 region test of the reference takes its
-// face branch as well.
-__device__ __forceinline__ float tri_dist2_f(float ax, float ay, float az, float bx, float by, float bz, float cx,
-                                             float cy, float cz, bool& face)
-{
-    face = false;
-    const float abx = bx - ax, aby = by - ay, abz = bz - az;
-    const float acx = cx - ax, acy = cy - ay, acz = cz - az;
-    const float d1 = -(abx * ax + aby * ay + abz * az), d2 = -(acx * ax + acy * ay + acz * az);
-    if (d1 <= 0.f && d2 <= 0.f) return ax * ax + ay * ay + az * az;
-    const float d3 = -(abx * bx + aby * by + abz * bz), d4 = -(acx * bx + acy * by + acz * bz);
-    if (d3 >= 0.f && d4 <= d3) return bx * bx + by * by + bz * bz;
-    const float vc = d1 * d4 - d3 * d2;
-    float qx, qy, qz;
-    if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) {
-        const float v = d1 / (d1 - d3);
-        qx = ax + v * abx;
-        qy = ay + v * aby;
-        qz = az + v * abz;
-        return qx * qx + qy * qy + qz * qz;
-    }
-    const float d5 = -(abx * cx + aby * cy + abz * cz), d6 = -(acx * cx + acy * cy + acz * cz);
-    if (d6 >= 0.f && d5 <= d6) return cx * cx + cy * cy + cz * cz;
-    const float vb = d5 * d2 - d1 * d6;
-    if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) {
-        const float w = d2 / (d2 - d6);
-        qx = ax + w * acx;
-        qy = ay + w * acy;
-        qz = az + w * acz;
-        return qx * qx + qy * qy + qz * qz;
-    }
-    const float va = d3 * d6 - d5 * d4;
-    if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {
-        const float w = (d4 - d3) / ((d4 - d3) + (d5 - d6));
-        qx = bx + w * (cx - bx);
-        qy = by + w * (cy - by);
-        qz = bz + w * (cz - bz);
-        return qx * qx + qy * qy + qz * qz;
-    }
-    const float den = 1.f / (va + vb + vc);
-    const float v = vb * den, w = vc * den;
-    face = va * den > 1e-5f && v > 1e-5f && w > 1e-5f;
-    qx = ax + v * abx + w * acx;
-    qy = ay + v * aby + w * acy;
-    qz = az + v * abz + w * acz;
-    return qx * qx + qy * qy + qz * qz;
 }
 
 // The face normal particle_polygonObject_collision_kernel<1> pushes along
