@@ -107,6 +107,27 @@ void set_params(const Params& p)
 
 using namespace xd;
 
+// A word that kernels write and the calling thread reads after a
+// synchronisation, one a thread (a checked reorder returns with its work done,
+// so its next one finds the word free), given back when the thread ends.
+namespace {
+struct HostWord {
+    unsigned* p = nullptr;
+    HostWord()
+    {
+        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) !=
+            cudaSuccess) {
+            p = nullptr;
+            (void)cudaGetLastError();
+        }
+    }
+    ~HostWord()
+    {
+        if (p) (void)cudaFreeHost(p);
+    }
+};
+}  // namespace
+
 #define XD_REQUIRE(cond, ...)                                     \
     do {                                                          \
         if (!(cond)) return set_error(XD_ERR_INVALID, __VA_ARGS__); \
@@ -251,8 +272,8 @@ int xd_reorder_and_find_cell_start(unsigned* hash, unsigned* index, unsigned* cs
     int st;
     void* ws = workspace(reorder_scratch_bytes(n), &st);
     if (!ws) return st;
-    return reorder_and_find_cell_start(hash, index, cstart, cend, sorted_index, n, ncell, ws, S(s),
-                                       true);
+    static thread_local HostWord word;
+    return reorder_and_find_cell_start(hash, index, cstart, cend, sorted_index, n, ncell, ws, S(s), true, word.p);
 }
 
 int xd_radix_sort_pairs(unsigned* keys, unsigned* values, unsigned n, unsigned key_bits, void* s)

@@ -133,48 +133,21 @@ int launch_fill_cells(unsigned* cstart, unsigned* cend, unsigned ncell, cudaStre
     return launch_status("fill_cells");
 }
 
-// A word that kernels write and the calling thread reads after a
-// synchronisation, one a thread (a checked reorder returns with its work done,
-// so its next one finds the word free), given back when the thread ends.
-namespace {
-struct HostWord {
-    unsigned* p = nullptr;
-    HostWord()
-    {
-        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) !=
-            cudaSuccess) {
-            p = nullptr;
-            (void)cudaGetLastError();
-        }
-    }
-    ~HostWord()
-    {
-        if (p) (void)cudaFreeHost(p);
-    }
-};
-}  // namespace
-
 // scratch layout: [0, 256) error word, then the radix sort's buffers
 //
-// A checked call waits for the error word.  It lies in host memory then, which
-// the kernel writes only where a hash value is wrong: a copy of the device's
-// word into pageable memory held the call up for 6 us more (the grid of
-// 1,000,000 spheres 98 -> 92 us, a step of 8,000 196 -> 187).
+// A checked call waits for the error word: word if given, which lies in host
+// memory and which the kernel writes only where a hash value is wrong, else
+// the scratch's, copied.  That copy into pageable memory held the call up for
+// 6 us more (the grid of 1,000,000 spheres 98 -> 92 us, a step of 8,000 196 ->
+// 187).
 int reorder_and_find_cell_start(unsigned* hash, unsigned* index, unsigned* cstart, unsigned* cend,
                                 unsigned* sorted_index, unsigned n, unsigned ncell, void* scratch,
-                                cudaStream_t s, bool check)
+                                cudaStream_t s, bool check, unsigned* word)
 {
     if (n == 0) return launch_fill_cells(cstart, cend, ncell, s);
-    unsigned* err = static_cast<unsigned*>(scratch);
-    volatile unsigned* host = nullptr;
-    if (check) {
-        static thread_local HostWord word;
-        if (word.p) {
-            host = word.p;
-            *host = 0;
-            err = word.p;
-        }
-    }
+    volatile unsigned* host = word;
+    if (host) *host = 0;
+    unsigned* err = host ? word : static_cast<unsigned*>(scratch);
     void* sort_scratch = static_cast<char*>(scratch) + 256;
     unsigned *sk = nullptr, *sv = nullptr;
     int st = radix_sort_pairs(hash, index, n, key_bits_for(ncell), sort_scratch, s, &sk, &sv);

@@ -20,9 +20,11 @@ int launch_fill_cells(unsigned* cstart, unsigned* cend, unsigned ncell, cudaStre
 // is skipped and raises *err.  Cells without keys are left as they are.
 int launch_cell_bounds_sorted(unsigned* hash, unsigned* index, unsigned* cstart, unsigned* cend,
                               unsigned* sorted_index, unsigned n, unsigned ncell, unsigned* err, cudaStream_t s);
+// check: wait, and report a key >= ncell.  word (nullable): an error word in
+// host memory that the call has to itself until then.
 int reorder_and_find_cell_start(unsigned* hash, unsigned* index, unsigned* cstart, unsigned* cend,
                                 unsigned* sorted_index, unsigned n, unsigned ncell, void* scratch,
-                                cudaStream_t s, bool check);
+                                cudaStream_t s, bool check, unsigned* word = nullptr);
 
 // integrator (xd_integrate.cu)
 int launch_vv_position(const Params& P, double* pos, const double* vel, const double* acc,
