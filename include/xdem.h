@@ -20,8 +20,11 @@
  *
  * Calls on the same stream are ordered like the reference's default-stream
  * launches.  The stateless calls share one library workspace (for the radix
- * sort) and the parameter block set by xd_set_symbolic_parameter; like the
- * reference they are meant for one host thread and one stream at a time.
+ * sort, the mesh's reactions and the reductions) and the parameter block set
+ * by xd_set_symbolic_parameter; like the reference they are meant for one host
+ * thread and one stream at a time.  xd_reorder_and_find_cell_start (and its _f
+ * twin), which waits for its result, has scratch of its own for the length of
+ * the call: several threads may call it at once, each on a stream of its own.
  * Independent scenes run concurrently through xd_scene_* handles, which own
  * their parameters and workspace.
  */
@@ -150,7 +153,8 @@ size_t xd_sizeof(const char* struct_name);
  * that this build does not implement (used by the reference-API shim);
  * returns XD_ERR_INVALID. */
 int xd_report_unsupported(const char* what);
-/* Free the shared workspace of the stateless calls. */
+/* Free the shared workspace of the stateless calls, and the scratch that calls
+ * which have returned have left for the next. */
 int xd_release_workspace(void);
 
 /* setSymbolicParameter (mphysics_cuda_dec.cuh:110; mphysics_cuda_def.cu:13-16).

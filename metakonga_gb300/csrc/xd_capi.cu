@@ -83,17 +83,79 @@ void* workspace(size_t bytes, int* status)
     return g_ws;
 }
 
+namespace {
+// Scratch that a call has to itself until it returns, for one that waits for
+// its work: calls that run at once on several threads, each on a stream of its
+// own, then take different buffers.  The buffers of calls that have returned
+// are kept, as many as have run at once but no more than kKept, until
+// xd_release_workspace.
+struct Buffer {
+    void* p = nullptr;
+    size_t bytes = 0;
+};
+constexpr unsigned kKept = 16;
+Buffer g_kept[kKept];       // (g_ws_mu)
+unsigned g_nkept = 0;
+
+class CallScratch {
+public:
+    CallScratch(size_t bytes, cudaStream_t s, int* status) : s_(s)
+    {
+        *status = XD_OK;
+        {
+            std::lock_guard<std::mutex> lk(g_ws_mu);
+            if (g_nkept) {   // the largest
+                unsigned k = 0;
+                for (unsigned j = 1; j < g_nkept; ++j)
+                    if (g_kept[j].bytes > g_kept[k].bytes) k = j;
+                b_ = g_kept[k];
+                g_kept[k] = g_kept[--g_nkept];
+            }
+        }
+        if (bytes <= b_.bytes) return;
+        if (b_.p) cudaFree(b_.p);
+        b_ = Buffer{ nullptr, bytes + bytes / 4 + 4096 };
+        const cudaError_t e = cudaMalloc(&b_.p, b_.bytes);
+        if (e != cudaSuccess) {
+            b_ = Buffer();
+            *status = cuda_status(e, "workspace allocation");
+        }
+    }
+    ~CallScratch()
+    {
+        if (!b_.p) return;
+        if (!done_) (void)cudaStreamSynchronize(s_);   // a call that failed half-way: what it launched still uses it
+        {
+            std::lock_guard<std::mutex> lk(g_ws_mu);
+            if (g_nkept < kKept) {
+                g_kept[g_nkept++] = b_;
+                return;
+            }
+        }
+        cudaFree(b_.p);
+    }
+    CallScratch(const CallScratch&) = delete;
+    CallScratch& operator=(const CallScratch&) = delete;
+    void* get() const { return b_.p; }
+    void done() { done_ = true; }   // the call's work has been waited for
+
+private:
+    Buffer b_;
+    cudaStream_t s_;
+    bool done_ = false;
+};
+}  // namespace
+
 int release_workspace()
 {
     std::lock_guard<std::mutex> lk(g_ws_mu);
-    if (g_ws) {
-        cudaError_t e = cudaDeviceSynchronize();
-        cudaFree(g_ws);
-        g_ws = nullptr;
-        g_ws_bytes = 0;
-        return cuda_status(e, "release_workspace");
-    }
-    return XD_OK;
+    cudaError_t e = cudaSuccess;
+    if (g_ws || g_nkept) e = cudaDeviceSynchronize();
+    if (g_ws) cudaFree(g_ws);
+    g_ws = nullptr;
+    g_ws_bytes = 0;
+    while (g_nkept) cudaFree(g_kept[--g_nkept].p);
+    return cuda_status(e, "release_workspace");
 }
 
 const Params* params() { return g_have_params ? &g_params : nullptr; }
@@ -270,10 +332,12 @@ int xd_reorder_and_find_cell_start(unsigned* hash, unsigned* index, unsigned* cs
     XD_REQUIRE(ncell > 0, "reorder_and_find_cell_start: ncell must be > 0");
     if (n > 0) XD_REQUIRE(hash && index && sorted_index, "reorder_and_find_cell_start: null pointer");
     int st;
-    void* ws = workspace(reorder_scratch_bytes(n), &st);
-    if (!ws) return st;
+    CallScratch ws(reorder_scratch_bytes(n), S(s), &st);
+    if (st != XD_OK) return st;
     static thread_local HostWord word;
-    return reorder_and_find_cell_start(hash, index, cstart, cend, sorted_index, n, ncell, ws, S(s), true, word.p);
+    st = reorder_and_find_cell_start(hash, index, cstart, cend, sorted_index, n, ncell, ws.get(), S(s), true, word.p);
+    if (st == XD_OK) ws.done();
+    return st;
 }
 
 int xd_radix_sort_pairs(unsigned* keys, unsigned* values, unsigned n, unsigned key_bits, void* s)
