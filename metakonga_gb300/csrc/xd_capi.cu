@@ -88,11 +88,18 @@ namespace {
 // its work: calls that run at once on several threads, each on a stream of its
 // own, then take different buffers.  The buffers of calls that have returned
 // are kept, as many as have run at once but no more than kKept, until
-// xd_release_workspace.
+// xd_release_workspace.  With each comes an error word in host memory (null if
+// there is none to be had: the call then takes the device's).
 struct Buffer {
     void* p = nullptr;
     size_t bytes = 0;
+    unsigned* word = nullptr;
 };
+void free_buffer(const Buffer& b)
+{
+    if (b.p) (void)cudaFree(b.p);
+    if (b.word) (void)cudaFreeHost(b.word);
+}
 constexpr unsigned kKept = 16;
 Buffer g_kept[kKept];       // (g_ws_mu)
 unsigned g_nkept = 0;
@@ -114,11 +121,19 @@ public:
         }
         if (bytes <= b_.bytes) return;
         if (b_.p) cudaFree(b_.p);
-        b_ = Buffer{ nullptr, bytes + bytes / 4 + 4096 };
+        b_.bytes = bytes + bytes / 4 + 4096;
         const cudaError_t e = cudaMalloc(&b_.p, b_.bytes);
         if (e != cudaSuccess) {
+            b_.p = nullptr;
+            free_buffer(b_);
             b_ = Buffer();
             *status = cuda_status(e, "workspace allocation");
+            return;
+        }
+        if (!b_.word && cudaHostAlloc(reinterpret_cast<void**>(&b_.word), sizeof(unsigned),
+                                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            b_.word = nullptr;
+            (void)cudaGetLastError();
         }
     }
     ~CallScratch()
@@ -132,11 +147,12 @@ public:
                 return;
             }
         }
-        cudaFree(b_.p);
+        free_buffer(b_);
     }
     CallScratch(const CallScratch&) = delete;
     CallScratch& operator=(const CallScratch&) = delete;
     void* get() const { return b_.p; }
+    unsigned* word() const { return b_.word; }
     void done() { done_ = true; }   // the call's work has been waited for
 
 private:
@@ -154,7 +170,7 @@ int release_workspace()
     if (g_ws) cudaFree(g_ws);
     g_ws = nullptr;
     g_ws_bytes = 0;
-    while (g_nkept) cudaFree(g_kept[--g_nkept].p);
+    while (g_nkept) free_buffer(g_kept[--g_nkept]);
     return cuda_status(e, "release_workspace");
 }
 
@@ -168,27 +184,6 @@ void set_params(const Params& p)
 }  // namespace xd
 
 using namespace xd;
-
-// A word that kernels write and the calling thread reads after a
-// synchronisation, one a thread (a checked reorder returns with its work done,
-// so its next one finds the word free), given back when the thread ends.
-namespace {
-struct HostWord {
-    unsigned* p = nullptr;
-    HostWord()
-    {
-        if (cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) !=
-            cudaSuccess) {
-            p = nullptr;
-            (void)cudaGetLastError();
-        }
-    }
-    ~HostWord()
-    {
-        if (p) (void)cudaFreeHost(p);
-    }
-};
-}  // namespace
 
 #define XD_REQUIRE(cond, ...)                                     \
     do {                                                          \
@@ -334,8 +329,7 @@ int xd_reorder_and_find_cell_start(unsigned* hash, unsigned* index, unsigned* cs
     int st;
     CallScratch ws(reorder_scratch_bytes(n), S(s), &st);
     if (st != XD_OK) return st;
-    static thread_local HostWord word;
-    st = reorder_and_find_cell_start(hash, index, cstart, cend, sorted_index, n, ncell, ws.get(), S(s), true, word.p);
+    st = reorder_and_find_cell_start(hash, index, cstart, cend, sorted_index, n, ncell, ws.get(), S(s), true, ws.word());
     if (st == XD_OK) ws.done();
     return st;
 }
