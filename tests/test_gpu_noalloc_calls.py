@@ -1,11 +1,11 @@
 """The allocation-free reorder allocates nothing, page-locked host memory included, on a thread that has not called it
 before as well: no CUDA allocation is among the runtime calls that a profiler sees it make."""
-import threading
-
 import pytest
 import torch
 
 from metakonga_gb300._lib import XdemError, call, ptr
+
+from .cuda_calls import runtime_calls
 
 pytestmark = pytest.mark.gpu
 ALLOCATIONS = ("Alloc", "Free", "HostRegister")
@@ -32,12 +32,7 @@ def test_a_thread_s_first_call_allocates_nothing(cuda, n, bad):
         except XdemError:
             got.append(True)
 
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        t = threading.Thread(target=work)
-        t.start()
-        t.join()
-        torch.cuda.synchronize()
-    assert got == [bad]
-    names = [e.name for e in prof.events()]
+    names = runtime_calls(work)
+    assert got and set(got) == {bad}
     assert any("Launch" in x for x in names), names     # the call's launches are among them
     assert not [x for x in names if any(a in x for a in ALLOCATIONS)], names
