@@ -3231,8 +3231,8 @@ void mixed_destroy(MixedScene* s)
 {
     if (!s) return;
     cudaDeviceSynchronize();
-    for (int k = 0; k < 5; ++k)
-        if (s->graph[k]) cudaGraphExecDestroy(s->graph[k]);
+    for (cudaGraphExec_t g : s->graph)
+        if (g) cudaGraphExecDestroy(g);
     for (void* p : s->allocs) cudaFree(p);
     delete s;
 }
