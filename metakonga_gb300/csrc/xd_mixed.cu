@@ -247,7 +247,7 @@ struct MixedScene {
     // host-order transfer buffers
     double* xfer = nullptr;
     bool ready = false;                // grid and buffers set up (first upload)
-    cudaGraphExec_t graph[6] = {};   // step graphs (kFirstStep to kLoop)
+    cudaGraphExec_t graph[7] = {};   // step graphs (kFirstStep to kOneStep)
     // tangential-spring history (an extension): [s * n + slot] tables in the
     // state's slot order, permuted with the particles at re-binning
     unsigned hslots = 0;
@@ -3776,7 +3776,14 @@ static int step_once(MixedScene* s, cudaStream_t q, const Phases& ph, bool recor
 // spheres 25 -> 18 us a step, 199,583 80 -> 75, 1,000,000 115 -> 108.  A skipped
 // kernel costs 1 to 2 us, so what eight steps save, a re-binning amid them loses
 // again in part; scenes that re-bin on every step take about as long as before.
-enum { kFirstStep = 0, kSteps1 = 1, kSteps2 = 2, kSteps4 = 3, kSteps8 = 4, kLoop = 5, kGraphKinds = 6 };
+//
+// kOneStep is a whole call of one step, its first and last kernels included:
+// one launch and one node instead of two of each and kernels beside them.  8,000
+// spheres take 38.6 us a call that is waited for, 57.6 by kFirstStep and kSteps1
+// (and 51 with a node after every advance); 199,583 112, 137 and 177.  Two steps
+// take 90 us by the graphs above and 103 with a node each.  Captured by the
+// first call of one step.
+enum { kFirstStep = 0, kSteps1 = 1, kSteps2 = 2, kSteps4 = 3, kSteps8 = 4, kLoop = 5, kOneStep = 6, kGraphKinds = 7 };
 
 constexpr unsigned kGraphMinSteps = 16;
 
@@ -3827,6 +3834,21 @@ static int capture_chunk(MixedScene* s, cudaStream_t q, unsigned steps, const Me
     return st == XD_OK ? capture_conditional(s, q, g.rebin, rebuild) : st;
 }
 
+// The last velocity update, and the call's body reactions.
+static int finish_call(MixedScene* s, cudaStream_t q, const Phases& ph)
+{
+    ph.begin(0, q);
+    k_mx_finish<<<blocks(s->n, 256), 256, 0, q>>>(s->P, s->m[0], s->Fc, s->Mc, s->Fw);
+    int st = launch_status("mixed finish");
+    ph.end(0, q);
+    if (st == XD_OK) {
+        ph.begin(3, q);
+        st = flush_reactions(s, q);
+        ph.end(3, q);
+    }
+    return st;
+}
+
 static int capture_steps(MixedScene* s, int kind)
 {
     cudaStream_t cs = nullptr;
@@ -3864,6 +3886,12 @@ static int capture_steps(MixedScene* s, int kind)
             st = capture_conditional(
                 s, cs, more, [&](MixedScene* sc, cudaStream_t q) { return capture_chunk(sc, q, 8, mb, &more); },
                 cudaGraphCondTypeWhile);
+    } else if (st == XD_OK && kind == kOneStep) {
+        k_call_begin<<<1, 1, 0, cs>>>(s->counters, 1, 0);
+        st = launch_status("mixed call");
+        if (st == XD_OK) st = capture_chunk(s, cs, 0, mb, nullptr);
+        if (st == XD_OK) st = contact_step<1>(s, cs, Phases(), false, 0, false);
+        if (st == XD_OK) st = finish_call(s, cs, Phases());
     } else if (st == XD_OK) {
         st = capture_chunk(s, cs, kind == kFirstStep ? 0u : 1u << (kind - 1), mb, nullptr);
     }
@@ -3913,14 +3941,21 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
     // whose graphs an emission has just dropped (its particle count changed)
     // launches directly
     const bool graphs = s->use_graphs && ph.fn == nullptr &&
-                        (!s->emitted || s->graph[kFirstStep] || nsteps >= kGraphMinSteps);
+                        (!s->emitted || s->graph[kFirstStep] || s->graph[kOneStep] || nsteps >= kGraphMinSteps);
     if (graphs) {
         // Every step in a graph, re-binning decided on the device: the call
         // never waits for the GPU.  A scene without cells yet (after an
         // upload) is made to re-bin through the same flag.
-        // all step graphs are captured at the first call, so that later calls
-        // of any length only replay
-        for (int kind = 0; kind < kGraphKinds && st == XD_OK; ++kind)
+        if (nsteps == 1) {
+            if (!s->cells_clean)
+                st = cuda_status(cudaMemsetAsync(s->counters + CN_REBUILD, 1, 1, q), "mixed re-binning flag");
+            if (st == XD_OK) st = launch_steps(s, kOneStep, q);
+            if (st == XD_OK) s->cells_clean = true;
+            return st;
+        }
+        // the other step graphs are captured together, so that later calls of
+        // any length only replay
+        for (int kind = 0; kind <= kLoop && st == XD_OK; ++kind)
             if (!s->graph[kind]) st = capture_steps(s, kind);
         if (st != XD_OK) return st;
         k_call_begin<<<1, 1, 0, q>>>(s->counters, nsteps, s->cells_clean ? 0 : 1);
@@ -3930,8 +3965,7 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
         for (; st == XD_OK && left >= 8; left -= 8) st = launch_steps(s, kSteps8, q);
         for (int kind = kSteps4; kind >= kSteps1 && st == XD_OK; --kind)
             if (left & (1u << (kind - 1))) st = launch_steps(s, kind, q);
-        // (single steps never fall short)
-        if (st == XD_OK && nsteps > 1) st = launch_steps(s, kLoop, q);
+        if (st == XD_OK) st = launch_steps(s, kLoop, q);
         if (st != XD_OK) return st;
         s->cells_clean = true;
     } else {
@@ -3940,17 +3974,7 @@ int mixed_step(MixedScene* s, unsigned nsteps, cudaStream_t q, const Phases& ph)
         for (unsigned t = 1; t < nsteps && st == XD_OK; ++t) st = step_once<1>(s, q, ph, false, 0);
         if (st != XD_OK) return st;
     }
-    // the last velocity update, and the call's body reactions
-    ph.begin(0, q);
-    k_mx_finish<<<blocks(s->n, 256), 256, 0, q>>>(s->P, s->m[0], s->Fc, s->Mc, s->Fw);
-    st = launch_status("mixed finish");
-    ph.end(0, q);
-    if (st == XD_OK) {
-        ph.begin(3, q);
-        st = flush_reactions(s, q);
-        ph.end(3, q);
-    }
-    return st;
+    return finish_call(s, q, ph);
 }
 
 unsigned long long mixed_launches(MixedScene* s, unsigned nsteps)
@@ -4140,7 +4164,7 @@ int mixed_set_active(MixedScene* s, unsigned active, bool restore, cudaStream_t 
     s->cells_clean = false;
     // the step graphs hold the particle count: replaced once the launches
     // queued from them have run
-    if (s->graph[kFirstStep]) st = cuda_status(cudaStreamSynchronize(q), "scene emitter");
+    if (s->graph[kFirstStep] || s->graph[kOneStep]) st = cuda_status(cudaStreamSynchronize(q), "scene emitter");
     destroy_graphs(s);
     s->emitted = true;
     return st;
