@@ -77,7 +77,7 @@ struct Params {
     double cohesion;
     double g[3];
     double wo[3];
-    float wof[3];    // FP32 estimates of wo and 1 / cs (set_cell_estimate): cell_of
+    float wof[3];    // FP32 estimates of wo and 1 / cs (set_cell_estimate): cell_of; with inv_csf 0 it divides
     float inv_csf;
 };
 

@@ -68,6 +68,7 @@ bool legacy_block(Legacy* out)
         L.P.g[a] = h.gravity[a];
         L.P.wo[a] = h.world_origin[a];
     }
+    set_cell_estimate(L.P);
     L.law = Fc{ h.kn, h.vn, h.ks, h.vs, h.mu };
     L.coh = h.cohesive;
     *out = L;

@@ -36,7 +36,8 @@ __device__ __forceinline__ float f32_of(double x)
 // bound it has the same integer part, and elsewhere (about one coordinate in
 // 4,000 on a 128-cell axis, or a value that is not finite) the FP64 division
 // decides.  Bound: x is cut by 2^-23 of itself, wo rounded by 2^-24, and the
-// difference, the product and the reciprocal round by 2^-24 each.
+// difference, the product and the reciprocal round by 2^-24 each.  (Without an
+// estimate, inv_csf 0, both sides of the first comparison are zero: divided.)
 __device__ __forceinline__ int cell_of(const Params& P, double x, int a)
 {
     const float xf = f32_of(x), q = (xf - P.wof[a]) * P.inv_csf, f = floorf(q);
