@@ -1055,7 +1055,7 @@ def run_batched(a):
     adv_gbs = n_tot * B_ADVANCE / (adv_ms / 1e3) / 1e9
     con_gbs = contact_bytes / (con_ms / 1e3) / 1e9
     adv_traffic = _traffic_from_profiles("advance_batch_hopper.md", "traffic_bytes_per_particle")
-    con_traffic = _traffic_from_profiles("contact_mixed_hopper_settled.md", "traffic_bytes_per_listed_sphere")
+    con_traffic = _traffic_from_profiles("contact_hopper_one_launch.md", "traffic_bytes_per_listed_sphere")
     kernels = {
         "advance": {"kernel": "k_batch_advance<1> (velocity-Verlet kick and drift, contact view and skin test of "
                               "every scene's spheres in one launch)",
@@ -1085,7 +1085,7 @@ def run_batched(a):
                         "launches after the timed ones",
             "kernels": kernels,
             "traffic_note": "DRAM bytes per unit of one ncu-captured launch (profiles/advance_batch_hopper.md per "
-                            "sphere, profiles/contact_mixed_hopper_settled.md per listed sphere, pair and wall "
+                            "sphere, profiles/contact_hopper_one_launch.md per listed sphere, pair and wall "
                             "passes) times the units here"}
     # per step: advance, decision, run prefix and contact over all scenes; per
     # call the finish and each scene's body-reaction sum; per re-binning its
