@@ -79,9 +79,9 @@ __device__ __forceinline__ bool spheres_near(const Near4& a, const Near4& b)
 // mesh) are tested in FP32 from integer-cut coordinates, and the FP64 law
 // runs on contacts alone, one per lane (xd_scan.cuh).  Every operation on a
 // contact and the order of every sum are the thread-per-particle form's, so
-// the results are the same bits.  A bed of 120,989 spheres: 0.4 ms, 3.5 ms
-// with the law evaluated where a thread found a contact; 8,000 spheres 50 us
-// (438), 17,159 on a mesh's cells of 2.5 cm 212 us (2,527).
+// the results are the same bits.  A bed of 120,989 spheres: 327 us, 3.5 ms
+// with the law evaluated where a thread found a contact; 8,000 spheres 37.5 us
+// (438), 17,159 on a mesh's cells of 2.5 cm 213 us (2,527).
 template <int LP, int NW>
 __global__ void __launch_bounds__(32 * NW, 16 / NW) k_p2p(Params P, const double* __restrict__ pos,
                                                const double* __restrict__ vel, const double* __restrict__ omega,
@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(128) k_p2p_hist(Params P, const double* __rest
 // uw), so a particle whose FP32 offset exceeds r by more than its rounding
 // has no contact and adds zero.  The few that remain are gathered by block
 // and run the FP64 code side by side: one warp of a block's eight instead of
-// every warp that holds a particle near the wall.
+// every warp that holds a particle near the wall.  8,000 spheres: 14 us a plane
+// (30 to 45 before), 17 for all five in one launch.
 __global__ void __launch_bounds__(256) k_planes(Params P, const xd_plane_info* __restrict__ planes,
                                                 const xd_contact_property* __restrict__ cps, unsigned cp_stride,
                                                 unsigned nplanes, const double* __restrict__ pos,
@@ -468,7 +469,7 @@ __device__ __forceinline__ bool triangle_near(const Near4& p, const xd_polygon_i
 // triangles touch it.  Entries are tested in FP32 (tri_near) and the
 // FP64 closest point and law run on those that pass, one per lane, each
 // particle adding its own in search order (xd_scan.cuh).  A bed of 17,159
-// spheres on a cone of 4,096 triangles: 136 us, 3,512 with the closest point
+// spheres on a cone of 4,096 triangles: 130 us, 3,512 with the closest point
 // of every triangle in the cells formed in FP64 by a thread per particle.
 //
 // Reaction on the polygon bodies: NB > 0 keeps sums for NB bodies, summed per

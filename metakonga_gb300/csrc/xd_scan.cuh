@@ -120,7 +120,9 @@ __device__ __forceinline__ unsigned stage_runs(Buf& B, bool valid, int3 gp, cons
 // or two of most particles and the adding runs on most lanes.  The groups run
 // on across the block's warps: the FP64 pipe takes as long for a group of
 // three contacts as for one of 32, and a warp's own last group was half empty
-// (us a call: P2P_FIGURES).
+// (pairs, us a call, a warp's own groups and a block's: 8,000 spheres 50 and
+// 40.5, 120,989 343 and 327, FP32 100,003 80 and 70; on a mesh's wide cells,
+// which the search bounds, 17,159 212 and 215).
 template <int LP, typename Buf, typename Near, typename Eval, typename Add>
 __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsigned* __restrict__ sorted, Near near,
                                               Eval eval, Add add)
@@ -221,17 +223,18 @@ __device__ __forceinline__ void scan_contacts(Buf& B, unsigned nruns, const unsi
 // fills its lanes best (131 contacts of a bed in five groups); with few
 // particles the chip is not full and more lanes shorten the chain of loads
 // and contacts that one warp goes through.  FP64 pairs, us with 1 / 4 / 8
-// lanes: a bed of 2,000 spheres 70 / 37 / 25, 8,000 79 / 46 / 46, 17,000
+// lanes: a bed of 2,000 spheres 70 / 37 / 25, 8,000 78 / 46 / 42, 17,000
 // 99 / 73 / 85, 40,000 144 / 139 / 163, 60,000 184 / 210 / 226, 120,989
-// 339 / 400 / 427; on a mesh's wide cells 17,159 581 / 218 / 255 and 60,000
-// 2,025 / 1,858 / 2,303.
+// 339 / 400 / 426; on a mesh's wide cells 17,159 583 / 220 / 254 and 60,000
+// 2,032 / 1,860 / 2,301.
 //
 // Warps whose contacts a block pools: for the FP64 law 2, 4 or 8 by lanes per
 // particle, about 32 to 64 particles a block, but with fewer than 152 blocks of
-// 8 warps half as many (2,000 spheres: 8 warps 31 us, 4 25, 2 27; 8,000: 46, 48
-// and 54).  The FP32 law gains from full groups only where there are many: 2
-// warps (8,000 spheres: 8 warps 20.8 us, 2 18.6), and 1 lane a particle from
-// 28,000 on (30,000: 35.3 us, with 4 lanes 37.3; 100,003: 70 and 94).
+// 8 warps half as many (2,000 spheres: 8 warps 31 us, 4 25, 2 27; 8,000, before
+// every SM got as many blocks: 46, 48 and 54).  The FP32 law gains from full
+// groups only where there are many: 2 warps (8,000 spheres: 8 warps 20.8 us, 2
+// 18.8), and 1 lane a particle from 28,000 on (30,000: 36.6 us, with 4 lanes
+// 37.3; 100,003: 72 and 94).
 //
 // f(lanes, warps), each as a type's value, for np particles.
 template <int V>

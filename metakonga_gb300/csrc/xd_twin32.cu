@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256) k_hash_f(ParamsF P, unsigned* __restrict_
 // search order (xd_scan.cuh).  The law holds a power and an FP64 quotient and
 // root: 100,003 spheres in a bed took 242 us with it evaluated where a thread
 // found a contact, and the partners' velocities read for every candidate;
-// they take 81 us here.
+// they take 70 us here.
 template <unsigned L>
 __device__ __forceinline__ void put3f(float (*res)[L], int a, unsigned lane, f3 v)
 {
