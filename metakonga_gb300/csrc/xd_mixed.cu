@@ -1257,9 +1257,9 @@ __device__ __forceinline__ d3 tri_vertex(const double* v) { return mk(__ldg(v), 
 
 // Per particle: the triangles of its cell within r + skin, in id order.  The
 // test is FP32 (vertices and centre relative to the grid origin, rounded
-// within about 1e-7 m) with a 1e-5 m margin: a list may hold a triangle just
-// out of reach (the contact pass decides each contact exactly), never miss
-// one within it.
+// within about 1e-7 m) with a 1e-5 m margin, a needle's by its longest edge: a
+// list may hold a triangle just out of reach (the contact pass decides each
+// contact exactly), never miss one within it.
 __global__ void __launch_bounds__(256) k_tri_build(MixParams P, const float4* __restrict__ pf,
                                                    const unsigned* __restrict__ keys,
                                                    const unsigned* __restrict__ tpk,
@@ -1285,10 +1285,13 @@ __global__ void __launch_bounds__(256) k_tri_build(MixParams P, const float4* __
         if (sqrtf(sx * sx + sy * sy + sz * sz) - bs.w > lim) continue;
         const float* v = tri_ref + 9 * (size_t)t;
         bool face;
-        const float d2 = tri_dist2_f(__ldg(v) - p.x, __ldg(v + 1) - p.y, __ldg(v + 2) - p.z, __ldg(v + 3) - p.x,
-                                     __ldg(v + 4) - p.y, __ldg(v + 5) - p.z, __ldg(v + 6) - p.x,
-                                     __ldg(v + 7) - p.y, __ldg(v + 8) - p.z, face);
-        if (d2 < lim * lim || !(d2 < 3.0e38f)) {
+        const float ax = __ldg(v), ay = __ldg(v + 1), az = __ldg(v + 2), bx = __ldg(v + 3), by = __ldg(v + 4);
+        const float bz = __ldg(v + 5), cx = __ldg(v + 6), cy = __ldg(v + 7), cz = __ldg(v + 8);
+        const float d2 = tri_dist2_f(ax - p.x, ay - p.y, az - p.z, bx - p.x, by - p.y, bz - p.z, cx - p.x, cy - p.y,
+                                     cz - p.z, face);
+        if (d2 < lim * lim || !(d2 < 3.0e38f) ||
+            (tri_needle(bx - ax, by - ay, bz - az, cx - ax, cy - ay, cz - az) &&
+             tri_edge_near(p.x - ax, p.y - ay, p.z - az, lim, bx - ax, by - ay, bz - az, cx - ax, cy - ay, cz - az))) {
             if (c < P.tcap) tlist[(size_t)c * n + i] = t;
             ++c;
         }
@@ -2275,7 +2278,8 @@ __device__ __forceinline__ void contact_entry(const MixParams& P, const ContactA
                 const float span = fabsf(ax) + fabsf(ay) + fabsf(az) + fabsf(bx) + fabsf(by) + fabsf(bz) + fabsf(cx) +
                                    fabsf(cy) + fabsf(cz);
                 const float lim = (float)r + 1e-6f + 1e-5f * span;
-                if (d2f > lim * lim && d2f < 3.0e38f) continue;
+                if (d2f > lim * lim && d2f < 3.0e38f && !tri_needle(bx - ax, by - ay, bz - az, cx - ax, cy - ay, cz - az))
+                    continue;
             }
             const d3 cpt = closest_pt_triangle(Pv, Qv, Rv, ip);
             const double cdist = r - length(ip - cpt);

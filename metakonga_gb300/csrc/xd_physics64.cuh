@@ -401,7 +401,9 @@ __device__ __forceinline__ d3 triangle_normal(d3 P, d3 Q, d3 R)
 // Per-triangle record of the mixed form's contact pass, written whenever a
 // mesh is placed: vertex P and the face normal in FP64 (the plane distance
 // of a face contact is n . (x - P)), the edges Q - P and R - P in FP32 (the
-// region test relative to the sphere), and the polygon body.
+// region test relative to the sphere), and the polygon body.  A needle's edge
+// is not a number: no FP32 test of it passes or fails, and the pass takes the
+// FP64 closest point.
 struct __align__(16) TriRec {
     double p[3];
     double n[3];
@@ -418,6 +420,7 @@ __device__ __forceinline__ void write_tri_rec(TriRec* __restrict__ out, d3 P, d3
     t.n[0] = n.x; t.n[1] = n.y; t.n[2] = n.z;
     t.q[0] = (float)rn::sub(Q.x, P.x); t.q[1] = (float)rn::sub(Q.y, P.y); t.q[2] = (float)rn::sub(Q.z, P.z);
     t.r[0] = (float)rn::sub(R.x, P.x); t.r[1] = (float)rn::sub(R.y, P.y); t.r[2] = (float)rn::sub(R.z, P.z);
+    if (tri_needle(t.q[0], t.q[1], t.q[2], t.r[0], t.r[1], t.r[2])) t.q[0] = __int_as_float(0x7fffffff);
     t.body = body;
     t.pad = 0;
     *out = t;
