@@ -1162,7 +1162,8 @@ __global__ void __launch_bounds__(256) k_tri_count(MixParams P, const xd_polygon
     float v[9];
     tri_box(P, poly + t, lo, hi, v);
     for (int k = 0; k < 9; ++k) tri_ref[9 * (size_t)t + k] = v[k];
-    // bounding sphere for the list build: centroid and farthest vertex
+    // bounding sphere for the list build: centroid and farthest vertex (a needle's
+    // radius with its sign set)
     const float gx = (v[0] + v[3] + v[6]) * (1.f / 3.f), gy = (v[1] + v[4] + v[7]) * (1.f / 3.f),
                 gz = (v[2] + v[5] + v[8]) * (1.f / 3.f);
     float rb = 0.f;
@@ -1170,7 +1171,8 @@ __global__ void __launch_bounds__(256) k_tri_count(MixParams P, const xd_polygon
         const float dx = v[3 * k] - gx, dy = v[3 * k + 1] - gy, dz = v[3 * k + 2] - gz;
         rb = fmaxf(rb, sqrtf(dx * dx + dy * dy + dz * dz));
     }
-    tbound[t] = make_float4(gx, gy, gz, rb);
+    const bool needle = tri_needle(v[3] - v[0], v[4] - v[1], v[5] - v[2], v[6] - v[0], v[7] - v[1], v[8] - v[2]);
+    tbound[t] = make_float4(gx, gy, gz, needle ? -rb : rb);
     tcells[t] = (unsigned)((hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1));
 }
 
@@ -1282,16 +1284,17 @@ __global__ void __launch_bounds__(256) k_tri_build(MixParams P, const float4* __
         // the triangle's bounding sphere first
         const float4 bs = __ldg(tbound + t);
         const float sx = bs.x - p.x, sy = bs.y - p.y, sz = bs.z - p.z;
-        if (sqrtf(sx * sx + sy * sy + sz * sz) - bs.w > lim) continue;
+        if (sqrtf(sx * sx + sy * sy + sz * sz) - fabsf(bs.w) > lim) continue;
         const float* v = tri_ref + 9 * (size_t)t;
         bool face;
-        const float ax = __ldg(v), ay = __ldg(v + 1), az = __ldg(v + 2), bx = __ldg(v + 3), by = __ldg(v + 4);
-        const float bz = __ldg(v + 5), cx = __ldg(v + 6), cy = __ldg(v + 7), cz = __ldg(v + 8);
-        const float d2 = tri_dist2_f(ax - p.x, ay - p.y, az - p.z, bx - p.x, by - p.y, bz - p.z, cx - p.x, cy - p.y,
-                                     cz - p.z, face);
-        if (d2 < lim * lim || !(d2 < 3.0e38f) ||
-            (tri_needle(bx - ax, by - ay, bz - az, cx - ax, cy - ay, cz - az) &&
-             tri_edge_near(p.x - ax, p.y - ay, p.z - az, lim, bx - ax, by - ay, bz - az, cx - ax, cy - ay, cz - az))) {
+        const float d2 = tri_dist2_f(__ldg(v) - p.x, __ldg(v + 1) - p.y, __ldg(v + 2) - p.z, __ldg(v + 3) - p.x,
+                                     __ldg(v + 4) - p.y, __ldg(v + 5) - p.z, __ldg(v + 6) - p.x,
+                                     __ldg(v + 7) - p.y, __ldg(v + 8) - p.z, face);
+        bool near = d2 < lim * lim || !(d2 < 3.0e38f);
+        if (!near && __float_as_int(bs.w) < 0)   // a needle
+            near = tri_edge_near(p.x - v[0], p.y - v[1], p.z - v[2], lim, v[3] - v[0], v[4] - v[1], v[5] - v[2],
+                                 v[6] - v[0], v[7] - v[1], v[8] - v[2]);
+        if (near) {
             if (c < P.tcap) tlist[(size_t)c * n + i] = t;
             ++c;
         }
